@@ -103,6 +103,46 @@ def test_gemm_ref_shapes_epilogues_and_row_independence(ops, dtype):
         ops.gemm_ref(ad, wd[:, :-1].contiguous())
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 33, 4), (8, 64, 36), (16, 32, 16), (17, 31, 20), (33, 129, 200), (200, 2048, 1536), (257, 6000, 52)])
+def test_gemm_ref_float32_tiles_give_the_plain_kernels_bits(ops, m, n, k):
+    """The kernel for rows of whole 16-byte pieces at the edges of its tile sizes, against the one that takes any
+    row (a left operand whose rows lie an odd number of words apart): the same sums in the same order, so the same bits."""
+    a, w, bias = rand(m, k).to(DEV), rand(n, k, scale=0.1, seed=1).to(DEV), rand(n, seed=2).to(DEV)
+    odd = torch.zeros(m + 1, k + 1, device=DEV)[:m, :k].copy_(a)
+    assert odd.stride(0) % 4
+    for epilogue in (ops.EPILOGUE_STORE, ops.EPILOGUE_STORE_F32, ops.EPILOGUE_RELU2):
+        assert torch.equal(ops.gemm_ref(a, w, bias, epilogue=epilogue), ops.gemm_ref(odd, w, bias, epilogue=epilogue))
+    base = rand(m, n, seed=3).to(DEV)
+    got, want = base.clone(), base.clone()
+    ops.gemm_ref(a, w, bias, out=got, epilogue=ops.EPILOGUE_ADD_F32)
+    ops.gemm_ref(odd, w, bias, out=want, epilogue=ops.EPILOGUE_ADD_F32)
+    assert torch.equal(got, want)
+    up = rand(n, k, scale=0.1, seed=4).to(DEV)
+    shifted = torch.zeros(n * k + 1, device=DEV)[1:].view(n, k).copy_(up)  # not on a 16-byte boundary: the plain kernel
+    assert torch.equal(ops.gemm_ref_swiglu(a, w, up), ops.gemm_ref_swiglu(a, w, shifted))
+
+
+@pytest.mark.parametrize("n,k", [(100, 1540), (65, 3584), (96, 8960), (33, 18948)])
+def test_gemm_ref_float32_cut_inner_dimension(ops, n, k):
+    """Inner dimensions that are cut over a cluster: the error bound of chains of 16 (16 units of 2^-24 of the sum of
+    magnitudes) and of the compensated sums behind them (2 more, and 1 for the store), and the same bits for a row
+    whatever the number of rows, which picks the tile."""
+    rows = 150
+    a, w = rand(rows, k), rand(n, k, scale=0.1, seed=1)
+    ad, wd = a.to(DEV), w.to(DEV)
+    got = ops.gemm_ref(ad, wd)
+    bound = 19 * 2.0**-24 * (a.double().abs() @ w.double().abs().T)
+    assert ((got.cpu().double() - a.double() @ w.double().T).abs() <= bound).all()
+    for some in (1, 8, 9, 17, 33, 64, 149):
+        assert torch.equal(ops.gemm_ref(ad[:some], wd), got[:some])
+    up = rand(n, k, scale=0.1, seed=2).to(DEV)
+    both = ops.gemm_ref_swiglu(ad, wd, up)
+    for some in (1, 9, 40):
+        assert torch.equal(ops.gemm_ref_swiglu(ad[:some], wd, up), both[:some])
+    want = (torch.nn.functional.silu(got) * ops.gemm_ref(ad, up)).cpu()
+    torch.testing.assert_close(both.cpu(), want, rtol=4e-6, atol=1e-6)  # (two exponentials and a division apart)
+
+
 def test_gemm_ref_is_true_float32(ops):
     """Operands that need 13 mantissa bits, chosen so that every product and every partial sum is
     exact in float32 (22 bits at most) whatever the order of summation: the result must equal the
