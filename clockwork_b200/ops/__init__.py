@@ -429,6 +429,9 @@ def copy_pages(cache: torch.Tensor, pairs: torch.Tensor, status: torch.Tensor) -
                                   _ptr(status), _stream()), "copy_pages")
 
 
+ATTENTION_ROWS_FROM = 4  # rows per request from which the kernel that shares a request's keys among 16 rows takes a step
+
+
 def attention_ref(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: torch.Tensor,
                   tok_seq: torch.Tensor, positions: torch.Tensor, num_heads: int, num_kv_heads: int,
                   head_dim: int, scale: float, window: int | None, status: torch.Tensor) -> torch.Tensor:
@@ -448,6 +451,14 @@ def attention_ref(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
     if head_dim > 256:
         raise ValueError(f"head_dim {head_dim} is larger than the attention kernels take (256)")
     out = torch.empty((n, num_heads * head_dim), dtype=q.dtype, device=q.device)
+    # float32 steps that are mostly prompts: blocks of 16 rows that share a request's keys (the same bits).  From four rows per
+    # request on; with fewer, blocks of rows of several requests would take them one after the other
+    if (q.dtype == torch.float32 and not window and n >= ATTENTION_ROWS_FROM * block_tables.shape[0] and head_dim % 4 == 0 and head_dim <= 128
+            and q.stride(0) % 4 == 0 and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16):
+        check(library().cw_attention_rows(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
+                                          _ptr(tok_seq), _ptr(positions), n, num_heads, num_kv_heads, head_dim, page_size,
+                                          block_tables.shape[1], pages, float(scale), _ptr(status), _stream()), "attention_rows")
+        return out
     check(library().cw_attention_ref(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
                                      _ptr(tok_seq), _ptr(positions), n, num_heads, num_kv_heads, head_dim, page_size,
                                      block_tables.shape[1], pages, float(scale), int(window or 0),

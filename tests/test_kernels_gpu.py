@@ -257,6 +257,30 @@ def test_attention_ref_mixed_batch(ops, status, dtype, nh, nkv, hd, ps, window):
     torch.testing.assert_close(out.float().cpu().view(n, nh, hd), want, **tol(dtype))
 
 
+@pytest.mark.parametrize("nh,nkv,hd,ps", [(6, 2, 128, 16), (3, 3, 48, 8), (2, 1, 4, 4), (4, 1, 16, 32)])
+def test_attention_ref_rows_that_share_keys_give_the_plain_kernels_bits(ops, status, monkeypatch, nh, nkv, hd, ps):
+    """Blocks of 16 rows against a block per row: portions that end within a block, single tokens among them, padding rows,
+    contexts at the edges of a chunk of 128 keys, and values that are not finite behind the keys a row sees."""
+    ctx_lens, q_lens = [128, 333, 1, 129, 41, 300], [23, 1, 1, 129, 41, 17]
+    k_cache, v_cache, tables, _, _ = paged_setup(ctx_lens, nkv, hd, ps, torch.float32)
+    last = [int(tables[s, (c - 1) // ps]) * ps + (c - 1) % ps for s, c in enumerate(ctx_lens)]
+    for s in (0, 3):  # the last token's value is seen by the last row of the request alone
+        v_cache.view(-1, nkv, hd)[last[s]] = float("inf")
+    n = sum(q_lens) + 5
+    g = torch.Generator().manual_seed(5)
+    wide = torch.randn(n, (nh + 2 * nkv) * hd, generator=g) * 2
+    pad = torch.full((5,), -1, dtype=torch.int32)
+    tok_seq = torch.cat([torch.full((q,), s, dtype=torch.int32) for s, q in enumerate(q_lens)] + [pad])
+    positions = torch.cat([torch.arange(c - q, c, dtype=torch.int32) for c, q in zip(ctx_lens, q_lens)] + [0 * pad])
+    args = [t.to(DEV) for t in (wide, k_cache, v_cache, tables, tok_seq, positions)]
+    got = ops.attention_ref(*args, nh, nkv, hd, hd**-0.5, None, status)
+    monkeypatch.setattr(ops, "ATTENTION_ROWS_FROM", 1 << 30)
+    want = ops.attention_ref(*args, nh, nkv, hd, hd**-0.5, None, status)
+    ops.raise_on_status(status)
+    assert torch.isinf(want).any() and not torch.isinf(want[: q_lens[0] - 1]).any()
+    assert torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0)) and torch.equal(got.isnan(), want.isnan())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_attention_ref_finds_one_far_key_and_the_windows_edge(ops, status, dtype):
     """One key among hundreds gets a score that stands out; the output must be that key's value.
