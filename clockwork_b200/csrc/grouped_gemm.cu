@@ -12,29 +12,11 @@
 // over the chosen or by their shares of the softmax over all; optionally only experts of the best runs of
 // neighbours), the grouping of (token, choice) pairs by expert, and the weighted sum of the experts'
 // outputs into the float32 residual, in choice order.
-#include "common.cuh"
+#include "grouped_gemm.cuh"
 
 #define GG_TM 32
 #define GG_TN 64
 #define GG_TK 32
-
-#define GG_EPI_STORE 0        // C (T) = acc
-#define GG_EPI_STORE_F32 1    // C (float) = acc
-#define GG_EPI_SILU_MUL 2     // C (T) = silu(acc) * acc2, acc2 from B2; with a positive `glu_limit` the clamped form below
-#define GG_EPI_SIGMOID_GATE 3 // C (T) = acc * sigmoid(gate[dst, c_group_off*g + n])
-#define GG_EPI_RELU2 4        // C (T) = max(acc, 0)^2
-#define GG_EPI_GROUP_GATE 5   // C (T) = acc * sigmoid(gate[dst, g]), `gate` float32: one number per row and group
-
-// The gated activation of the two-product form: silu(a) b, or, with a positive limit,
-//   a' = min(a, limit), b' = clamp(b, -limit, limit):  a' sigmoid(1.702 a') (b' + 1)
-__device__ __forceinline__ float gg_glu(float a, float b, float limit) {
-    if (limit > 0.f) {
-        a = fminf(a, limit);
-        b = fminf(fmaxf(b, -limit), limit);
-        return a / (1.f + expf(-1.702f * a)) * (b + 1.f);
-    }
-    return a / (1.f + expf(-a)) * b;
-}
 
 template <typename T, int EPI>
 __global__ void __launch_bounds__(256)
@@ -325,7 +307,8 @@ static int launch_grouped_mma(dim3 grid, cudaStream_t stream, const void* A, int
 }
 
 static int g_grouped_mma = 1;
-extern "C" int cw_grouped_gemm_set_mma(int on) { g_grouped_mma = on ? 1 : 0; return CW_OK; }
+// 1 (the default): the tensor-core kernels where they take the sizes; 2: the mma.sync kernel alone; 0: the CUDA-core kernel alone.
+extern "C" int cw_grouped_gemm_set_mma(int on) { g_grouped_mma = on < 0 || on > 2 ? 1 : on; return CW_OK; }
 
 template <typename T>
 static int launch_grouped(int epi, dim3 grid, cudaStream_t stream, const void* A, int lda, int a_group_off, const void* B,
@@ -354,7 +337,7 @@ static int launch_grouped(int epi, dim3 grid, cudaStream_t stream, const void* A
 extern "C" int cw_grouped_gemm(const void* A, int lda, int a_group_off, const void* B, const void* B2, long long b_stride,
                                void* C, int ldc, int c_group_off, const int* offsets, const int* a_index, int a_div,
                                const int* c_index, const void* gate, int ldg, int M, int Nout, int K, int G, int epilogue,
-                               float glu_limit, int dtype, cudaStream_t stream) {
+                               float glu_limit, int dtype, int* status, cudaStream_t stream) {
     if (M == 0) return CW_OK;
     if (M < 0 || Nout <= 0 || K <= 0 || G <= 0 || a_div <= 0) return CW_ERR_BAD_SIZE;
     if (epilogue == GG_EPI_SILU_MUL && B2 == nullptr) return CW_ERR_BAD_SIZE;
@@ -365,6 +348,9 @@ extern "C" int cw_grouped_gemm(const void* A, int lda, int a_group_off, const vo
     if (dtype == 0)
         return launch_grouped<float>(epilogue, grid, stream, A, lda, a_group_off, B, B2, b_stride, C, ldc, c_group_off, offsets,
                                      a_index, a_div, c_index, gate, ldg, M, Nout, K, G, glu_limit);
+    const GroupedArgs args = {(const bf16*)A, (const bf16*)B, (const bf16*)B2, lda, a_group_off, b_stride, C, ldc, c_group_off, offsets, a_index,
+                              a_div, c_index, gate, ldg, M, Nout, K, G, glu_limit, status};
+    if (dtype == 1 && g_grouped_mma == 1 && grouped_tc_takes(args, epilogue)) return grouped_tc_run(args, epilogue, stream);
     const bool aligned = K % 8 == 0 && lda % 8 == 0 && a_group_off % 8 == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)B & 15) == 0 &&
                          ((uintptr_t)B2 & 15) == 0;
     if (dtype == 1 && g_grouped_mma && aligned) {

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import torch
 
-from . import _need, _ptr, _stream, dtype_code
+from . import _need, _ptr, _stream, device_status, dtype_code
 from .library import check, library
 
 EPI_STORE, EPI_STORE_F32, EPI_SILU_MUL, EPI_SIGMOID_GATE, EPI_RELU2, EPI_GROUP_GATE = 0, 1, 2, 3, 4, 5
@@ -14,6 +14,12 @@ def set_tensor_cores(on: bool) -> None:
     """bfloat16 products in groups run on the tensor cores when their sizes allow (the default); ``False`` keeps them
     on the CUDA-core kernel that float32 runs use (for comparisons)."""
     library().cw_grouped_gemm_set_mma(1 if on else 0)
+
+
+def use_warp_products(only: bool) -> None:
+    """``True``: of the tensor-core kernels the one on ``mma.sync`` alone, which takes what TMA cannot address (for
+    comparisons); ``False``: the default."""
+    library().cw_grouped_gemm_set_mma(2 if only else 1)
 
 
 def per_head_product(a: torch.Tensor, a_head_width: int, w: torch.Tensor, out: torch.Tensor, out_head_width: int,
@@ -36,7 +42,7 @@ def per_head_product(a: torch.Tensor, a_head_width: int, w: torch.Tensor, out: t
             raise ValueError("head_gate must be float32 [N, >= heads] with unit column stride, and the only gate")
         gate, epilogue, ldg = head_gate, EPI_GROUP_GATE, head_gate.stride(0) if rows > 1 else max(head_gate.stride(0), head_gate.shape[1])
     check(library().cw_grouped_gemm(_ptr(a), a.shape[1], a_head_width, _ptr(w), None, n * k, _ptr(out), out.shape[1], out_head_width,
-                                    None, None, 1, None, _ptr(gate), ldg, rows, n, k, heads, epilogue, 0.0, dtype_code(a.dtype), _stream()),
+                                    None, None, 1, None, _ptr(gate), ldg, rows, n, k, heads, epilogue, 0.0, dtype_code(a.dtype), _ptr(device_status(a.device)), _stream()),
           "per_head_product")
     return out
 
@@ -79,6 +85,22 @@ def moe_group(sel: torch.Tensor, experts: int):
     return offsets, order
 
 
+GATHER_FROM = 32  # pairs per expert, on average, from which rows are copied into the order of their experts
+
+
+def _sorted_rows(x: torch.Tensor, offsets: torch.Tensor | None, order: torch.Tensor | None, top: int, experts: int):
+    """(rows, index, divisor) for a product of pairs in sorted order: ``x`` itself with the index that finds a pair's row, or,
+    for a prompt's bfloat16 rows, a copy of the rows in that order (TMA fetches rows that lie next to one another several
+    times as fast as it gathers them; gate and up of 2,048 tokens, 64 experts of 1,408 of which 6: 190 us beside the copy of
+    14 us, 385 us gathered; the copy of a few rows would cost a launch for nothing)."""
+    if order is None or order.numel() <= GATHER_FROM * experts or x.dtype != torch.bfloat16 or x.shape[1] % 8 or x.data_ptr() % 16:
+        return x, order, top
+    rows = torch.empty((order.numel(), x.shape[1]), dtype=x.dtype, device=x.device)
+    check(library().cw_gather_rows(_ptr(x), _ptr(rows), _ptr(order), _ptr(offsets[experts:]), order.numel(), top, x.shape[1] * 2, _stream()),
+          "gather_rows")
+    return rows, None, 1
+
+
 def expert_gate_up(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, offsets: torch.Tensor | None, order: torch.Tensor | None,
                    top: int, limit: float = 0.0) -> torch.Tensor:
     """silu(x Wg_e^T) * (x Wu_e^T) for every pair, rows in sorted order; weights [E, ff, W].  With a positive ``limit`` the
@@ -87,9 +109,10 @@ def expert_gate_up(x: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor, of
     experts, ff, w = w_gate.shape
     pairs = order.numel() if order is not None else x.shape[0]
     act = torch.empty((pairs, ff), dtype=x.dtype, device=x.device)
+    x, index, div = _sorted_rows(x, offsets, order, top, experts)
     check(library().cw_grouped_gemm(_ptr(x), x.shape[1], 0, _ptr(w_gate), _ptr(w_up), ff * w, _ptr(act), ff, 0, _ptr(offsets),
-                                    _ptr(order), top, None, None, 0, pairs, ff, w, experts, EPI_SILU_MUL, float(limit), dtype_code(x.dtype),
-                                    _stream()), "expert_gate_up")
+                                    _ptr(index), div, None, None, 0, pairs, ff, w, experts, EPI_SILU_MUL, float(limit), dtype_code(x.dtype),
+                                    _ptr(device_status(x.device)), _stream()), "expert_gate_up")
     return act
 
 
@@ -98,8 +121,10 @@ def expert_up_relu2(x: torch.Tensor, w_up: torch.Tensor, offsets: torch.Tensor, 
     experts, ff, w = w_up.shape
     pairs = order.numel()
     act = torch.empty((pairs, ff), dtype=x.dtype, device=x.device)
-    check(library().cw_grouped_gemm(_ptr(x), x.shape[1], 0, _ptr(w_up), None, ff * w, _ptr(act), ff, 0, _ptr(offsets), _ptr(order), top,
-                                    None, None, 0, pairs, ff, w, experts, EPI_RELU2, 0.0, dtype_code(x.dtype), _stream()), "expert_up_relu2")
+    x, index, div = _sorted_rows(x, offsets, order, top, experts)
+    check(library().cw_grouped_gemm(_ptr(x), x.shape[1], 0, _ptr(w_up), None, ff * w, _ptr(act), ff, 0, _ptr(offsets), _ptr(index), div,
+                                    None, None, 0, pairs, ff, w, experts, EPI_RELU2, 0.0, dtype_code(x.dtype),
+                                    _ptr(device_status(x.device)), _stream()), "expert_up_relu2")
     return act
 
 
@@ -109,7 +134,8 @@ def expert_down(act: torch.Tensor, w_down: torch.Tensor, offsets: torch.Tensor, 
     pairs = order.numel()
     y = torch.empty((pairs, w), dtype=torch.float32, device=act.device)
     check(library().cw_grouped_gemm(_ptr(act), ff, 0, _ptr(w_down), None, w * ff, _ptr(y), w, 0, _ptr(offsets), None, 1, _ptr(order),
-                                    None, 0, pairs, w, ff, experts, EPI_STORE_F32, 0.0, dtype_code(act.dtype), _stream()), "expert_down")
+                                    None, 0, pairs, w, ff, experts, EPI_STORE_F32, 0.0, dtype_code(act.dtype),
+                                    _ptr(device_status(act.device)), _stream()), "expert_down")
     return y
 
 

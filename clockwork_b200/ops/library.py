@@ -59,7 +59,8 @@ _SIGNATURES: dict[str, list] = {
     "cw_sum_rmsnorm_add": [P, P, P, F, F, P, F, I, I, P],
     "cw_softcap": [P, LL, F, F, P],
     # products in groups and the mixture of experts (csrc/grouped_gemm.cu)
-    "cw_grouped_gemm": [P, I, I, P, P, LL, P, I, I, P, P, I, P, P, I, I, I, I, I, I, F, I, P],
+    "cw_grouped_gemm": [P, I, I, P, P, LL, P, I, I, P, P, I, P, P, I, I, I, I, I, I, F, I, P, P],
+    "cw_gather_rows": [P, P, P, P, I, I, LL, P],
     "cw_grouped_gemm_set_mma": [I],
     "cw_latent_attention_set_mma": [I],
     "cw_moe_choose": [P, P, P, P, P, I, I, I, I, I, I, P, F, I, I, P],
