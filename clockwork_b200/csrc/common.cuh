@@ -120,12 +120,14 @@ __device__ __forceinline__ int sum_tokens_over_lanes(float (&part)[TOKENS], int 
     return first;
 }
 
-// Dynamic shared memory that a scan over a long portion asks for so that no two of its blocks share an SM: a step of `rows`
-// rows whose grid holds blocks for requests that bring none must not put two of the blocks that do work side by side while
-// other SMs idle.  Short steps keep what they need.
-static inline size_t cw_scan_smem(size_t needed, long long rows) {
-    const size_t alone = 120u << 10;
-    return rows >= 256 && needed < alone ? alone : needed;
+// Dynamic shared memory that a scan over a long portion asks for so that its blocks spread evenly: a request that has a block
+// for at most every SM gets no two of them on one (a step of `rows` rows whose grid holds blocks for requests that bring none
+// would otherwise put two of the blocks that do work side by side while other SMs idle); a request with up to two for every SM
+// gets no three (64 heads of 128 x 64 over 900, 333 and 65 tokens, token by token: 337 us in rounds of one per SM, 257 in one
+// round of two, 290 without a bound).  Short steps keep what they need.
+static inline size_t cw_scan_smem(size_t needed, long long rows, long long blocks_per_request) {
+    const size_t want = blocks_per_request <= 148 ? 120u << 10 : blocks_per_request <= 296 ? 76u << 10 : 0;
+    return rows >= 256 && needed < want ? want : needed;
 }
 
 // Block-wide reductions with a fixed order (warp tree, then warp 0 over the warp results),

@@ -419,7 +419,8 @@ extern "C" int cw_recurrence_scan(int form, const float* q, int ldq, const float
     if ((form != 3 && pre == nullptr) || (form == 3 && p0 == nullptr)) return CW_ERR_BAD_SIZE;
     const int wide = Dk % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && (!ch || ldp % 4 == 0) && ((uintptr_t)q & 15) == 0 &&
                      ((uintptr_t)k & 15) == 0 && (!ch || ((uintptr_t)pre & 15) == 0);
-    const size_t smem = cw_scan_smem(2 * sizeof(float) * (size_t)(2 * RC * Dk + (ch ? RC * Dk : (form == 1 || form == 4 ? 2 * RC : 0)) + RC * JB), rows);
+    const size_t smem = cw_scan_smem(2 * sizeof(float) * (size_t)(2 * RC * Dk + (ch ? RC * Dk : (form == 1 || form == 4 ? 2 * RC : 0)) + RC * JB), rows,
+                                     (long long)grid.x * H);
     const int which = wide && Dk % RS == 0 ? log_ip : 6;
     static size_t allowed[5][7] = {};
     using Kernel = void (*)(const float*, int, const float*, int, const float*, int, const float*, int, const float*, const float*,

@@ -475,7 +475,8 @@ extern "C" int cw_delta_scan(const float* q, int ldq, const float* k, int ldk, c
     const int wide = Dk % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ((uintptr_t)q & 15) == 0 && ((uintptr_t)k & 15) == 0 &&
                      (head_decay || (lda % 4 == 0 && ((uintptr_t)a & 15) == 0));
     const bool vec = wide && Dk % DS == 0;
-    const size_t smem = cw_scan_smem(2 * sizeof(float) * (size_t)((head_decay ? 2 : 3) * DC * Dk + DC * JB + (head_decay ? 2 : 1) * DC), rows);
+    const size_t smem = cw_scan_smem(2 * sizeof(float) * (size_t)((head_decay ? 2 : 3) * DC * Dk + DC * JB + (head_decay ? 2 : 1) * DC), rows,
+                                     (long long)grid.x * H);
     using Kernel = void (*)(const DeltaScanArgs);
     static const Kernel kernels[2][7] = {
         {delta_scan_kernel<1, false>, delta_scan_kernel<2, false>, delta_scan_kernel<4, false>, delta_scan_kernel<8, false>,

@@ -36,6 +36,7 @@ _SIGNATURES: dict[str, list] = {
     "cw_causal_conv": [P, I, P, P, P, LL, LL, P, P, P, P, I, I, I, P],
     "cw_carry_rows": [P, I, P, LL, LL, P, P, P, I, I, I, I, P],
     "cw_recurrence_scan": [I, P, I, P, I, P, I, P, I, P, P, P, P, LL, LL, P, P, P, I, I, I, I, I, P, I, F, I, P],
+    "cw_chunk_scan": [I, P, I, P, I, P, I, P, I, P, I, P, F, I, P, LL, LL, P, P, P, I, I, I, I, I, P, P, P, I, I, I, LL, I, P],
     "cw_sigmoid_power_decay": [P, I, I, I, F, P],
     "cw_activation_cols": [P, I, I, I, I, I, P],
     "cw_recurrence_coefficients": [I, P, I, P, P, P, I, I, P],

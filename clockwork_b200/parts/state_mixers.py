@@ -80,6 +80,12 @@ from .registry import register_mixer
 from .rotary import check_rotary, rotary_tables
 
 
+def takes_chunks(mixer: Mixer, ctx: StepContext) -> bool:
+    """Whether a scan may take a portion's tokens a chunk at a time: in bfloat16 steps that hold portions.  (A float32 run's bits do
+    not depend on how a prompt was cut into steps; a chunk of one token costs what sixteen do.)"""
+    return mixer.dtype == torch.bfloat16 and not ctx.all_single_token
+
+
 class Mamba2Mixer(Mixer):
     graph_safe = True
     graph_safe_portions = True
@@ -134,7 +140,7 @@ class Mamba2Mixer(Mixer):
             rec_ops.FORM_STEP_SIZE, q=xbc[:, inner + gn :], k=xbc[:, inner : inner + gn], v=xbc[:, :inner],
             pre=proj[:, inner + self.channels :], p0=self.dt_bias, p1=self.a_log, p2=self.skip, view=view,
             offset=self.scan_offset, ctx=ctx, heads=self.heads, dk=self.state_size, dv=self.vdim,
-            heads_per_group=self.heads // self.groups)
+            heads_per_group=self.heads // self.groups, chunks=takes_chunks(self, ctx))
         out = rec_ops.gated_group_norm(y, proj[:, :inner], self.norm_w, self.norm_groups, self.eps, True, self.dtype)
         return self.o.add_or_defer(out, stream)
 
@@ -285,7 +291,7 @@ class DecayLinearMixer(_LinearAttention):
         proj = rec_ops.activation_cols_(self.w_in.to_float32(x), 2 * self.qk + self.inner, rec_ops.ACT_SILU)  # q, k, v; not the gate
         q, k, v, g = self._split(proj)
         o = rec_ops.recurrence_scan(rec_ops.FORM_HEAD_DECAY, q=q, k=k, v=v, pre=None, p0=self.decay, p1=None, p2=None, view=view,
-                                    offset=0, ctx=ctx, heads=self.heads, dk=self.dim, dv=self.vdim)
+                                    offset=0, ctx=ctx, heads=self.heads, dk=self.dim, dv=self.vdim, chunks=takes_chunks(self, ctx))
         return rec_ops.gated_group_norm(o, g, self.norm_w, 1, self.eps, False, self.dtype, gate=rec_ops.GATE_SIGMOID)
 
 
@@ -313,7 +319,8 @@ class RetentionMixer(_LinearAttention):
                               self.rot_amplitude)
         q, k, v, g = self._split(proj)
         o = rec_ops.recurrence_scan(rec_ops.FORM_HEAD_DECAY, q=q, k=k, v=v, pre=None, p0=self.decay, p1=None, p2=None, view=view,
-                                    offset=0, ctx=ctx, heads=self.heads, dk=self.dim, dv=self.vdim, q_scale=self.dim ** -0.5)
+                                    offset=0, ctx=ctx, heads=self.heads, dk=self.dim, dv=self.vdim, q_scale=self.dim ** -0.5,
+                                    chunks=takes_chunks(self, ctx))
         return rec_ops.gated_group_norm(o, g, None, self.heads, self.eps, False, self.dtype, gate=rec_ops.GATE_SILU)
 
 
@@ -435,7 +442,7 @@ class HeadDeltaMixer(_DeltaRule):
         proj = self.w_in.to_float32(x)  # [N, q | k | v | gate | beta | decay], float32
         o = rec_ops.head_delta(proj, self.conv_w, proj[:, c + i : c + i + h], proj[:, c + i + h :], self.dt_bias, self.a_log, view,
                                self.scan_offset, self.conv_offset, ctx, self.kv_heads, h, self.dim, self.vdim, self.UNIT_EPS,
-                               self.dim ** -0.5)
+                               self.dim ** -0.5, chunks=takes_chunks(self, ctx))
         return rec_ops.gated_group_norm(o, proj[:, c : c + i], self.norm_w, h, self.eps, False, self.dtype, gate=rec_ops.GATE_SILU,
                                         shared_weight=True)
 
@@ -520,7 +527,7 @@ class MatrixMemoryMixer(Mixer):
         coef = rec_ops.gate_scan(proj[:, at : at + h], proj[:, at + h :], self.bias_i, self.bias_f, self.cap, view, self.max_offset, ctx, h)
         y = rec_ops.recurrence_scan(rec_ops.FORM_GATED_WITH_KEY_SUM, q=proj[:, :qk], k=proj[:, qk : 2 * qk], v=proj[:, 2 * qk : 2 * qk + inner],
                                     pre=coef, p0=None, p1=None, p2=None, view=view, offset=self.scan_offset, ctx=ctx, heads=h, dk=self.dim,
-                                    dv=self.vdim + 1, q_scale=self.dim ** -0.5)
+                                    dv=self.vdim + 1, q_scale=self.dim ** -0.5, chunks=takes_chunks(self, ctx))
         return rec_ops.memory_norm(y, coef[:, 2 * h :], proj[:, 2 * qk + inner : at], self.norm_w, h, self.vdim, self.eps, self.dtype)
 
     def mix(self, ctx: StepContext, x, view: StateView):
