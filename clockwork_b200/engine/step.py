@@ -14,6 +14,7 @@ context lengths and the rows whose logits are wanted, uploaded in one copy from 
 
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -35,6 +36,31 @@ class StepEntry:
 
 def _pad4(n: int) -> int:
     return (n + 3) & ~3
+
+
+def _flat(lists) -> np.ndarray:
+    """Lists of numbers one after the other.  (Converted a list at a time: a step that asked for logits at every place of a
+    2,048-token prompt spent 0.5 of its 0.6 ms of host time in loops over single numbers, more than the layer it fed took.)"""
+    flat = array("q")
+    for numbers in lists:
+        n = len(flat)
+        try:
+            flat.extend(iter(numbers))
+        except TypeError:  # numbers that are whole but no integers to Python
+            del flat[n:]
+            flat.extend(int(x) for x in numbers)
+    return np.frombuffer(flat, dtype=np.int64)
+
+
+def _wanted_places(entries: list[StepEntry]) -> tuple[np.ndarray, list[int]]:
+    """The entries' wanted places one after the other, and how many each has; refuses places outside an entry's tokens."""
+    flat, counts = _flat(e.want for e in entries), [len(e.want) for e in entries]
+    if len(flat) and ((flat < 0) | (flat >= np.repeat([len(e.tokens) for e in entries], counts))).any():
+        for e in entries:
+            bad = [w for w in e.want if not 0 <= w < len(e.tokens)]
+            if bad:
+                raise ValueError(f"request {e.request_id!r}: wanted places {bad} outside its {len(e.tokens)} tokens")
+    return flat, counts
 
 
 @dataclass
@@ -67,7 +93,7 @@ class StepBuilder:
 
     def requests_of(self, entries: list[StepEntry]) -> list:
         """The entries' requests, with room reserved for the tokens they bring; refuses a request that
-        appears twice and wanted places outside an entry's tokens."""
+        appears twice."""
         cache = self.cache
         reqs = []
         seen = set()
@@ -78,13 +104,11 @@ class StepBuilder:
             req = cache.get(e.request_id)
             cache.reserve(req, req.num_computed + len(e.tokens))
             reqs.append(req)
-            bad = [w for w in e.want if not 0 <= w < len(e.tokens)]
-            if bad:
-                raise ValueError(f"request {e.request_id!r}: wanted places {bad} outside its {len(e.tokens)} tokens")
         return reqs
 
     def prepare(self, entries: list[StepEntry]) -> PreparedStep:
         cache = self.cache
+        wanted, counts = _wanted_places(entries)
         reqs = self.requests_of(entries)
         S = len(entries)
         q_lens = [len(e.tokens) for e in entries]
@@ -114,14 +138,14 @@ class StepBuilder:
             o, size = seg[name]
             h[o : o + size] = values
 
-        put("tokens", np.fromiter((t for e in entries for t in e.tokens), dtype=np.int64, count=N))
+        put("tokens", _flat(e.tokens for e in entries))
         put("positions", np.concatenate([np.arange(s, s + q, dtype=np.int32) for s, q in zip(starts, q_lens)]))
         put("tok_seq", np.repeat(np.arange(S, dtype=np.int32), q_lens))
         q_start = np.zeros(S + 1, dtype=np.int32)
         np.cumsum(q_lens, out=q_start[1:])
         put("q_start", q_start)
         put("ctx_lens", ctx_lens)
-        put("rows", [int(q_start[i]) + w for i, e in enumerate(entries) for w in e.want])
+        put("rows", wanted + np.repeat(q_start[:S], counts))
         put("state", [r.state_slot if r.state_slot is not None else 0 for r in reqs])
         ps = cache.page_size
         for g in range(G):
@@ -446,8 +470,8 @@ class PortionGraph:
             for key, (_, fill, _) in self._arrays.items():
                 h[("array", key)][:] = fill([], [])
 
-    def fill(self, cache: CacheManager, entries: list[StepEntry], reqs: list) -> list[int]:
-        """The step's description written into the pinned buffer.  Returns the context lengths after the step."""
+    def fill(self, cache: CacheManager, entries: list[StepEntry], reqs: list, wants: tuple) -> list[int]:
+        """``wants``: see ``_wanted_places``.  The step's description written into the pinned buffer.  Returns the context lengths after the step."""
         self._uploaded.synchronize()  # the last upload has left the pinned buffer
         h, ps = self.h, cache.page_size
         S = len(entries)
@@ -455,31 +479,37 @@ class PortionGraph:
         N = sum(q_lens)
         starts = [r.num_computed for r in reqs]
         ctx_lens = [a + q for a, q in zip(starts, q_lens)]
-        rows = [w for e in entries for w in e.want]
-        R = len(rows)
-        h["tokens"][:N] = np.fromiter((t for e in entries for t in e.tokens), dtype=np.int64, count=N)
-        h["positions"][:N] = np.concatenate([np.arange(a, a + q, dtype=np.int32) for a, q in zip(starts, q_lens)])
+        R = sum(len(e.want) for e in entries)
+        h["tokens"][:N] = _flat(e.tokens for e in entries)
         h["tok_seq"][:N] = np.repeat(np.arange(S, dtype=np.int32), q_lens)
         q_start = np.zeros(S + 1, dtype=np.int32)
         np.cumsum(q_lens, out=q_start[1:])
         h["q_start"][: S + 1] = q_start
+        h["positions"][:N] = np.arange(N) + np.repeat(np.array(starts) - q_start[:S], q_lens)
         h["ctx_lens"][:S] = ctx_lens
-        h["rows"][:R] = [int(q_start[i]) + w for i, e in enumerate(entries) for w in e.want]
+        h["rows"][:R] = wants[0] + np.repeat(q_start[:S], wants[1])
         h["state"][:S] = [r.state_slot if r.state_slot is not None else cache.state.scratch_slot for r in reqs]
         for g in range(len(cache.groups)):
-            slots, tables = h[f"slots{g}"], h[f"tables{g}"]
+            slots, tables, every = h[f"slots{g}"], h[f"tables{g}"], cache.groups[g].every
+            # (a request may hold pages for tokens far beyond this step's: the scheduler reserves a
+            # whole prompt's at admission; the step reads the table up to its context bound only)
+            held = [min(len(r.tables[g]), self.max_blocks) for r in reqs]
+            flat = _flat(r.tables[g][:k] for r, k in zip(reqs, held)).astype(np.int32)
             tables[:S] = NO_PAGE
+            o = 0
             for i, r in enumerate(reqs):
-                table = np.asarray(r.tables[g], dtype=np.int32)
-                # (a request may hold pages for tokens far beyond this step's: the scheduler reserves a
-                # whole prompt's at admission; the step reads the table up to its context bound only)
-                held = min(len(table), self.max_blocks)
-                tables[i, :held] = table[:held]
-                pos = np.arange(starts[i], ctx_lens[i], dtype=np.int32) // cache.groups[g].every
-                pages = table[pos // ps]
-                if (pages == NO_PAGE).any():
+                table = r.tables[g]
+                tables[i, : held[i]] = flat[o : o + held[i]]
+                o += held[i]
+                first, last = starts[i] // every // ps, (ctx_lens[i] - 1) // every // ps
+                pages = table[first : last + 1]
+                if NO_PAGE in pages:
                     raise RuntimeError(f"request {r.request_id!r}: a token lands in a page that was given back")
-                slots[q_start[i] : q_start[i + 1]] = pages * ps + pos % ps
+                if q_lens[i] == 1:
+                    slots[q_start[i]] = pages[0] * ps + starts[i] // every % ps
+                else:
+                    pos = np.arange(starts[i], ctx_lens[i], dtype=np.int32) // every
+                    slots[q_start[i] : q_start[i + 1]] = np.array(pages, dtype=np.int32)[pos // ps - first] * ps + pos % ps
         self._write_padding(cache, N, S, R)
         single_ctx = [c for q, c in zip(q_lens, ctx_lens) if q == 1]
         for name, rule in self._scalar_rules.items():
@@ -627,7 +657,8 @@ class ModelRunner:
     # size (the gaps between launches cost a long step about 5 %; more padding than that would cost more).
     # The small buckets are those of the products' token tiles: a prompt of 8 to 64 tokens, or the rest of one
     # behind a prefix-cache hit, costs 1.4 to 1.8 ms at the 1.5B sizes instead of the 2.2 ms of 128 tokens.
-    PORTION_TOKEN_BUCKETS = (16, 32, 64, 128, 192, 256, 384, 512, 768, 1024)
+    # (From 512 on every 128: a step of 545 tokens padded to 768 ran 0.54 ms through a layer of the 7B sizes, 0.52 padded to 640.)
+    PORTION_TOKEN_BUCKETS = (16, 32, 64, 128, 192, 256, 384, 512, 640, 768, 896, 1024)
     PORTION_MAX_TOKENS = 4096
     PORTION_LONG_STEP = 256
     PORTION_LONG_WASTE = 0.04
@@ -699,6 +730,7 @@ class ModelRunner:
         return made
 
     def _step_with_portion_graph(self, entries: list[StepEntry], key: tuple) -> torch.Tensor | None:
+        wants = _wanted_places(entries)
         reqs = self.builder.requests_of(entries)
         graph = self.portion_graphs.pop(key, None)
         if graph is None:
@@ -707,7 +739,7 @@ class ModelRunner:
                 del self.portion_graphs[next(iter(self.portion_graphs))]
             graph = PortionGraph(self, *key)
         self.portion_graphs[key] = graph  # (the dictionary's order is the order of last use)
-        ctx_lens = graph.fill(self.cache, entries, reqs)
+        ctx_lens = graph.fill(self.cache, entries, reqs, wants)
         logits = graph.launch()
         self.builder.commit(PreparedStep(None, None, None, reqs, ctx_lens))
         self.graph_kernel_launches += graph.kernels
