@@ -32,6 +32,9 @@ struct StepFromStateParams {
     int* ctx_lens;    // [B] out: position + 1
     int* tok_seq;     // [B] out: the row itself, or -1 for padding
     float* temperature; int* top_k; float* top_p; float* uniform;  // [B] out
+    // [B] out (null: not wanted): the row of the mixers' own states, row_slot or for padding scratch_slot.  (Made here and not by
+    // kernels of torch's, four launches that a single-token step of a recurrent layer spent a twelfth of its time in.)
+    long long* state_rows; int scratch_slot;
     int* status;
 };
 
@@ -57,6 +60,7 @@ __global__ void step_from_state_kernel(const StepFromStateParams p) {
     const int slot = p.row_slot[r];
     if (slot < 0 || slot >= p.num_slots) {
         if (slot >= p.num_slots) cw_report(p.status, CW_ST_ROW_RANGE, r, slot);
+        if (p.state_rows != nullptr) p.state_rows[r] = p.scratch_slot;
         p.tokens[r] = 0;
         p.positions[r] = 0;
         p.ctx_lens[r] = 0;
@@ -68,6 +72,7 @@ __global__ void step_from_state_kernel(const StepFromStateParams p) {
         for (int g = 0; g < p.num_groups; ++g) p.kv_slots[g][r] = -1;
         return;
     }
+    if (p.state_rows != nullptr) p.state_rows[r] = slot;
     int* col = p.state + slot;
     if (p.fresh[r]) {
         for (int f = 0; f < CW_RS_FIELDS; ++f) col[f * p.num_slots] = p.fresh_values[f * p.B + r];
@@ -104,7 +109,7 @@ extern "C" int cw_step_from_state(const int* row_slot, int* fresh, const int* fr
                                   const int* group_pages, const int* group_every,
                                   const int* const* tables, int* const* kv_slots, int* tokens, int* positions,
                                   int* ctx_lens, int* tok_seq, float* temperature, int* top_k, float* top_p,
-                                  float* uniform, int* status, cudaStream_t stream) {
+                                  float* uniform, long long* state_rows, int scratch_slot, int* status, cudaStream_t stream) {
     if (B == 0) return CW_OK;
     if (B < 0 || num_slots <= 0 || page_size <= 0 || max_blocks <= 0 || num_groups < 0 || num_groups > CW_RS_MAX_GROUPS)
         return CW_ERR_BAD_SIZE;
@@ -121,6 +126,7 @@ extern "C" int cw_step_from_state(const int* row_slot, int* fresh, const int* fr
     }
     p.tokens = tokens; p.positions = positions; p.ctx_lens = ctx_lens; p.tok_seq = tok_seq;
     p.temperature = temperature; p.top_k = top_k; p.top_p = top_p; p.uniform = uniform; p.status = status;
+    p.state_rows = state_rows; p.scratch_slot = scratch_slot;
     const int threads = 64;
     return cw_launch(step_from_state_kernel, dim3((B + threads - 1) / threads), dim3(threads), 0, stream, 1, p);
 }

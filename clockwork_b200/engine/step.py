@@ -282,13 +282,11 @@ class DecodeGraph:
         as_float = lambda name: view(name).view(torch.float32)  # noqa: E731
 
         def run():
-            if state_rows is not None:
-                row_slot = view("row_slot")
-                state_rows.copy_(torch.where(row_slot < 0, cache.state.scratch_slot, row_slot))
             ops.step_from_state(view("row_slot"), view("fresh"), view("fresh_values").view(F, batch), state, tables, kv_slots,
                                 cache.page_size, [group.allocator.num_pages for group in cache.groups], view("tokens"), view("positions"), view("ctx_lens"),
                                 view("tok_seq"), as_float("temperature"), view("top_k"), as_float("top_p"),
-                                as_float("uniform"), runner.status, every=[group.every for group in cache.groups])
+                                as_float("uniform"), runner.status, every=[group.every for group in cache.groups],
+                                state_rows=state_rows, scratch_slot=cache.state.scratch_slot)
             # the logits of every row stay readable after a replay (trace replay reads them; generation
             # reads the sampled tokens only)
             logits = self.logits = model.forward(ctx, view("tokens"), view("rows"))

@@ -499,13 +499,14 @@ def step_from_state(row_slot: torch.Tensor, fresh: torch.Tensor, fresh_values: t
                     tables: list[torch.Tensor], kv_slots: list[torch.Tensor], page_size: int, num_pages,
                     tokens: torch.Tensor, positions: torch.Tensor, ctx_lens: torch.Tensor, tok_seq: torch.Tensor,
                     temperature: torch.Tensor, top_k: torch.Tensor, top_p: torch.Tensor, uniform: torch.Tensor,
-                    status: torch.Tensor, every=None) -> None:
+                    status: torch.Tensor, every=None, state_rows: torch.Tensor | None = None, scratch_slot: int = 0) -> None:
     """The inputs of a single-token step from the per-request state table: row r of the step belongs to
     the request in slot ``row_slot[r]`` (< 0: padding).  Rows flagged in ``fresh`` first take their column
     from ``fresh_values`` [fields, B] (the flag is cleared).  Written: the token to feed, position,
     context length, the row's request index, the cache slot per page group (from ``tables`` [B, max_blocks]
     each), and the sampling parameters with the draw's uniform number.  ``num_pages``: the pages of every group's
-    pool (one number for all, or one per group); ``every``: per group, positions per cache row (None: one)."""
+    pool (one number for all, or one per group); ``every``: per group, positions per cache row (None: one).  ``state_rows``
+    (int64 [B]): also the row of the mixers' own states, ``row_slot`` or for padding ``scratch_slot``."""
     import ctypes
 
     b = row_slot.shape[0]
@@ -518,6 +519,10 @@ def step_from_state(row_slot: torch.Tensor, fresh: torch.Tensor, fresh_values: t
     _need(state, torch.int32, "state", 2)
     if state.shape[0] != len(REQUEST_STATE_FIELDS) or tuple(fresh_values.shape) != (len(REQUEST_STATE_FIELDS), b):
         raise ValueError("state must be [fields, slots] and fresh_values [fields, B]")
+    if state_rows is not None:
+        _need(state_rows, torch.int64, "state_rows", 1)
+        if state_rows.shape[0] != b:
+            raise ValueError("state_rows needs an entry per row")
     if len(tables) != len(kv_slots):
         raise ValueError("one block table and one slot array per page group")
     max_blocks = 1
@@ -539,7 +544,7 @@ def step_from_state(row_slot: torch.Tensor, fresh: torch.Tensor, fresh_values: t
         max(pages, default=1), g, ctypes.cast(page_counts, ctypes.c_void_p), ctypes.cast(strides, ctypes.c_void_p),
         ctypes.cast(table_ptrs, ctypes.c_void_p), ctypes.cast(slot_ptrs, ctypes.c_void_p), _ptr(tokens),
         _ptr(positions), _ptr(ctx_lens), _ptr(tok_seq), _ptr(temperature), _ptr(top_k), _ptr(top_p), _ptr(uniform),
-        _ptr(status), _stream()), "step_from_state")
+        _ptr(state_rows), int(scratch_slot), _ptr(status), _stream()), "step_from_state")
 
 
 _sample_work: dict[int, torch.Tensor] = {}

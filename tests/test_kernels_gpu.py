@@ -1140,3 +1140,20 @@ def test_attention_decode_fused_position_and_store(ops, status, fast, nh, nkv, h
     ops.raise_on_status(status)
     assert torch.equal(k2, k1) and torch.equal(v2, v1)
     assert torch.equal(got, want)
+
+
+def test_step_from_state_names_the_rows_of_the_mixers_states(ops, status):
+    rows = torch.tensor([2, -1, 0, 5, -1], dtype=torch.int32, device=DEV)
+    b, fields = 5, len(ops.REQUEST_STATE_FIELDS)
+    ints = [torch.zeros(b, dtype=torch.int32, device=DEV) for _ in range(6)]
+    floats = [torch.zeros(b, device=DEV) for _ in range(3)]
+    state_rows = torch.full((b,), -7, dtype=torch.int64, device=DEV)
+    ops.step_from_state(rows, ints[0], torch.zeros(fields, b, dtype=torch.int32, device=DEV), torch.zeros(fields, 6, dtype=torch.int32, device=DEV),
+                        [], [], 16, 1, ints[1], ints[2], ints[3], ints[4], floats[0], ints[5], floats[1], floats[2], status,
+                        state_rows=state_rows, scratch_slot=9)
+    ops.raise_on_status(status)
+    assert state_rows.tolist() == [2, 9, 0, 5, 9]
+    with pytest.raises(ValueError, match="an entry per row"):
+        ops.step_from_state(rows, ints[0], torch.zeros(fields, b, dtype=torch.int32, device=DEV), torch.zeros(fields, 6, dtype=torch.int32, device=DEV),
+                            [], [], 16, 1, ints[1], ints[2], ints[3], ints[4], floats[0], ints[5], floats[1], floats[2], status,
+                            state_rows=state_rows[:3], scratch_slot=9)
