@@ -42,7 +42,7 @@
 // finite values, so they cannot leak.  Every wait is bounded (CW_ST_WAIT_TIMEOUT in the status
 // words, then the kernel frees TMEM and returns).
 #include <type_traits>
-#include "tc_common.cuh"
+#include "tc_attention.cuh"
 
 #define AQ 128  // query rows per CTA
 #define AK 128  // keys per tile
@@ -103,73 +103,6 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
         : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-// Descriptor of an MN-major operand with the 128-byte swizzle: rows of the K dimension are 128 bytes
-// (64 contiguous elements of the MN dimension), groups of 8 rows are `group_bytes` apart (stride byte
-// offset) and the next 64 elements of the MN dimension lie `mn_block_bytes` further (leading byte offset).
-__device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t addr, uint32_t mn_block_bytes, uint32_t group_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr >> 4) & 0x3FFF);
-    d |= (uint64_t)((mn_block_bytes >> 4) & 0x3FFF) << 16;
-    d |= (uint64_t)((group_bytes >> 4) & 0x3FFF) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-__device__ __forceinline__ float ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
-        ::"r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-          "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])),
-          "r"(__float_as_uint(v[7])), "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])),
-          "r"(__float_as_uint(v[11])), "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])),
-          "r"(__float_as_uint(v[15]))
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-// This lane's row of an accumulator in tensor memory times alpha (rare: a rolled loop over 16 columns
-// at a time, so that it takes few registers from the softmax loop around it).
-template <int COLS>
-__device__ __forceinline__ void rescale_o(uint32_t taddr, float alpha) {
-#pragma unroll 1
-    for (int c = 0; c < COLS; c += 16) {
-        float v[16];
-        tmem_ld16(taddr + c, v);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) v[i] *= alpha;
-        tmem_st16(taddr + c, v);
-    }
-}
-// D (+)= A B with A in tensor memory: lane i holds row i, a 32-bit column two consecutive bfloat16 of the
-// inner dimension (the lower half first), so 16 of them take 8 columns.
-__device__ __forceinline__ void umma_bf16_a_tmem(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 // A named barrier of n threads that also tells every one of them whether all came with `pred` true.
 __device__ __forceinline__ bool bar_and(int id, int n, bool pred) {
     uint32_t all;
@@ -179,11 +112,6 @@ __device__ __forceinline__ bool bar_and(int id, int n, bool pred) {
                  : "memory");
     return all != 0;
 }
-__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
-    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *reinterpret_cast<uint32_t*>(&v);
-}
-
 template <int HD>
 __global__ void __launch_bounds__(A_THREADS, 1)  // (18 warps: five on one scheduler, whose 16,384 registers allow 96 per thread)
 attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,

@@ -14,7 +14,7 @@
 //                        the cache row of the token's slot; rotation of the queries' rotated parts
 //   cw_latent_attention  causal attention of a flat batch (prompt portions beside single tokens) over the
 //                        paged rows; float32 scores, weights and accumulation in both run precisions
-#include "request_tiles.cuh"
+#include "latent_attention.cuh"
 #include "rotation.cuh"
 
 // down [N, rank + rot] (row stride ldd, float32: the projection's output); q [N, H*(dim + rot)] (row stride ldq, QT: float32
@@ -279,22 +279,6 @@ __device__ __forceinline__ void lt_mma(float (&c)[4], const unsigned (&a)[4], un
 __device__ __forceinline__ unsigned lt_pack(bf16 a, bf16 b) {
     return (unsigned)__bfloat16_as_ushort(a) | ((unsigned)__bfloat16_as_ushort(b) << 16);
 }
-
-struct LatentArgs {
-    const bf16* qa;           // [N*H, D]
-    bf16* out;                // [N*H, rank]
-    const bf16* cache;        // [slots, D]
-    const int* block_tables;  // [S, max_blocks]
-    const int* tok_seq;       // [N], < 0: padding
-    const int* positions;     // [N]
-    const int* q_start;       // [S + 1]
-    const float* sink;        // [H] or null
-    int N, S, H, rank, rot, page_size, max_blocks, num_pages;
-    float scale;
-    int parts;
-    float* partial;           // parts > 1: [parts, N*H, rank] sums, then [parts, N*H, 2] running maxima and denominators
-    int* status;
-};
 
 template <int MT>
 struct LatentTile {
@@ -647,7 +631,8 @@ latent_merge_kernel(const float* __restrict__ partial, const int* __restrict__ t
 }
 
 static int g_latent_mma = 1;
-extern "C" int cw_latent_attention_set_mma(int on) { g_latent_mma = on ? 1 : 0; return CW_OK; }
+// 1 (the default): the tensor-core kernels where they take the sizes; 2: the mma.sync kernel alone; 0: the CUDA-core kernel alone.
+extern "C" int cw_latent_attention_set_mma(int on) { g_latent_mma = on < 0 || on > 2 ? 1 : on; return CW_OK; }
 
 template <int MT>
 static int launch_latent_mma(const LatentArgs& a, cudaStream_t stream) {
@@ -688,6 +673,9 @@ extern "C" int cw_latent_attention(const void* qa, void* out, const void* cache,
         ((uintptr_t)cache & 15) == 0 && ((uintptr_t)out & 3) == 0) {
         const LatentArgs args = {(const bf16*)qa, (bf16*)out, (const bf16*)cache, block_tables, tok_seq, positions, q_start, sink, N, S, H,
                                  rank, rot, page_size, max_blocks, num_pages, scale, parts, partial, status};
+        // (in one chain of key tiles; the mma.sync kernel adds up parts: 2 parts, 256 tokens behind 8,192, 541 us there and 476 here;
+        //  3 parts, 128 tokens, 361 us there, and the chain would be as long as before)
+        if (!few_rows && parts <= 2 && g_latent_mma == 1 && latent_tc_takes(args)) return latent_tc_run(args, stream);
         return few_rows ? launch_latent_mma<1>(args, stream) : launch_latent_mma<4>(args, stream);
     }
     if (rank > LA_CH * LA_NC || (H + LA_HB - 1) / LA_HB > 65535) return CW_ERR_UNSUPPORTED;
