@@ -35,7 +35,7 @@
 // Scores, weights, the softmax statistics and the weighted sums are float32 in both run precisions; T names
 // the type of the product's output and of the cache.  A token's result depends on its position alone: keys
 // are taken in tiles that start at the window's first position, in order, whatever else the step holds.
-#include "request_tiles.cuh"
+#include "window_attention.cuh"
 #include "rotation.cuh"
 
 #define WA_MAX_COLS 16  // output columns per thread
@@ -315,43 +315,6 @@ extern "C" int cw_pool_rows(const void* cache, const int* block_tables, int max_
     return CW_ERR_BAD_DTYPE;
 }
 
-struct WindowAttentionArgs {
-    const void* q;            // [N, ldq]: head h's query at columns h*dk ..
-    int ldq;
-    const void* cache;        // [rows, G, dk + dv]
-    const int* block_tables;  // [S, max_blocks]
-    int max_blocks, page_size, num_pages;
-    const int* positions;     // [N]
-    const int* tok_seq;       // [N], < 0: padding
-    int H, G, dk, dv, window;
-    float scale;
-    const float* head_scale;  // [H] or null: multiplied into the score
-    const float* talk;        // [H, H] or null: score_h <- sum_g talk[h, g] score_g
-    const float* head_bias;   // [H] or null: added to the mixed score
-    int sigmoid_weights;      // 0: softmax over the visible keys; 1: sigmoid of each score, not normalised
-    int blocked;              // 0: p sees the last `window` positions; 1: p sees its own block of `window` positions up to itself
-    const float* sink;        // [H] or null: a logit per head that counts once in the softmax's denominator
-    void* out;                // [N, H*dv]
-    int tile;                 // keys per tile (<= 32)
-    int parts, part_keys;     // a token's window in `parts` pieces of `part_keys` keys (a multiple of tile)
-    float* partial;           // parts > 1: [N, parts, H*dv + 2H] sums, running maxima and denominators
-    int* status;
-    // further switches (all off when zero or null)
-    float softcap;            // > 0: score <- softcap tanh(score / softcap)
-    const float* slopes;      // [H] or null: slopes[h] * (p - j) is taken off the score
-    float temp_coef;          // with temp_every > 0: the score of a query at position p is multiplied by
-    int temp_every;           //   1 + temp_coef ln(floor((p + 1) / temp_every) + 1)
-    const float* gate;        // [N, ldg] or null: head h's output is multiplied by sigmoid(gate[n * ldg + h])
-    int ldg;
-    int pool;                 // > 0: blocks of `pool` positions that end at or before p - window are seen as one row each
-    const void* pool_cache;   // [rows, G, dk + dv]: row b of a request is the mean of its positions b*pool .. b*pool + pool - 1
-    const int* pool_tables;   // [S, pool_max_blocks]
-    int pool_max_blocks, pool_pages;
-    int keep;                 // the sequence's first `keep` positions are seen by every later one
-    int voff;                 // where a head's value begins in its row (row width voff + dv; below dk: key and value overlap)
-    int gate_entries;         // 1: the gate has a number per output entry ([N, ldg], ldg >= H*dv) instead of one per head
-};
-
 // how many pooled blocks position p sees: those that end at or before p - window
 __device__ __forceinline__ int wa_pooled_blocks(int p, int window, int pool) {
     const int behind = p - window + 1;  // positions before the window
@@ -359,10 +322,6 @@ __device__ __forceinline__ int wa_pooled_blocks(int p, int window, int pool) {
 }
 // how many kept positions lie before a window that starts at `first`
 __device__ __forceinline__ int wa_kept_before(int first, int keep) { return min(first, keep); }
-__device__ __forceinline__ float wa_query_temperature(int p, float coef, int every) {
-    return every > 0 ? 1.f + coef * logf((float)((p + 1) / every + 1)) : 1.f;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(1024)
 window_attention_kernel(const WindowAttentionArgs a) {
@@ -988,7 +947,8 @@ window_attention_mma_kernel(const WindowMmaArgs args) {
 }
 
 static int g_window_mma = 1;
-extern "C" int cw_window_attention_set_mma(int on) { g_window_mma = on ? 1 : 0; return CW_OK; }
+// 1 (the default): the tensor-core kernels where they take the sizes; 2: the mma.sync kernel alone; 0: the CUDA-core kernel alone.
+extern "C" int cw_window_attention_set_mma(int on) { g_window_mma = on < 0 || on > 2 ? 1 : on; return CW_OK; }
 
 // The tensor-core form if it takes the sizes (returns 1 and launches), else 0; negative or positive: an error.
 static int window_attention_mma(const WindowAttentionArgs& base, const int* q_start, int S, int N, cudaStream_t stream, int* launched) {
@@ -1063,6 +1023,7 @@ extern "C" int cw_window_attention(const void* q, int ldq, const void* cache, co
                                           window, scale, head_scale, talk, head_bias, sigmoid_weights, blocked, sink, out, WM_BN, parts, 0,
                                           partial, status, softcap, slopes, temp_coef, temp_every, gate, ldg, pool, pool_cache, pool_tables,
                                           pool_max_blocks, pool_pages, keep, voff, gate_entries};
+        if (g_window_mma == 1 && q_start != nullptr && window_tc_takes(base, N)) return window_tc_run(base, q_start, S, N, stream);
         int launched = 0;
         const int rc = window_attention_mma(base, q_start, S, N, stream, &launched);
         if (rc != 0) return rc;
