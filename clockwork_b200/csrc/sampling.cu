@@ -229,37 +229,43 @@ extern "C" int cw_sample(const float* logits, const float* temperature, const in
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same rule over many thread blocks per row.
+// The same rule with a cluster of SR_CTAS thread blocks per row.
 //
 // sample_kernel above walks a row 65 times with one block: a vocabulary of 150,000 costs it a
-// millisecond and more.  Here a row is cut into SP_BLOCKS chunks, a block each, and the two searches
-// become radix selections over the order-preserving keys, 11 + 11 + 10 bits at a time, with
-// histograms in global memory that every pass's blocks add to and the next pass's blocks read:
+// millisecond and more.  Here every block of a cluster reads its part of the row once, keeps the
+// order-preserving keys in shared memory, and both searches run there: histograms over bins that fall
+// in the order of the keys, added up over the cluster through distributed shared memory, each search
+// going on inside the bin that it found until one key is left:
 //   top-k: counts per bin; the bin in which the count from the top reaches k is refined;
 //   top-p: mass per bin (of the keys top-k kept); the highest bin at which the mass from the top
 //          exceeds top_p * Z is refined; the key found is the lowest one kept.
+// The first bins are 1/73 wide in units of the logits (scaled by the temperature) and count down from
+// the row's maximum: leading bits of a key would put most of a vocabulary into a handful of bins, whose
+// atomics then wait for one another.  The last of them takes all that is too far below to have any mass;
+// what falls there is summed in registers.  Later levels cut the range of the bin's keys in 2,048.
+// What can still be kept is moved together, in index order.  Under a top-k of at most SR_THREADS, first of all within each
+// block: the k-th largest of its threads' maxima bounds the row's k-th largest from below.  Then what lies in the first bin
+// found or above it: in one block's memory if it fits there (the other blocks are then done, and no barrier of the cluster
+// is left: top-k of 50 keeps some sixty logits), else within each block.
 // Masses are integers, exp(l - max) * 2^40 truncated: sums of integers do not depend on the order in
 // which blocks and threads add them up, so a row's token is the same on every run whatever the
 // scheduling (floating-point atomics would not give that), and the final walk along the row in index
-// order compares exact cumulative sums with u * total.  Workspace (zeroed before the first kernel):
-// per row SP_WORDS 64-bit words.
+// order compares exact cumulative sums with u * total.
+// What bounds it: the instructions of the first passes (37 keys a thread), then the latency of the barriers.
+// Measured (B200, 64 rows of 151,936 with top-k 50 and top-p 0.9): 62 us; a chain of eight kernels that
+// re-read the row from L2 and kept its histograms in global memory took 224; one row: 21 and 68.
+// Rows of more than SR_CTAS * SR_STAGED logits are read again from global memory on each pass.
 // ---------------------------------------------------------------------------------------------
-#define SP_THREADS 256
-#define SP_BLOCKS 32
-#define SP_L1 2048  // bins of key bits 31..21
-#define SP_L2 2048  // bits 20..10
-#define SP_L3 1024  // bits 9..0
+#define SR_CTAS 8
+#define SR_THREADS 512
+#define SR_WARPS (SR_THREADS / 32)
+#define SR_BINS 2048
+#define SR_SLICE (SR_BINS / SR_CTAS)  // the bins that a block adds up for the cluster
+#define SR_RANGE 28.0f                // exp(-28) * 2^40 < 1: no mass beyond
+#define SR_STAGED 49152               // keys that a block holds in shared memory
+#define SR_LOADS 16                   // logits of a thread in flight
+#define SR_LIST 1024                  // and of those that are left, its own and the cluster's
 #define SP_MASS_ONE 1099511627776.0f  // 2^40
-// words of a row's workspace: [0] best (key << 32 | ~index), [1] Z, then counts (as 64-bit words, for one
-// kind of atomic) and masses per level, then the blocks' kept mass
-#define SP_CNT1 2
-#define SP_CNT2 (SP_CNT1 + SP_L1)
-#define SP_CNT3 (SP_CNT2 + SP_L2)
-#define SP_MASS1 (SP_CNT3 + SP_L3)
-#define SP_MASS2 (SP_MASS1 + SP_L1)
-#define SP_MASS3 (SP_MASS2 + SP_L2)
-#define SP_BLOCKSUM (SP_MASS3 + SP_L3)
-#define SP_WORDS (SP_BLOCKSUM + SP_BLOCKS)
 
 typedef unsigned long long u64;
 
@@ -272,303 +278,403 @@ __device__ __forceinline__ u64 mass_of(float l, float mx) { return (u64)(expf(l 
 struct SampleParams {
     const float* logits; size_t row_stride; int V;
     const float* temperature; const int* top_k; const float* top_p; const float* uniform;
-    u64* work;  // [rows][SP_WORDS]
     int* out; const int* row_slot; int* state; int num_slots;
+    int chunk, staged;  // logits of a block's part; whether its keys stay in shared memory
 };
 
-// Walks a histogram of `bins` 64-bit words from the top and finds the bin at which the running sum
-// first satisfies the rule: counts, sum >= want (the want-th largest key lies in it); masses, sum >
-// want.  Returns the bin (the lowest one if rounding lets none qualify) and leaves the sum above it in
-// *above.  Every thread of the block calls it and gets the same answer.  `scratch`: 16 words.
-__device__ int find_bin(const u64* hist, int bins, double want, bool strictly, u64* above, u64* scratch) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, per = bins / SP_THREADS;
-    // thread 0 owns the highest bins; an inclusive scan over the threads' sums, from the top down
-    u64 mine = 0;
-    for (int j = 0; j < per; ++j) mine += hist[bins - 1 - (tid * per + j)];
-    u64 incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const u64 n = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += n;
-    }
-    if (lane == 31) scratch[warp] = incl;
-    if (tid == 0) scratch[8] = (u64)0xffffffffu;  // the first thread whose sum qualifies
-    __syncthreads();
-    u64 before = 0;
-    for (int w = 0; w < warp; ++w) before += scratch[w];
-    incl += before;
-    const bool ok = strictly ? (double)incl > want : (double)incl >= want;
-    if (ok) atomicMin((unsigned*)&scratch[8], (unsigned)tid);
-    __syncthreads();
-    const int owner = (int)(unsigned)scratch[8];
-    if (tid == (owner < SP_THREADS ? owner : SP_THREADS - 1)) {
-        u64 run = incl - mine;
-        int bin = 0;
-        bool found = false;
-        for (int j = 0; j < per && !found; ++j) {
-            const int c = bins - 1 - (tid * per + j);
-            const u64 next = run + hist[c];
-            if (strictly ? (double)next > want : (double)next >= want) {
-                bin = c;
-                found = true;
-            } else {
-                run = next;
-            }
-        }
-        if (!found) {  // (rounding: take the lowest bin, with everything above it)
-            bin = 0;
-            run = incl - hist[0];
-        }
-        scratch[9] = (u64)bin;
-        scratch[10] = run;
-    }
-    __syncthreads();
-    const int bin = (int)scratch[9];
-    *above = scratch[10];
-    __syncthreads();
-    return bin;
+__device__ __forceinline__ void sr_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// The word of block `rank` that lies where `mine` does here.
+__device__ __forceinline__ unsigned sr_remote(const void* mine, unsigned rank) {
+    unsigned at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(mine)), "r"(rank));
+    return at;
+}
+__device__ __forceinline__ u64 sr_read(const u64* mine, unsigned rank) {
+    u64 v;
+    asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(sr_remote(mine, rank)) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned sr_read(const unsigned* mine, unsigned rank) {
+    unsigned v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(sr_remote(mine, rank)) : "memory");
+    return v;
 }
 
-// What a pass settles (the bits of the key found so far, and what is still wanted inside them) is kept
-// in the row's workspace, a pair of words per pass: pass n reads what pass n - 1 left and leaves its own
-// (every block computes the same; block 0 writes it).
-#define SP_STATE (SP_BLOCKSUM + SP_BLOCKS)
-#undef SP_WORDS
-#define SP_WORDS (SP_STATE + 16)
+struct SampleShared {
+    unsigned low[SR_BINS], high[SR_BINS];  // a bin's sum here, in two words (shared memory adds 32 bits at a time)
+    u64 slice[SR_SLICE];                   // the cluster's sums of this block's slice of the bins
+    u64 box[6];                            // for the other blocks: best, slice's sum, lowest and highest key, kept mass, keys left
+    u64 gathered[SR_CTAS];
+    u64 warp[SR_WARPS];
+    u64 above;
+    int bin, first;
+    unsigned list[2][SR_LIST], index[2][SR_LIST];  // the keys that are left and where they lie in the row: here, in the cluster
+};
 
-// PASS 0: best (largest key, first index) of every row, and top-k's counts of key bits 31..21.
-//      1, 2: top-k's counts of the next bits, inside the bins found so far.
-//      3: top-k settled (its lowest key kept: state word 6); top-p's masses of bits 31..21 and Z.
-//      4, 5: top-p's masses of the next bits.
-//      6: top-p settled (the lowest key kept at all: state word 12); the blocks' kept mass.
-template <int PASS>
-__global__ void __launch_bounds__(SP_THREADS)
-sample_pass_kernel(const SampleParams p) {
-    __shared__ u64 hist[SP_L1];
-    __shared__ u64 scratch[16];
+enum { SR_SUM, SR_MAX, SR_MIN };
+template <int OP>
+__device__ __forceinline__ u64 sr_combine(u64 a, u64 b) {
+    return OP == SR_SUM ? a + b : (OP == SR_MAX ? (a > b ? a : b) : (a < b ? a : b));
+}
+template <int OP>
+__device__ u64 sr_block(u64 v, SampleShared& s) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = sr_combine<OP>(v, __shfl_xor_sync(0xffffffffu, v, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) s.warp[threadIdx.x >> 5] = v;
+    __syncthreads();
+    u64 all = s.warp[0];
+#pragma unroll
+    for (int w = 1; w < SR_WARPS; ++w) all = sr_combine<OP>(all, s.warp[w]);
+    return all;
+}
+// Every block's word `b` of its box, in s.gathered; the blocks' boxes are written (a cluster barrier lies between).
+__device__ __forceinline__ void sr_gather(SampleShared& s, int b) {
+    __syncthreads();
+    if (threadIdx.x < SR_CTAS) s.gathered[threadIdx.x] = sr_read(&s.box[b], threadIdx.x);
+    __syncthreads();
+}
+// A value per thread combined over the cluster, through word `b` of the boxes (alone: over this block).
+template <int OP>
+__device__ u64 sr_cluster(u64 v, SampleShared& s, int b, bool alone) {
+    v = sr_block<OP>(v, s);
+    if (alone) return v;
+    if (threadIdx.x == 0) s.box[b] = v;
+    sr_cluster_sync();
+    sr_gather(s, b);
+    u64 all = s.gathered[0];
+#pragma unroll
+    for (int c = 1; c < SR_CTAS; ++c) all = sr_combine<OP>(all, s.gathered[c]);
+    return all;
+}
+__device__ __forceinline__ void sr_add(SampleShared& s, int bin, u64 v, bool mass) {
+    if (!mass) {  // (a count: no carry to look for)
+        atomicAdd(&s.low[bin], (unsigned)v);
+        return;
+    }
+    const unsigned lo = (unsigned)v, old = atomicAdd(&s.low[bin], lo);
+    const unsigned hi = (unsigned)(v >> 32) + (old + lo < old ? 1u : 0u);
+    if (hi != 0) atomicAdd(&s.high[bin], hi);
+}
+
+// The sums of the warps before this thread's and of its own up to it; *all: of the block.
+__device__ __forceinline__ u64 sr_scan(u64 v, SampleShared& s, u64* all) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const u64 n = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += n;
+    }
+    __syncthreads();
+    if (lane == 31) s.warp[warp] = v;
+    __syncthreads();
+    u64 sum = 0;
+    for (int w = 0; w < SR_WARPS; ++w) {
+        if (w < warp) v += s.warp[w];
+        sum += s.warp[w];
+    }
+    *all = sum;
+    return v;
+}
+
+// One level of a search: the blocks' histograms are complete; the first bin at which the running sum from bin 0
+// satisfies the rule: counts, sum >= want (the want-th largest key lies in it); masses, sum > want.  `fraction` >= 0:
+// want is that fraction of the whole sum.  What lies before the bin is taken off `want`; the histogram is cleared.
+// Every thread of the cluster gets the same answer.  `alone`: the histogram is this block's only.
+__device__ int sr_level(SampleShared& s, unsigned rank, bool alone, double& want, double fraction, bool strictly) {
+    constexpr int PER = SR_BINS / SR_THREADS;
+    const int tid = threadIdx.x;
+    auto enough = [&](u64 sum) { return strictly ? (double)sum > want : (double)sum >= want; };
+    u64 v[PER] = {}, before = 0;  // this thread's bins of those among which the answer is
+    int first_bin = tid * PER, bins = PER;
+    if (alone) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < PER; ++i) {
+            v[i] = (u64)s.low[tid * PER + i] + ((u64)s.high[tid * PER + i] << 32);
+            s.low[tid * PER + i] = s.high[tid * PER + i] = 0u;
+        }
+    } else {
+        sr_cluster_sync();
+        u64 mine = 0;
+        if (tid < SR_SLICE) {
+#pragma unroll
+            for (int c = 0; c < SR_CTAS; ++c) {
+                const int b = (int)rank * SR_SLICE + tid;
+                mine += (u64)sr_read(&s.low[b], c) + ((u64)sr_read(&s.high[b], c) << 32);
+            }
+            s.slice[tid] = mine;
+        }
+        const u64 sum = sr_block<SR_SUM>(mine, s);
+        if (tid == 0) s.box[1] = sum;
+        sr_cluster_sync();
+        for (int i = tid; i < SR_BINS; i += SR_THREADS) s.low[i] = s.high[i] = 0u;
+        sr_gather(s, 1);
+        if (fraction >= 0.) {
+            u64 all = 0;
+            for (int c = 0; c < SR_CTAS; ++c) all += s.gathered[c];
+            want = fraction * (double)all;
+        }
+        int slice = 0;
+        for (; slice < SR_CTAS - 1 && !enough(before + s.gathered[slice]); ++slice) before += s.gathered[slice];
+        if (tid < SR_SLICE) v[0] = sr_read(&s.slice[tid], slice);
+        first_bin = slice * SR_SLICE + tid;
+        bins = 1;
+    }
+    u64 mine = 0, all;
+    for (int i = 0; i < PER; ++i) mine += v[i];
+    if (tid == 0) s.first = SR_THREADS;
+    const u64 incl = before + sr_scan(mine, s, &all);
+    if (alone && fraction >= 0.) want = fraction * (double)all;
+    const int last = alone ? SR_THREADS - 1 : SR_SLICE - 1;
+    if (tid <= last && enough(incl)) atomicMin(&s.first, tid);
+    __syncthreads();
+    if (tid == min(s.first, last)) {  // (no bin qualifies, by rounding: the lowest, with everything before it)
+        u64 run = incl - mine;
+        int i = 0;
+        for (; i < bins - 1 && !enough(run + v[i]); ++i) run += v[i];
+        s.bin = first_bin + i;
+        s.above = run;
+    }
+    __syncthreads();
+    want -= (double)s.above;
+    return s.bin;
+}
+
+__global__ void __launch_bounds__(SR_THREADS, 2)
+sample_rows_kernel(const SampleParams p) {
+    extern __shared__ unsigned sr_keys[];
+    __shared__ SampleShared s;
     pdl_launch_dependents();
     pdl_wait();
-    const int r = blockIdx.y, tid = threadIdx.x;
+    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+    const unsigned rank = blockIdx.z;
     const float temp = p.temperature[r];
     const bool sampled = temp > 0.f;
-    if (PASS > 0 && !sampled) return;  // (a greedy row needs its best only)
-    const float* row = p.logits + (size_t)r * p.row_stride;
-    u64* w = p.work + (size_t)r * SP_WORDS;
-    u64* state = w + SP_STATE;
-    const int chunk = (p.V + SP_BLOCKS - 1) / SP_BLOCKS;
-    const int lo = min(p.V, (int)blockIdx.x * chunk), hi = min(p.V, lo + chunk);
+    const int from = min(p.V, (int)rank * p.chunk), n = min(p.V, from + p.chunk) - from;
+    const float* row = p.logits + (size_t)r * p.row_stride + from;
     const int k = p.top_k[r];
-    const bool by_k = sampled && k > 0 && k < p.V;
     const float lim = p.top_p[r];
-    const bool by_p = sampled && lim < 1.0f;
+    const bool by_k = sampled && k > 0 && k < p.V, by_p = sampled && lim < 1.0f;
+    auto read = [&](int i) { return ordered_key(sampled ? row[i] / temp : row[i]); };
+    int count = n;       // the keys that are left here ..
+    int packed = 0;      // .. in the row itself, or s.list[packed - 1]
+    bool alone = false;  // and nowhere else
+    auto key_at = [&](int i) { return packed != 0 ? s.list[packed - 1][i] : (p.staged ? sr_keys[i] : read(i)); };
+    auto index_of = [&](int i) { return packed != 0 ? s.index[packed - 1][i] : (unsigned)(from + i); };
 
-    // ---- what the passes before this one settled --------------------------------------------------
-    unsigned prefix = 0u, keep_k = 0u, keep = 0u;
-    if (PASS == 1 || PASS == 2 || PASS == 3) {
-        if (by_k) {
-            double want = PASS == 1 ? (double)k : __longlong_as_double((long long)state[2 * (PASS - 1) + 1]);
-            prefix = PASS == 1 ? 0u : (unsigned)state[2 * (PASS - 1)];
-            u64 above;
-            const int bin = find_bin(w + (PASS == 1 ? SP_CNT1 : (PASS == 2 ? SP_CNT2 : SP_CNT3)), PASS == 3 ? SP_L3 : SP_L1, want,
-                                     false, &above, scratch);
-            want -= (double)above;
-            prefix |= (unsigned)bin << (PASS == 1 ? 21 : (PASS == 2 ? 10 : 0));
-            if (PASS == 3) keep_k = prefix;
-            if (blockIdx.x == 0 && tid == 0) {
-                state[2 * PASS] = prefix;
-                state[2 * PASS + 1] = (u64)__double_as_longlong(want);
-            }
-        } else if (PASS == 3 && blockIdx.x == 0 && tid == 0) {
-            state[6] = 0u;
-        }
-        if (PASS < 3 && !by_k) return;
-    }
-    if (PASS >= 4) {
-        keep_k = (unsigned)state[6];
-        if (by_p) {
-            double want = PASS == 4 ? (double)lim * (double)w[1] : __longlong_as_double((long long)state[2 * (PASS - 1) + 1]);
-            prefix = PASS == 4 ? 0u : (unsigned)state[2 * (PASS - 1)];
-            u64 above;
-            const int bin = find_bin(w + (PASS == 4 ? SP_MASS1 : (PASS == 5 ? SP_MASS2 : SP_MASS3)), PASS == 6 ? SP_L3 : SP_L1, want,
-                                     true, &above, scratch);
-            want -= (double)above;
-            prefix |= (unsigned)bin << (PASS == 4 ? 21 : (PASS == 5 ? 10 : 0));
-            if (blockIdx.x == 0 && tid == 0) {
-                state[2 * PASS] = prefix;
-                state[2 * PASS + 1] = (u64)__double_as_longlong(want);
-            }
-        } else if (PASS < 6) {
-            return;
-        }
-        if (PASS == 6) keep = by_p ? max(keep_k, prefix) : keep_k;
-    }
-    if (PASS == 3 && !by_p) return;
-
-    // ---- this pass's walk over the block's part of the row ------------------------------------------
-    if (PASS != 6)
-        for (int i = tid; i < SP_L1; i += SP_THREADS) hist[i] = 0;
-    __syncthreads();
-    const float mx = PASS >= 3 ? key_to_float((unsigned)(w[0] >> 32)) : 0.f;
-    u64 best = 0, total = 0;
-    for (int i = lo + tid; i < hi; i += SP_THREADS) {
-        const float l = sampled ? row[i] / temp : row[i];
-        const unsigned key = ordered_key(l);
-        if (PASS == 0) {
-            const u64 cand = ((u64)key << 32) | (u64)(~(unsigned)i);
-            best = cand > best ? cand : best;
-            if (by_k) atomicAdd(&hist[key >> 21], 1ULL);
-        } else if (PASS == 1) {
-            if ((key >> 21) == (prefix >> 21)) atomicAdd(&hist[(key >> 10) & (SP_L2 - 1)], 1ULL);
-        } else if (PASS == 2) {
-            if ((key >> 10) == (prefix >> 10)) atomicAdd(&hist[key & (SP_L3 - 1)], 1ULL);
-        } else if (PASS == 3) {
-            if (key >= keep_k) {
-                const u64 q = mass_of(l, mx);
-                total += q;
-                atomicAdd(&hist[key >> 21], q);
-            }
-        } else if (PASS == 4) {
-            if (key >= keep_k && (key >> 21) == (prefix >> 21)) atomicAdd(&hist[(key >> 10) & (SP_L2 - 1)], mass_of(l, mx));
-        } else if (PASS == 5) {
-            if (key >= keep_k && (key >> 10) == (prefix >> 10)) atomicAdd(&hist[key & (SP_L3 - 1)], mass_of(l, mx));
-        } else {
-            if (key >= keep) total += mass_of(l, mx);
-        }
-    }
-    __syncthreads();
-    // ---- the block's share goes to the row's workspace -------------------------------------------------
-    if (PASS == 0) {
+    u64 best = 0;  // the largest key, its first index behind it
+    auto load = [&](auto scaled) {
+        for (int i0 = tid; i0 < n; i0 += SR_LOADS * SR_THREADS) {  // (loads first: a store to shared memory between them would hold the next ones up)
+            float l[SR_LOADS];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const u64 other = __shfl_xor_sync(0xffffffffu, best, o);
-            best = other > best ? other : best;
-        }
-        if ((tid & 31) == 0 && best != 0) atomicMax(&w[0], best);
-    }
-    if (PASS == 3 || PASS == 6) {
+            for (int j = 0; j < SR_LOADS; ++j) l[j] = i0 + j * SR_THREADS < n ? __ldg(row + i0 + j * SR_THREADS) : 0.f;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-        if ((tid & 31) == 0) scratch[tid >> 5] = total;
-        __syncthreads();
-        if (tid == 0) {
-            u64 t = 0;
-            for (int i = 0; i < SP_THREADS / 32; ++i) t += scratch[i];
-            if (PASS == 3) {
-                atomicAdd(&w[1], t);
-            } else {
-                w[SP_BLOCKSUM + blockIdx.x] = t;
-                if (blockIdx.x == 0) state[12] = keep;
+            for (int j = 0; j < SR_LOADS; ++j) {
+                const int i = i0 + j * SR_THREADS;
+                if (i >= n) break;
+                const unsigned key = ordered_key(scaled() ? l[j] / temp : l[j]);
+                if (scaled() && p.staged) sr_keys[i] = key;
+                const u64 cand = ((u64)key << 32) | (u64)(~(unsigned)(from + i));
+                best = cand > best ? cand : best;
             }
         }
-    }
-    if (PASS != 6 && (PASS != 0 || by_k)) {
-        constexpr int OUT = PASS == 0 ? SP_CNT1 : (PASS == 1 ? SP_CNT2 : (PASS == 2 ? SP_CNT3 : (PASS == 3 ? SP_MASS1 : (PASS == 4 ? SP_MASS2 : SP_MASS3))));
-        constexpr int NB = (PASS == 2 || PASS == 5) ? SP_L3 : SP_L1;
-        for (int i = tid; i < NB; i += SP_THREADS)
-            if (hist[i] != 0) atomicAdd(&w[OUT + i], hist[i]);
-    }
-}
-
-// The last kernel of the chain, a block per row: the token.  A greedy row's is its best; a sampled row's
-// is the first index, in index order, at which the kept mass so far exceeds u * total: the block of the
-// row in which that happens follows from the blocks' sums, and that block's part of the row is walked.
-__global__ void __launch_bounds__(SP_THREADS)
-sample_pick_kernel(const SampleParams p) {
-    __shared__ u64 warp_tot[SP_THREADS / 32];
-    __shared__ int first_thread;
-    pdl_launch_dependents();
-    pdl_wait();
-    const int r = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const u64* w = p.work + (size_t)r * SP_WORDS;
-    const int best_index = (int)(~(unsigned)(w[0] & 0xffffffffu));
-    const float temp = p.temperature[r];
-    if (!(temp > 0.f) || w[0] == 0) {
-        if (tid == 0) emit_token(r, w[0] == 0 ? 0 : best_index, p.out, p.row_slot, p.state, p.num_slots);
+    };
+    if (sampled)
+        load([] { return true; });
+    else
+        load([] { return false; });
+    for (int i = tid; i < SR_BINS; i += SR_THREADS) s.low[i] = s.high[i] = 0u;
+    const u64 my_best = best;
+    best = sr_cluster<SR_MAX>(best, s, 0, false);
+    const int best_index = (int)(~(unsigned)(best & 0xffffffffu));
+    if (!sampled || (by_p && lim < 0.f)) {  // (a limit below nothing keeps nothing)
+        if (rank == 0 && tid == 0) emit_token(r, best_index, p.out, p.row_slot, p.state, p.num_slots);
+        sr_cluster_sync();  // (the others may still read this block's word)
         return;
     }
-    const unsigned keep = (unsigned)w[SP_STATE + 12];
-    const float mx = key_to_float((unsigned)(w[0] >> 32));
-    u64 total = 0;
-    for (int b = 0; b < SP_BLOCKS; ++b) total += w[SP_BLOCKSUM + b];
-    const double target = (double)p.uniform[r] * (double)total;
-    int part = -1;
-    u64 base = 0;
-    for (int b = 0; b < SP_BLOCKS && part < 0; ++b) {
-        const u64 next = base + w[SP_BLOCKSUM + b];
-        if ((double)next > target)
-            part = b;
+    const float mx = key_to_float((unsigned)(best >> 32));
+    auto first_bin = [&](unsigned key) {  // falls with the key; not-a-numbers, the lowest keys, go last
+        const float below = mx - key_to_float(key);
+        return below < SR_RANGE ? (int)(below * ((SR_BINS - 1) / SR_RANGE)) : SR_BINS - 1;
+    };
+    // Moves what lies in first bin `bin` or above together, `joint`: in the first block's memory if it fits there, else within
+    // each block, and leaves it where it is if it does not fit there either.  false: the first block goes on.
+    auto pack = [&](unsigned floor, int bin, bool joint) -> bool {
+        const int per = ((count + SR_THREADS - 1) / SR_THREADS) | 1, lo = min(count, tid * per), hi = min(count, lo + per);  // (odd: no bank twice)
+        auto left = [&](unsigned key) { return key >= floor && first_bin(key) <= bin; };
+        u64 found = 0, here;  // which of the thread's first 64 keys stay
+        int mine = 0;
+#pragma unroll 4
+        for (int i = lo; i < hi; ++i)
+            if (left(key_at(i))) {
+                if (i - lo < 64) found |= 1ULL << (i - lo);
+                ++mine;
+            }
+        u64 at = sr_scan((u64)mine, s, &here) - (u64)mine;
+        bool together = false;
+        u64 all = 0, before = 0;
+        if (joint) {
+            if (tid == 0) s.box[5] = here;
+            sr_cluster_sync();
+            sr_gather(s, 5);
+            for (int c = 0; c < SR_CTAS; ++c) {
+                if (c < (int)rank) before += s.gathered[c];
+                all += s.gathered[c];
+            }
+            together = all <= SR_LIST;
+        }
+        if (!together && (packed != 0 || here > SR_LIST)) return true;
+        if (together) at += before;
+        const int to = together ? 1 : 0;
+        if (mine != 0) {
+            const unsigned list = sr_remote(s.list[to], together ? 0 : rank), index = sr_remote(s.index[to], together ? 0 : rank);
+            auto put = [&](int i) {
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(list + 4 * (unsigned)at), "r"(key_at(i)) : "memory");
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(index + 4 * (unsigned)at), "r"(index_of(i)) : "memory");
+                ++at;
+            };
+            for (; found != 0; found &= found - 1) put(lo + __ffsll((long long)found) - 1);
+            for (int i = lo + 64; i < hi; ++i)
+                if (left(key_at(i))) put(i);
+        }
+        if (together)
+            sr_cluster_sync();
         else
-            base = next;
-    }
-    if (part < 0) {  // (no mass at all: cannot happen while the best key's mass is 2^40)
-        if (tid == 0) emit_token(r, best_index, p.out, p.row_slot, p.state, p.num_slots);
-        return;
-    }
-    const float* row = p.logits + (size_t)r * p.row_stride;
-    const int chunk = (p.V + SP_BLOCKS - 1) / SP_BLOCKS;
-    const int lo = min(p.V, part * chunk), hi = min(p.V, lo + chunk);
-    const int per = (hi - lo + SP_THREADS - 1) / SP_THREADS;
-    const int my_lo = min(hi, lo + tid * per), my_hi = min(hi, my_lo + per);
-    u64 mine = 0;
-    for (int i = my_lo; i < my_hi; ++i) {
-        const float l = row[i] / temp;
-        if (ordered_key(l) >= keep) mine += mass_of(l, mx);
-    }
-    u64 incl = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const u64 n = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += n;
-    }
-    if (lane == 31) warp_tot[warp] = incl;
-    if (tid == 0) first_thread = SP_THREADS;
-    __syncthreads();
-    u64 before = base;
-    for (int wi = 0; wi < warp; ++wi) before += warp_tot[wi];
-    incl += before;
-    if (mine > 0 && (double)incl > target) atomicMin(&first_thread, tid);
-    __syncthreads();
-    if (tid == first_thread) {
-        u64 run = incl - mine;
-        int pick = my_lo;
-        for (int i = my_lo; i < my_hi; ++i) {
-            const float l = row[i] / temp;
-            if (ordered_key(l) >= keep) {
-                run += mass_of(l, mx);
-                pick = i;
-                if ((double)run > target) break;
+            __syncthreads();
+        packed = to + 1;
+        alone = together;
+        count = (int)(together ? all : here);
+        return !together || rank == 0;
+    };
+    // The key at which the sum over keys >= `floor`, from the top, of 1 or of their masses satisfies the rule.  false: another
+    // block goes on.
+    auto search = [&](bool masses, unsigned floor, double want, unsigned& found) -> bool {
+        u64 far = 0;
+#pragma unroll 4
+        for (int i = tid; i < count; i += SR_THREADS) {
+            const unsigned key = key_at(i);
+            if (key < floor) continue;
+            const int bin = first_bin(key);
+            const u64 v = masses ? mass_of(key_to_float(key), mx) : 1;
+            if (bin == SR_BINS - 1)
+                far += v;
+            else if (v != 0)
+                sr_add(s, bin, v, masses);
+        }
+        far = sr_block<SR_SUM>(far, s);
+        if (tid == 0 && far != 0) sr_add(s, SR_BINS - 1, far, masses);
+        const int bin = sr_level(s, rank, alone, want, masses ? (double)lim : -1., masses);
+        if (!alone && !pack(floor, bin, true)) return false;
+        u64 lowest = 0xffffffffu, highest = 0;
+        for (int i = tid; i < count; i += SR_THREADS) {
+            const unsigned key = key_at(i);
+            if (key >= floor && first_bin(key) == bin) {
+                lowest = sr_combine<SR_MIN>(lowest, key);
+                highest = sr_combine<SR_MAX>(highest, key);
             }
         }
-        emit_token(r, pick, p.out, p.row_slot, p.state, p.num_slots);
-    } else if (first_thread == SP_THREADS && tid == 0) {
-        emit_token(r, best_index, p.out, p.row_slot, p.state, p.num_slots);  // (unreachable: the part's sum exceeds the target)
+        unsigned lo = (unsigned)sr_cluster<SR_MIN>(lowest, s, 2, alone), hi = (unsigned)sr_cluster<SR_MAX>(highest, s, 3, alone);
+        found = 0u;
+        if (lo > hi) return true;  // (no key at all: only where no bin qualified)
+        while (lo < hi) {
+            const int bits = 32 - __clz(hi - lo), shift = bits > 11 ? bits - 11 : 0;
+            for (int i = tid; i < count; i += SR_THREADS) {
+                const unsigned key = key_at(i);
+                if (key < lo || key > hi) continue;
+                const u64 v = masses ? mass_of(key_to_float(key), mx) : 1;
+                if (v != 0) sr_add(s, (hi - key) >> shift, v, masses);
+            }
+            const unsigned b = min((unsigned)sr_level(s, rank, alone, want, -1., masses), (hi - lo) >> shift);
+            hi -= b << shift;
+            const unsigned width = (1u << shift) - 1u;
+            lo = hi - lo > width ? hi - width : lo;
+        }
+        found = hi;
+        return true;
+    };
+    unsigned keep = 0u;
+    if (by_k && k <= SR_THREADS) {
+        int bin = SR_BINS - 1;
+        if (n >= k) {
+            if (tid < n) sr_add(s, first_bin((unsigned)(my_best >> 32)), 1, false);
+            double want = (double)k;
+            bin = sr_level(s, rank, true, want, -1., false);
+        }
+        pack(0u, bin, false);
     }
+    if (by_k && !search(false, 0u, (double)k, keep)) return;
+    if (by_p) {
+        unsigned found;
+        if (!search(true, keep, 0., found)) return;
+        keep = max(keep, found);
+    }
+
+    // the token: the first index, in index order, at which the kept mass so far exceeds u * total
+    u64 mine = 0, all;
+    const int per = ((count + SR_THREADS - 1) / SR_THREADS) | 1, my_lo = min(count, tid * per), my_hi = min(count, my_lo + per);
+#pragma unroll 4
+    for (int i = my_lo; i < my_hi; ++i) {
+        const unsigned key = key_at(i);
+        if (key >= keep) mine += mass_of(key_to_float(key), mx);
+    }
+    const u64 incl = sr_scan(mine, s, &all);
+    u64 total = all, base = 0;
+    int part = 0;
+    if (tid == 0) s.first = SR_THREADS;
+    if (!alone) total = sr_cluster<SR_SUM>(mine, s, 4, false);
+    const double target = (double)p.uniform[r] * (double)total;
+    if (!alone)
+        for (; part < SR_CTAS && !((double)(base + s.gathered[part]) > target); ++part) base += s.gathered[part];
+    __syncthreads();
+    if ((int)rank == part && mine > 0 && (double)(base + incl) > target) atomicMin(&s.first, tid);
+    __syncthreads();
+    if (s.first < SR_THREADS) {
+        if (tid == s.first) s.above = base + incl - mine;
+        __syncthreads();
+        if (tid < 32) {  // the keys of the thread that was first, a lane each
+            const int lo = s.first * per, hi = min(count, lo + per);
+            u64 run = s.above;
+            for (int i = lo + lane; __any_sync(0xffffffffu, i < hi); i += 32) {
+                const unsigned key = i < hi ? key_at(i) : 0u;
+                const u64 mass = i < hi && key >= keep ? mass_of(key_to_float(key), mx) : 0;
+                u64 sum = mass;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const u64 v = __shfl_up_sync(0xffffffffu, sum, o);
+                    if (lane >= o) sum += v;
+                }
+                const unsigned over = __ballot_sync(0xffffffffu, mass > 0 && (double)(run + sum) > target);
+                if (over != 0) {
+                    if (lane == __ffs(over) - 1) emit_token(r, (int)index_of(i), p.out, p.row_slot, p.state, p.num_slots);
+                    break;
+                }
+                run += __shfl_sync(0xffffffffu, sum, 31);
+            }
+        }
+    } else if (tid == 0 && rank == 0 && (alone || part == SR_CTAS)) {
+        emit_token(r, best_index, p.out, p.row_slot, p.state, p.num_slots);  // (no mass: cannot happen while the best key's is 2^40)
+    }
+    if (!alone) sr_cluster_sync();  // (the others may still read this block's words)
 }
 
-// Words of workspace that cw_sample_rows needs for R rows (64-bit words).
-extern "C" long long cw_sample_workspace_words(int R) { return (long long)(R > 0 ? R : 0) * SP_WORDS; }
-
-// As cw_sample_state, over SP_BLOCKS thread blocks per row: `work` holds cw_sample_workspace_words(R)
-// 64-bit words, which this call zeroes first.
+// As cw_sample_state, over SR_CTAS thread blocks per row.
 extern "C" int cw_sample_rows(const float* logits, const float* temperature, const int* top_k, const float* top_p,
                               const float* uniform, int* out, int R, int V, long long row_stride, const int* row_slot,
-                              int* state, int num_slots, unsigned long long* work, cudaStream_t stream) {
+                              int* state, int num_slots, cudaStream_t stream) {
     if (R == 0) return CW_OK;
-    if (R < 0 || V <= 0 || row_stride < V || work == nullptr || (state != nullptr && (row_slot == nullptr || num_slots <= 0)))
-        return CW_ERR_BAD_SIZE;
+    if (R < 0 || V <= 0 || row_stride < V || (state != nullptr && (row_slot == nullptr || num_slots <= 0))) return CW_ERR_BAD_SIZE;
     if (R > 65535) return CW_ERR_BAD_SIZE;
-    if (cudaMemsetAsync(work, 0, (size_t)R * SP_WORDS * sizeof(u64), stream) != cudaSuccess) return (int)cudaGetLastError();
-    SampleParams p;
-    p.logits = logits; p.row_stride = (size_t)row_stride; p.V = V;
-    p.temperature = temperature; p.top_k = top_k; p.top_p = top_p; p.uniform = uniform;
-    p.work = work; p.out = out; p.row_slot = row_slot; p.state = state; p.num_slots = num_slots;
-    const dim3 grid(SP_BLOCKS, R), block(SP_THREADS);
-    int rc;
-#define CW_PASS(n) \
-    if ((rc = cw_launch(sample_pass_kernel<n>, grid, block, 0, stream, 1, p)) != CW_OK) return rc;
-    CW_PASS(0) CW_PASS(1) CW_PASS(2) CW_PASS(3) CW_PASS(4) CW_PASS(5) CW_PASS(6)
-#undef CW_PASS
-    return cw_launch(sample_pick_kernel, dim3(R), block, 0, stream, 1, p);
+    const int chunk = (V - 1) / SR_CTAS + 1, staged = chunk <= SR_STAGED;
+    const SampleParams p = {logits, (size_t)row_stride, V, temperature, top_k, top_p, uniform, out, row_slot, state, num_slots, chunk, staged};
+    const size_t smem = staged ? (size_t)chunk * sizeof(unsigned) : 0;
+    if (smem > (12u << 10)) {  // (with the tables, beyond the 48 KB that need no asking)
+        const cudaError_t e = cudaFuncSetAttribute(sample_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SR_STAGED * (int)sizeof(unsigned));
+        if (e != cudaSuccess) return (int)e;
+    }
+    return cw_launch(sample_rows_kernel, dim3(R, 1, SR_CTAS), dim3(SR_THREADS), smem, stream, SR_CTAS, p);
 }
 
 CW_TRACE_TU(sampling)

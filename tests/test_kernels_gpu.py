@@ -378,6 +378,29 @@ def test_sample_over_many_blocks_per_row_at_the_real_vocabulary(ops):
     assert many[0] == int(logits[0].argmax()) and many[9] == int(logits[9].argmax()) and many[5] == 777
 
 
+@pytest.mark.parametrize("v", [1, 8, 4096, 262144, 8 * 49152, 8 * 49152 + 1])
+def test_sample_with_a_cluster_per_row(ops, v):
+    """Vocabularies of fewer logits than a cluster's blocks, of exactly what its shared memory holds and of one more; logits so far
+    apart that most have no mass (the k-th largest among them), so close that they share a bin, rows with infinities, and numbers of
+    kept logits that fit in one block's list, in each block's own, and in none."""
+    r = 12
+    logits = rand(r, v, scale=3.0, seed=90)
+    logits[1:4] *= 20.0
+    logits[4:6] = 5.0 + logits[4:6] * 1e-5
+    logits[6, v // 2 :] = float("-inf")
+    logits[7, : v // 2] = float("-inf")
+    logits[8, :: 2] = float("-inf")
+    temps = torch.tensor([0.8, 0.3, 0.5, 1.0, 1.0, 0.7, 1.0, 0.9, 1.2, 0.0, 1.0, 1.0])
+    ks = torch.tensor([50, max(1, v // 2), 0, 3, 50, 0, max(1, v - 1), 0, 20, 0, 1, 0], dtype=torch.int32)
+    ps = torch.tensor([0.9, 1.0, 0.95, 0.5, 0.9, 0.3, 1.0, 0.8, 0.7, 1.0, 1.0, 0.0])
+    dev = lambda t: t.to(DEV)  # noqa: E731
+    for salt in (0.123, 0.77):
+        u = (torch.arange(r, dtype=torch.float32) * 0.61803 + salt) % 1.0
+        args = (dev(logits), dev(temps), dev(ks), dev(ps), dev(u))
+        many, one = ops.sample(*args).cpu().tolist(), ops.sample(*args, one_block=True).cpu().tolist()
+        assert many == one, [(i, a, b) for i, (a, b) in enumerate(zip(many, one)) if a != b]
+
+
 def test_step_inputs_from_the_request_state_table(ops, status):
     """``step_from_state``: rows name slots of the state table; fresh rows overwrite their column first;
     token, position, context length, cache slot (through the row's block table, two page groups) and the
