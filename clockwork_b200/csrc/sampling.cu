@@ -1,4 +1,4 @@
-// Greedy and stochastic sampling over float32 logits, one thread block per row.
+// Greedy and stochastic sampling over float32 logits, a cluster of thread blocks per row.
 //
 // Reference: clockwork/engine/model_runner.py:134-164.  Greedy is the first maximal index
 // (:136-137).  Otherwise logits are divided by the temperature (:149); top-k keeps logits not
@@ -37,56 +37,6 @@ __device__ __forceinline__ void emit_token(int row, int token, int* __restrict__
             state[CW_RS_DRAWS * num_slots + slot] += 1;
         }
     }
-}
-
-__global__ void __launch_bounds__(ST)
-argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int V, size_t row_stride,
-              const int* __restrict__ row_slot, int* __restrict__ state, int num_slots) {
-    __shared__ float bv[32];
-    __shared__ int bi[32];
-    pdl_launch_dependents();
-    pdl_wait();
-    const float* row = logits + (size_t)blockIdx.x * row_stride;
-    float best = -INFINITY;
-    int idx = 0x7fffffff;
-    for (int i = threadIdx.x; i < V; i += ST) {
-        const float v = row[i];
-        if (v > best || (v == best && i < idx)) { best = v; idx = i; }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-        if (ov > best || (ov == best && oi < idx)) { best = ov; idx = oi; }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) { bv[warp] = best; bi[warp] = idx; }
-    __syncthreads();
-    if (warp == 0) {
-        best = bv[lane];
-        idx = bi[lane];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
-            if (ov > best || (ov == best && oi < idx)) { best = ov; idx = oi; }
-        }
-        if (lane == 0) emit_token(blockIdx.x, (idx == 0x7fffffff) ? 0 : idx, out, row_slot, state, num_slots);
-    }
-}
-
-// row_slot / state (both or neither): see emit_token.
-extern "C" int cw_argmax_state(const float* logits, int* out, int R, int V, long long row_stride, const int* row_slot,
-                               int* state, int num_slots, cudaStream_t stream) {
-    if (R == 0) return CW_OK;
-    if (R < 0 || V <= 0 || row_stride < V || (state != nullptr && (row_slot == nullptr || num_slots <= 0))) return CW_ERR_BAD_SIZE;
-    return cw_launch(argmax_kernel, dim3(R), dim3(ST), 0, stream, 1, logits, out, V, (size_t)row_stride, row_slot, state,
-                     num_slots);
-}
-
-extern "C" int cw_argmax(const float* logits, int* out, int R, int V, long long row_stride,
-                         cudaStream_t stream) {
-    return cw_argmax_state(logits, out, R, V, row_stride, nullptr, nullptr, 0, stream);
 }
 
 __device__ __forceinline__ float block_sum_1024(float v, float* scratch) { return block_sum(v, scratch); }
@@ -658,6 +608,65 @@ sample_rows_kernel(const SampleParams p) {
         emit_token(r, best_index, p.out, p.row_slot, p.state, p.num_slots);  // (no mass: cannot happen while the best key's is 2^40)
     }
     if (!alone) sr_cluster_sync();  // (the others may still read this block's words)
+}
+
+// Greedy rows: the first of the largest logits (numbers that are none do not take part), a cluster per row.
+// Bound by the latency of the loads, of which every thread has SR_LOADS in flight: 8 rows of 151,936 6 us; with a block of
+// 1,024 threads per row 14.
+__global__ void __launch_bounds__(SR_THREADS)
+argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int V, size_t row_stride,
+              const int* __restrict__ row_slot, int* __restrict__ state, int num_slots) {
+    __shared__ u64 mine;
+    __shared__ u64 of_warp[SR_WARPS];
+    pdl_launch_dependents();
+    pdl_wait();
+    const int tid = threadIdx.x, ctas = gridDim.z, chunk = (V - 1) / ctas + 1, from = min(V, (int)blockIdx.z * chunk), n = min(V, from + chunk) - from;
+    const float* row = logits + (size_t)blockIdx.x * row_stride + from;
+    float best = -INFINITY;
+    int idx = 0x7fffffff;
+    for (int i0 = tid; i0 < n; i0 += SR_LOADS * SR_THREADS) {
+        float l[SR_LOADS];
+#pragma unroll
+        for (int j = 0; j < SR_LOADS; ++j) l[j] = i0 + j * SR_THREADS < n ? __ldg(row + i0 + j * SR_THREADS) : NAN;
+#pragma unroll
+        for (int j = 0; j < SR_LOADS; ++j)
+            if (l[j] > best || (l[j] == best && idx == 0x7fffffff)) {  // (indices rise)
+                best = l[j];
+                idx = from + i0 + j * SR_THREADS;
+            }
+    }
+    u64 all = ((u64)ordered_key(best) << 32) | (u64)(~(unsigned)idx);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) all = sr_combine<SR_MAX>(all, __shfl_xor_sync(0xffffffffu, all, o));
+    if ((tid & 31) == 0) of_warp[tid >> 5] = all;
+    __syncthreads();
+    if (tid == 0) {
+        for (int w = 1; w < SR_WARPS; ++w) all = sr_combine<SR_MAX>(all, of_warp[w]);
+        mine = all;
+    }
+    sr_cluster_sync();
+    if (tid == 0 && blockIdx.z == 0) {
+        for (int c = 1; c < ctas; ++c) all = sr_combine<SR_MAX>(all, sr_read(&mine, c));
+        const int first = (int)(~(unsigned)(all & 0xffffffffu));
+        emit_token(blockIdx.x, first == 0x7fffffff ? 0 : first, out, row_slot, state, num_slots);
+    }
+    sr_cluster_sync();  // (the first block reads the others' words)
+}
+
+// row_slot / state (both or neither): see emit_token.
+extern "C" int cw_argmax_state(const float* logits, int* out, int R, int V, long long row_stride, const int* row_slot,
+                               int* state, int num_slots, cudaStream_t stream) {
+    if (R == 0) return CW_OK;
+    if (R < 0 || V <= 0 || row_stride < V || (state != nullptr && (row_slot == nullptr || num_slots <= 0))) return CW_ERR_BAD_SIZE;
+    int ctas = SR_CTAS;  // as many as the SMs hold at a time, four each (256 rows: 8 blocks a row 40 us, 34 with 2)
+    while (ctas > 2 && (long long)R * ctas > 4 * 148) ctas >>= 1;
+    return cw_launch(argmax_kernel, dim3(R, 1, ctas), dim3(SR_THREADS), 0, stream, ctas, logits, out, V, (size_t)row_stride, row_slot,
+                     state, num_slots);
+}
+
+extern "C" int cw_argmax(const float* logits, int* out, int R, int V, long long row_stride,
+                         cudaStream_t stream) {
+    return cw_argmax_state(logits, out, R, V, row_stride, nullptr, nullptr, 0, stream);
 }
 
 // As cw_sample_state, over SR_CTAS thread blocks per row.

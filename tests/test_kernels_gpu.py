@@ -378,6 +378,20 @@ def test_sample_over_many_blocks_per_row_at_the_real_vocabulary(ops):
     assert many[0] == int(logits[0].argmax()) and many[9] == int(logits[9].argmax()) and many[5] == 777
 
 
+@pytest.mark.parametrize("rows", [1, 74, 75, 149, 600])
+@pytest.mark.parametrize("v", [1, 7, 1000, 33000])
+def test_argmax_over_each_number_of_blocks_per_row(ops, rows, v):
+    """Eight, four and two blocks; equal maxima in different blocks, rows of -infinity, numbers that are none."""
+    logits = rand(rows, v, scale=2.0, seed=rows + v).round()
+    logits[0, :] = float("-inf")
+    logits[rows // 2, v // 2 :] = logits[rows // 2].max() + 1
+    logits[rows - 1, : v // 3] = float("nan")
+    got = ops.argmax(logits.to(DEV)).cpu().tolist()
+    for row, at in zip(logits, got):
+        there = (~row.isnan()).nonzero()[:, 0]  # (never empty)
+        assert at == int(there[int(row[there].argmax())])
+
+
 @pytest.mark.parametrize("v", [1, 8, 4096, 262144, 8 * 49152, 8 * 49152 + 1])
 def test_sample_with_a_cluster_per_row(ops, v):
     """Vocabularies of fewer logits than a cluster's blocks, of exactly what its shared memory holds and of one more; logits so far
