@@ -5,8 +5,9 @@
 //
 //   C[dst(r), c_group_off*g + n] = epilogue( sum_k A[src(r), a_group_off*g + k] * B_g[n, k] )
 //
-// float32 accumulation in k order on the CUDA cores in both run precisions: a row's result depends on
-// the row and its group only, never on which other rows share its tile.
+// float32 accumulation in both run precisions; a row's result depends on the row and its group only, never on which
+// other rows share its tile.  bfloat16 runs on tcgen05 (grouped_gemm_tc.cu) where TMA can address the operands, else
+// on the mma.sync kernel further down; float32 on the CUDA cores in k order.
 //
 // Beside it the router of a mixture of experts (float32 logits, the `top` largest, weighted by the softmax
 // over the chosen or by their shares of the softmax over all; optionally only experts of the best runs of

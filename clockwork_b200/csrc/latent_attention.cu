@@ -13,7 +13,9 @@
 //   cw_latent_prepare    RMS norm of the latent (float32) and rotation of the shared key part (rotation.cuh), written to
 //                        the cache row of the token's slot; rotation of the queries' rotated parts
 //   cw_latent_attention  causal attention of a flat batch (prompt portions beside single tokens) over the
-//                        paged rows; float32 scores, weights and accumulation in both run precisions
+//                        paged rows; float32 scores, weights and accumulation in both run precisions.  bfloat16 prompt
+//                        portions run on tcgen05 (latent_attention_tc.cu), single tokens and portions whose keys are cut in
+//                        more than two parts on the mma.sync kernel here, float32 on the CUDA-core kernel
 #include "latent_attention.cuh"
 #include "rotation.cuh"
 

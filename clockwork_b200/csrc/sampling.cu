@@ -11,8 +11,9 @@
 // top-p a token stays iff the mass of the logits strictly above it does not exceed top_p (the reference's
 // sort may cut between equal logits, in an order it does not define; every token it could keep stays here).
 //
-// Nothing is sorted: the k-th largest value and the top-p cut-off are found by a bitwise search
-// over an order-preserving integer image of the logits (32 counting passes each).
+// Nothing is sorted: the k-th largest value and the top-p cut-off are found by searches over an order-preserving
+// integer image of the logits: bit by bit in sample_kernel (32 counting passes each, a block per row, kept to compare
+// against), by histograms in sample_rows_kernel.
 #include "common.cuh"
 
 #define ST 1024

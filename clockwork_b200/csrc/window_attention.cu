@@ -29,8 +29,8 @@
 // Where a head's value begins within its row is a parameter (`voff`, dk by default).  A layer whose values are its keys
 // before the rotation keeps rows [key with its `voff` leading entries rotated | those entries unrotated]: the value, with
 // its entries in the order [rest | leading ones], is the row's tail from `voff` on, and what is not rotated is kept once.
-// bfloat16 calls run the tensor-core form further down when it takes the sizes; the CUDA-core kernel is the float32
-// path and the fallback.
+// bfloat16 calls run on tcgen05 (window_attention_tc.cu) when it takes the sizes and switches, else the mma.sync form
+// further down when that does; the CUDA-core kernel is the float32 path and the fallback.
 //
 // Scores, weights, the softmax statistics and the weighted sums are float32 in both run precisions; T names
 // the type of the product's output and of the cache.  A token's result depends on its position alone: keys

@@ -16,12 +16,6 @@ def set_tensor_cores(on: bool) -> None:
     library().cw_grouped_gemm_set_mma(1 if on else 0)
 
 
-def use_warp_products(only: bool) -> None:
-    """``True``: of the tensor-core kernels the one on ``mma.sync`` alone, which takes what TMA cannot address (for
-    comparisons); ``False``: the default."""
-    library().cw_grouped_gemm_set_mma(2 if only else 1)
-
-
 def per_head_product(a: torch.Tensor, a_head_width: int, w: torch.Tensor, out: torch.Tensor, out_head_width: int,
                      gate: torch.Tensor | None = None, head_gate: torch.Tensor | None = None) -> torch.Tensor:
     """For every head h: ``out[:, h*out_head_width : +n] = a[:, h*a_head_width : +k] @ w[h].T`` with ``w`` [H, n, k];
