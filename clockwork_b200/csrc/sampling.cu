@@ -661,6 +661,8 @@ extern "C" int cw_argmax_state(const float* logits, int* out, int R, int V, long
     if (R < 0 || V <= 0 || row_stride < V || (state != nullptr && (row_slot == nullptr || num_slots <= 0))) return CW_ERR_BAD_SIZE;
     int ctas = SR_CTAS;  // as many as the SMs hold at a time, four each (256 rows: 8 blocks a row 40 us, 34 with 2)
     while (ctas > 2 && (long long)R * ctas > 4 * 148) ctas >>= 1;
+    // .. and no more than leave a thread a full round of loads (1,000 logits: a cluster's launch and barriers cost a step 2 us)
+    while (ctas > 1 && V <= SR_THREADS * SR_LOADS * (ctas / 2)) ctas >>= 1;
     return cw_launch(argmax_kernel, dim3(R, 1, ctas), dim3(SR_THREADS), 0, stream, ctas, logits, out, V, (size_t)row_stride, row_slot,
                      state, num_slots);
 }

@@ -379,9 +379,9 @@ def test_sample_over_many_blocks_per_row_at_the_real_vocabulary(ops):
 
 
 @pytest.mark.parametrize("rows", [1, 74, 75, 149, 600])
-@pytest.mark.parametrize("v", [1, 7, 1000, 33000])
+@pytest.mark.parametrize("v", [1, 7, 8192, 8193, 33000])
 def test_argmax_over_each_number_of_blocks_per_row(ops, rows, v):
-    """Eight, four and two blocks; equal maxima in different blocks, rows of -infinity, numbers that are none."""
+    """Eight, four and two blocks and one; equal maxima in different blocks, rows of -infinity, numbers that are none."""
     logits = rand(rows, v, scale=2.0, seed=rows + v).round()
     logits[0, :] = float("-inf")
     logits[rows // 2, v // 2 :] = logits[rows // 2].max() + 1
