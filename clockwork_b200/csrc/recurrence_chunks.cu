@@ -299,11 +299,11 @@ __global__ void __launch_bounds__(Dk) chunk_scan_kernel(const ChunkArgs p) {
             for (int s = 0; s < CK; s += 4) {
                 const float4 w = *(const float4*)(row + s);
 #pragma unroll
-                for (int col = 0; col < 2; ++col) {
-                    y[i][col] = fmaf(w.x, u[col][s], y[i][col]);
-                    y1[col] = fmaf(w.y, u[col][s + 1], y1[col]);
-                    y[i][col] = fmaf(w.z, u[col][s + 2], y[i][col]);
-                    y1[col] = fmaf(w.w, u[col][s + 3], y1[col]);
+                for (int col = 0; col < 2; ++col) {  // (later tokens are left out, not multiplied by zero: theirs may be no numbers)
+                    if (s <= t) y[i][col] = fmaf(w.x, u[col][s], y[i][col]);
+                    if (s + 1 <= t) y1[col] = fmaf(w.y, u[col][s + 1], y1[col]);
+                    if (s + 2 <= t) y[i][col] = fmaf(w.z, u[col][s + 2], y[i][col]);
+                    if (s + 3 <= t) y1[col] = fmaf(w.w, u[col][s + 3], y1[col]);
                 }
             }
 #pragma unroll

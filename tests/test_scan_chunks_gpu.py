@@ -124,3 +124,45 @@ def test_one_decay_per_head(form, groups, heads, dk, dv):
         last[s] = s1.transpose(1, 2).reshape(-1)
         at += m
     compare(outs, states, want, last)
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+@pytest.mark.parametrize("form", ["delta", "step size", "constant", "gated"])
+@pytest.mark.parametrize("operand", ["q", "k", "v"])
+def test_a_token_that_is_not_finite_does_not_reach_earlier_ones(form, operand, bad):
+    """Outputs of the tokens before it, of a chunk that it shares with them and of the chunks before, keep their bits; so do the
+    other requests' outputs and states."""
+    groups, heads, dk, dv = 2, 2, 64, 32
+    g = torch.Generator().manual_seed(5)
+    qk, ones = groups * dk, form == "gated"
+    start_of, spoiled = sum(LENS[:5]), 5  # the request of 130 tokens; its 40th token, in the middle of a chunk
+    at = start_of + 39
+    x = torch.randn(N, 2 * qk + heads * (dv - ones), generator=g)
+    conv = torch.zeros(x.shape[1], TAPS)
+    conv[:, -1] = 1.0  # (the delta layer's convolution passes its current input on alone)
+    coef, decays = torch.rand(N, 3 * heads, generator=g), torch.linspace(0.5, 0.99, heads)
+    state = torch.randn(len(LENS) + 1, heads * dk * dv + (TAPS - 1) * x.shape[1], generator=g) * 0.3
+    on = lambda t: None if t is None else t.clone().to(DEV)  # noqa: E731
+    ctx, outs, states = Context(), [], []
+    for value in (None, bad):
+        rows, view = x.clone(), View(on(state))
+        if value is not None:
+            rows[at, {"q": 3, "k": qk + 3, "v": 2 * qk + 3}[operand]] = value
+        w = on(rows)
+        if form == "delta":
+            out = rec.head_delta(w, on(conv), on(coef[:, :heads]), on(coef[:, heads : 2 * heads]), on(decays - 2), on(decays - 1), view, 0, heads * dk * dv, ctx,
+                                 groups, heads, dk, dv, 1e-6, 1.0, chunks=True)
+        else:
+            number, args = {"step size": (rec.FORM_STEP_SIZE, dict(pre=coef[:, :heads].contiguous(), p0=decays, p1=decays, p2=decays)),
+                            "constant": (rec.FORM_HEAD_DECAY, dict(pre=None, p0=decays, p1=None, p2=None)),
+                            "gated": (rec.FORM_GATED_WITH_KEY_SUM, dict(pre=coef, p0=None, p1=None, p2=None))}[form]
+            out = rec.recurrence_scan(number, w[:, :qk], w[:, qk : 2 * qk], w[:, 2 * qk :], view=view, offset=0, ctx=ctx, heads=heads, dk=dk, dv=dv,
+                                      heads_per_group=heads // groups, chunks=True, **{name: on(t) for name, t in args.items()})
+        outs.append(out.cpu())
+        states.append(view.state.cpu())
+    end = start_of + LENS[spoiled]
+    assert torch.isfinite(outs[0][: N - PAD]).all()
+    assert torch.equal(outs[1][:at], outs[0][:at]) and torch.equal(outs[1][end : N - PAD], outs[0][end : N - PAD])
+    assert not torch.isfinite(outs[1][at:end]).all()  # (it does reach its own output or later ones)
+    others = [s for s in range(len(LENS)) if s != spoiled]
+    assert torch.equal(states[1][others], states[0][others])
