@@ -24,6 +24,9 @@ __device__ __forceinline__ unsigned ordered_key(float f) {
     return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 
+// The same with what is no number below everything else, whatever its sign: it is not the largest, and has no mass.
+__device__ __forceinline__ unsigned logit_key(float f) { return f == f ? ordered_key(f) : 0u; }
+
 // A sampled token leaves through here.  With a request-state table given (request_state.cu) the token
 // also becomes the request's `last token`, and its position and draw counter advance by one: the next
 // step can then be launched before the host has read this one's tokens.
@@ -224,7 +227,8 @@ __device__ __forceinline__ float key_to_float(unsigned key) {
     const unsigned b = (key & 0x80000000u) ? (key & 0x7fffffffu) : ~key;
     return __uint_as_float(b);
 }
-__device__ __forceinline__ u64 mass_of(float l, float mx) { return (u64)(expf(l - mx) * SP_MASS_ONE); }
+// (none where the exponential is no number, which the conversion would turn into 2^63)
+__device__ __forceinline__ u64 mass_of(float l, float mx) { return (u64)(fmaxf(expf(l - mx), 0.f) * SP_MASS_ONE); }
 
 struct SampleParams {
     const float* logits; size_t row_stride; int V;
@@ -409,7 +413,7 @@ sample_rows_kernel(const SampleParams p) {
     const int k = p.top_k[r];
     const float lim = p.top_p[r];
     const bool by_k = sampled && k > 0 && k < p.V, by_p = sampled && lim < 1.0f;
-    auto read = [&](int i) { return ordered_key(sampled ? row[i] / temp : row[i]); };
+    auto read = [&](int i) { return logit_key(sampled ? row[i] / temp : row[i]); };
     int count = n;       // the keys that are left here ..
     int packed = 0;      // .. in the row itself, or s.list[packed - 1]
     bool alone = false;  // and nowhere else
@@ -426,7 +430,7 @@ sample_rows_kernel(const SampleParams p) {
             for (int j = 0; j < SR_LOADS; ++j) {
                 const int i = i0 + j * SR_THREADS;
                 if (i >= n) break;
-                const unsigned key = ordered_key(scaled() ? l[j] / temp : l[j]);
+                const unsigned key = logit_key(scaled() ? l[j] / temp : l[j]);
                 if (scaled() && p.staged) sr_keys[i] = key;
                 const u64 cand = ((u64)key << 32) | (u64)(~(unsigned)(from + i));
                 best = cand > best ? cand : best;
@@ -447,7 +451,7 @@ sample_rows_kernel(const SampleParams p) {
         return;
     }
     const float mx = key_to_float((unsigned)(best >> 32));
-    auto first_bin = [&](unsigned key) {  // falls with the key; not-a-numbers, the lowest keys, go last
+    auto first_bin = [&](unsigned key) {  // falls with the key; what is no number, the lowest key, goes last
         const float below = mx - key_to_float(key);
         return below < SR_RANGE ? (int)(below * ((SR_BINS - 1) / SR_RANGE)) : SR_BINS - 1;
     };

@@ -415,6 +415,32 @@ def test_sample_with_a_cluster_per_row(ops, v):
         assert many == one, [(i, a, b) for i, (a, b) in enumerate(zip(many, one)) if a != b]
 
 
+@pytest.mark.parametrize("v", [9, 5000, 8 * 49152 + 1])
+def test_sample_leaves_out_what_is_no_number(ops, v):
+    """Logits that are no numbers, of both signs: a greedy row beside sampled ones takes what ``argmax`` takes, and a sampled row the
+    token that it takes with minus infinity in their place.  One infinite logit is the token."""
+    r = 9
+    logits = rand(r, v, scale=3.0, seed=91)
+    bad = torch.zeros(r, v, dtype=torch.bool)
+    bad[:6, 2::5] = True
+    nan = torch.tensor([0x7FC00000, 0xFFC00000, 0x7FFFFFFF, 0xFFFFFFFF], dtype=torch.int64).to(torch.int32).view(torch.float32)
+    spoiled = torch.where(bad, nan[torch.arange(v) % 4].expand(r, v), logits)
+    spoiled[6:8] = nan[0]
+    spoiled[8, v // 3] = float("inf")
+    temps = torch.tensor([0.0, 0.8, 1.0, 0.7, 1.0, 0.9, 0.0, 1.0, 1.0])
+    ks = torch.tensor([0, 50, 0, 3, v - 1, 0, 0, 4, 0], dtype=torch.int32)
+    ps = torch.tensor([1.0, 0.9, 1.0, 1.0, 0.8, 0.5, 1.0, 0.9, 0.9])
+    dev = lambda t: t.to(DEV)  # noqa: E731
+    best = ops.argmax(dev(spoiled)).cpu().tolist()
+    for salt in (0.05, 0.5, 0.98):
+        u = (torch.arange(r, dtype=torch.float32) * 0.61803 + salt) % 1.0
+        tokens, without = (ops.sample(dev(x), dev(temps), dev(ks), dev(ps), dev(u)).cpu().tolist()
+                           for x in (spoiled, spoiled.masked_fill(bad, float("-inf"))))
+        assert tokens == without
+        assert [tokens[i] for i in (0, 6, 8)] == [best[i] for i in (0, 6, 8)]
+        assert best[8] == v // 3 and tokens[6:8] == [0, 0]
+
+
 def test_step_inputs_from_the_request_state_table(ops, status):
     """``step_from_state``: rows name slots of the state table; fresh rows overwrite their column first;
     token, position, context length, cache slot (through the row's block table, two page groups) and the
