@@ -307,8 +307,9 @@ extern "C" int cw_attention_rows(const void* q, int q_stride, void* out, const v
     if (N < 0 || nh <= 0 || nkv <= 0 || nh % nkv != 0 || hd <= 0 || page_size <= 0 || max_blocks <= 0) return CW_ERR_BAD_SIZE;
     if (hd > 128 || hd % 4 || q_stride % 4 || nh > 65535 || ((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_cache | (uintptr_t)v_cache) % 16)
         return CW_ERR_UNSUPPORTED;
-    const size_t smem = sizeof(float) * (size_t)(CH * (2 * hd + 4) + ROWS_PER_BLOCK * (hd + CH)) + sizeof(int) * 2 * CH;
-    const cudaError_t err = cudaFuncSetAttribute(attn_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    auto bytes = [](int size) { return sizeof(float) * (size_t)(CH * (2 * size + 4) + ROWS_PER_BLOCK * (size + CH)) + sizeof(int) * 2 * CH; };
+    const size_t smem = bytes(hd);
+    const cudaError_t err = cudaFuncSetAttribute(attn_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes(128));
     if (err != cudaSuccess) return (int)err;
     const AttnRowsArgs args = {(const float*)q, q_stride, (float*)out, (const float*)k_cache, (const float*)v_cache, block_tables, tok_seq,
                                positions, N, nh, nkv, hd, page_size, max_blocks, num_pages, scale, status};

@@ -125,8 +125,9 @@ __device__ __forceinline__ int sum_tokens_over_lanes(float (&part)[TOKENS], int 
 // would otherwise put two of the blocks that do work side by side while other SMs idle); a request with up to two for every SM
 // gets no three (64 heads of 128 x 64 over 900, 333 and 65 tokens, token by token: 337 us in rounds of one per SM, 257 in one
 // round of two, 290 without a bound).  Short steps keep what they need.
+#define CW_SCAN_ALONE (120 << 10)
 static inline size_t cw_scan_smem(size_t needed, long long rows, long long blocks_per_request) {
-    const size_t want = blocks_per_request <= 148 ? 120u << 10 : blocks_per_request <= 296 ? 76u << 10 : 0;
+    const size_t want = blocks_per_request <= 148 ? CW_SCAN_ALONE : blocks_per_request <= 296 ? 76u << 10 : 0;
     return rows >= 256 && needed < want ? want : needed;
 }
 

@@ -349,7 +349,7 @@ template <int BN, int EPI>
 static int gt_launch(const GroupedArgs& p, const CUtensorMap& w, const CUtensorMap& w2, const CUtensorMap& x, int grid, cudaStream_t stream) {
     using C = GtCfg<BN, EPI == GG_EPI_SILU_MUL>;
     const int smem = C::smem(p.G);
-    const cudaError_t e = cudaFuncSetAttribute(grouped_gemm_tc_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = cudaFuncSetAttribute(grouped_gemm_tc_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(GT_MAX_GROUPS));
     if (e != cudaSuccess) return (int)e;
     return cw_launch_ordered(grouped_gemm_tc_kernel<BN, EPI>, dim3(grid), dim3(GT_THREADS), (size_t)smem, stream, w, w2, x, p);
 }

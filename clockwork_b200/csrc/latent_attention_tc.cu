@@ -379,7 +379,7 @@ int latent_tc_run(const LatentArgs& a, cudaStream_t stream) {
     CUtensorMap q, c;
     if (lc_map(&q, a.qa, rows, D, LC_ROWS) != 0 || lc_map(&c, a.cache, (long long)a.num_pages * a.page_size, D, p.box) != 0) return CW_ERR_UNSUPPORTED;
     const size_t smem = (size_t)(p.blocks - p.held) * LC_Q_BLOCK + (size_t)p.blocks * p.stages * LC_K_BLOCK + 2048;
-    const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM);
     if (e != cudaSuccess) return (int)e;
     return cw_launch_ordered(latent_attention_tc_kernel, dim3((unsigned)blocks), dim3(LC_THREADS), smem, stream, q, c, p);
 }

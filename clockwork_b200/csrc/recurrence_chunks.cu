@@ -22,6 +22,7 @@
 #include "request_tiles.cuh"
 
 #define CK 16        // tokens of a chunk, and value columns of a block
+#define CK_SMEM CW_SCAN_ALONE  // the most that a launch asks for
 #define CK_WORDS 36  // per token s and head: G_ts of every t [16]; per token t: q_scale c_ts (q_t . k_s) of every s [16]; four factors
 
 struct ChunkArgs {
@@ -351,8 +352,9 @@ template <int Dk, bool DELTA>
 static int launch_chunks(const ChunkArgs& p, long long rows, cudaStream_t stream) {
     const dim3 grid((p.Dv + CK - 1) / CK, p.H, p.S);
     const size_t need = sizeof(float) * (size_t)(2 * (2 * CK * Dk + CK * CK + CK * CK_WORDS) + (Dk / 32 * (DELTA ? 2 : 1) + 1) * CK * CK + CK);
+    static_assert(CK_SMEM >= sizeof(float) * (2 * (2 * CK * Dk + CK * CK + CK * CK_WORDS) + (Dk / 32 * 2 + 1) * CK * CK + CK), "what a block needs");
     const size_t smem = cw_scan_smem(need, rows, (long long)grid.x * grid.y);
-    const cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<Dk, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<Dk, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CK_SMEM);
     if (e != cudaSuccess) return (int)e;
     return cw_launch_ordered(chunk_scan_kernel<Dk, DELTA>, grid, dim3(Dk), smem, stream, p);
 }

@@ -385,7 +385,7 @@ int window_tc_run(const WindowAttentionArgs& a, const int* q_start, int S, int N
             return CW_ERR_UNSUPPORTED;
     }
     const size_t smem = (size_t)kb * WC_Q_BLOCK + (size_t)p.stages * (kb + vb) * WC_BLOCK + 2048;
-    const cudaError_t e = cudaFuncSetAttribute(window_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = cudaFuncSetAttribute(window_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WC_SMEM);
     if (e != cudaSuccess) return (int)e;
     return cw_launch_ordered(window_attention_tc_kernel, dim3((unsigned)blocks), dim3(WC_THREADS), smem, stream, q, c, p);
 }
