@@ -159,6 +159,13 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 static EncodeTiledFn g_encode = nullptr;
 
 static int load_encode() {
+    // (the encoder wants the device's context in the calling thread; a thread that has launched nothing yet has none)
+    static thread_local bool bound = false;
+    if (!bound) {
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return -1;
+        bound = true;
+    }
     if (g_encode) return 0;
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q;

@@ -123,3 +123,15 @@ def test_two_threads(monkeypatch, module, name, make, large, small):
     assert not refused, (len(refused), refused[0])
     if name != "cw_chunk_scan":  # (whose state moves on with every call)
         assert all(torch.equal(a, b) for a, b in zip(before, (t for t in kept if isinstance(t, torch.Tensor))))
+
+
+@pytest.mark.parametrize("module, name, make, large, small", KERNELS, ids=[k[1] for k in KERNELS])
+def test_a_thread_that_has_not_used_the_gpu(monkeypatch, module, name, make, large, small):
+    """(The tensor maps' encoder wants the device's context in the calling thread, which a launch would have put there.)"""
+    calls, kept = recorded(monkeypatch, module, name, make, (large,))
+    answers = []
+    thread = threading.Thread(target=lambda: answers.append(calls[0][0](*calls[0][1])))
+    thread.start()
+    thread.join()
+    torch.cuda.synchronize()
+    assert answers == [0] and kept
