@@ -16,6 +16,7 @@ from __future__ import annotations
 
 from array import array
 from dataclasses import dataclass, field
+from itertools import accumulate
 
 import numpy as np
 import torch
@@ -39,28 +40,73 @@ def _pad4(n: int) -> int:
 
 
 def _flat(lists) -> np.ndarray:
-    """Lists of numbers one after the other.  (Converted a list at a time: a step that asked for logits at every place of a
-    2,048-token prompt spent 0.5 of its 0.6 ms of host time in loops over single numbers, more than the layer it fed took.)"""
+    """Lists of numbers one after the other.  (``array`` takes a list at 16 ns a number, numpy at 40, a generator at 55.)"""
     flat = array("q")
     for numbers in lists:
-        n = len(flat)
+        numbers = numbers if isinstance(numbers, (list, tuple)) else list(numbers)
         try:
-            flat.extend(iter(numbers))
+            flat.extend(array("q", numbers))
         except TypeError:  # numbers that are whole but no integers to Python
-            del flat[n:]
-            flat.extend(int(x) for x in numbers)
+            flat.extend(array("q", [int(x) for x in numbers]))
     return np.frombuffer(flat, dtype=np.int64)
 
 
-def _wanted_places(entries: list[StepEntry]) -> tuple[np.ndarray, list[int]]:
-    """The entries' wanted places one after the other, and how many each has; refuses places outside an entry's tokens."""
-    flat, counts = _flat(e.want for e in entries), [len(e.want) for e in entries]
-    if len(flat) and ((flat < 0) | (flat >= np.repeat([len(e.tokens) for e in entries], counts))).any():
+def _wanted_rows(entries: list[StepEntry], firsts: list[int]):
+    """The rows of the entries' wanted places (``firsts``: where an entry's rows begin); refuses places outside an entry's tokens.
+    (A place or two of every entry, as generation asks for: one by one; a trace replay's places of a whole prompt: as arrays.)"""
+    wanted = sum(len(e.want) for e in entries)
+    if wanted <= 2 * len(entries):
+        rows = [a + w for e, a in zip(entries, firsts) for w in e.want if 0 <= w < len(e.tokens)]
+        bad = len(rows) < wanted
+    else:
+        counts, rows = [len(e.want) for e in entries], _flat(e.want for e in entries)
+        bad = ((rows < 0) | (rows >= np.repeat([len(e.tokens) for e in entries], counts))).any()
+        rows = rows + np.repeat(firsts[: len(entries)], counts)
+    if bad:
         for e in entries:
-            bad = [w for w in e.want if not 0 <= w < len(e.tokens)]
-            if bad:
-                raise ValueError(f"request {e.request_id!r}: wanted places {bad} outside its {len(e.tokens)} tokens")
-    return flat, counts
+            outside = [w for w in e.want if not 0 <= w < len(e.tokens)]
+            if outside:
+                raise ValueError(f"request {e.request_id!r}: wanted places {outside} outside its {len(e.tokens)} tokens")
+    return rows
+
+
+def _firsts(entries: list[StepEntry]) -> list[int]:
+    """Where every entry's rows begin in the step, and how many rows there are."""
+    return list(accumulate((len(e.tokens) for e in entries), initial=0))
+
+
+def _write_rows(entries: list[StepEntry], reqs: list, firsts: list[int], tokens, positions, tok_seq) -> None:
+    tokens[: firsts[-1]] = _flat(e.tokens for e in entries)
+    for i, (r, a, b) in enumerate(zip(reqs, firsts, firsts[1:])):
+        if b - a == 1:
+            positions[a], tok_seq[a] = r.num_computed, i
+        else:
+            positions[a:b] = np.arange(r.num_computed, r.num_computed + b - a, dtype=np.int32)
+            tok_seq[a:b] = i
+
+
+def _write_pages(reqs: list, firsts: list[int], group: int, every: int, page_size: int, tables, slots) -> None:
+    """A page group's block tables and the cache rows of the step's tokens (every row of a group stands for ``every`` positions)."""
+    tables[: len(reqs)] = NO_PAGE
+    for i, (r, a, b) in enumerate(zip(reqs, firsts, firsts[1:])):
+        # (a request may hold pages for tokens far beyond this step's: the scheduler reserves a whole prompt's at
+        # admission; a captured step reads the table up to its context bound only)
+        held = array("i", r.tables[group][: tables.shape[1]])
+        tables[i, : len(held)] = held
+        start, end = r.num_computed // every, (r.num_computed + b - a - 1) // every  # rows of the first and the last token
+        first = start // page_size
+        pages = held[first : end // page_size + 1]
+        if NO_PAGE in pages:
+            raise RuntimeError(f"request {r.request_id!r}: a token lands in a page that was given back")
+        if b - a == 1:
+            slots[a] = pages[0] * page_size + start % page_size
+            continue
+        rows = (np.asarray(pages)[:, None] * page_size + np.arange(page_size, dtype=np.int32)).reshape(-1)
+        if every == 1:
+            slots[a:b] = rows[start - first * page_size : end + 1 - first * page_size]
+        else:
+            at = np.arange(r.num_computed, r.num_computed + b - a, dtype=np.int32) // every
+            slots[a:b] = rows[at - first * page_size]
 
 
 @dataclass
@@ -108,16 +154,15 @@ class StepBuilder:
 
     def prepare(self, entries: list[StepEntry]) -> PreparedStep:
         cache = self.cache
-        wanted, counts = _wanted_places(entries)
+        firsts = _firsts(entries)
+        rows = _wanted_rows(entries, firsts)
         reqs = self.requests_of(entries)
         S = len(entries)
         q_lens = [len(e.tokens) for e in entries]
-        N = sum(q_lens)
-        starts = [r.num_computed for r in reqs]
-        ctx_lens = [s + q for s, q in zip(starts, q_lens)]
+        N, R = firsts[-1], len(rows)
+        ctx_lens = [r.num_computed + q for r, q in zip(reqs, q_lens)]
         G = len(cache.groups)
         max_blocks = max(1, max((len(r.tables[g]) for r in reqs for g in range(G)), default=1))
-        R = sum(len(e.want) for e in entries)
 
         # layout of the one staging buffer (every segment starts on a 16-byte boundary)
         seg = {}
@@ -132,36 +177,15 @@ class StepBuilder:
             seg[f"tables{g}"] = (off, S * max_blocks)
             off += _pad4(S * max_blocks)
         host = self._staging(off)
-        h = host.numpy()
+        h = {name: host.numpy()[o : o + size] for name, (o, size) in seg.items()}
 
-        def put(name, values):
-            o, size = seg[name]
-            h[o : o + size] = values
-
-        put("tokens", _flat(e.tokens for e in entries))
-        put("positions", np.concatenate([np.arange(s, s + q, dtype=np.int32) for s, q in zip(starts, q_lens)]))
-        put("tok_seq", np.repeat(np.arange(S, dtype=np.int32), q_lens))
-        q_start = np.zeros(S + 1, dtype=np.int32)
-        np.cumsum(q_lens, out=q_start[1:])
-        put("q_start", q_start)
-        put("ctx_lens", ctx_lens)
-        put("rows", wanted + np.repeat(q_start[:S], counts))
-        put("state", [r.state_slot if r.state_slot is not None else 0 for r in reqs])
-        ps = cache.page_size
-        for g in range(G):
-            slots = np.empty(N, dtype=np.int32)
-            tables = np.full((S, max_blocks), NO_PAGE, dtype=np.int32)
-            for i, r in enumerate(reqs):
-                table = np.asarray(r.tables[g], dtype=np.int32)
-                tables[i, : len(table)] = table
-                # (a group of one row per `every` positions: the row of the position's block)
-                pos = np.arange(starts[i], ctx_lens[i], dtype=np.int32) // cache.groups[g].every
-                pages = table[pos // ps]
-                if (pages == NO_PAGE).any():
-                    raise RuntimeError(f"request {r.request_id!r}: a token lands in a page that was given back")
-                slots[q_start[i] : q_start[i + 1]] = pages * ps + pos % ps
-            put(f"slots{g}", slots)
-            put(f"tables{g}", tables.reshape(-1))
+        _write_rows(entries, reqs, firsts, h["tokens"], h["positions"], h["tok_seq"])
+        h["q_start"][:] = firsts
+        h["ctx_lens"][:] = ctx_lens
+        h["rows"][:] = rows
+        h["state"][:] = [r.state_slot if r.state_slot is not None else 0 for r in reqs]
+        for g, group in enumerate(cache.groups):
+            _write_pages(reqs, firsts, g, group.every, cache.page_size, h[f"tables{g}"].reshape(S, max_blocks), h[f"slots{g}"])
 
         dev = torch.empty(off, dtype=torch.int32, device=self.device)
         dev.copy_(host[:off], non_blocking=True)
@@ -468,46 +492,21 @@ class PortionGraph:
             for key, (_, fill, _) in self._arrays.items():
                 h[("array", key)][:] = fill([], [])
 
-    def fill(self, cache: CacheManager, entries: list[StepEntry], reqs: list, wants: tuple) -> list[int]:
-        """``wants``: see ``_wanted_places``.  The step's description written into the pinned buffer.  Returns the context lengths after the step."""
+    def fill(self, cache: CacheManager, entries: list[StepEntry], reqs: list, firsts: list[int], rows) -> list[int]:
+        """The step's description written into the pinned buffer (``firsts``: ``_firsts``, ``rows``: ``_wanted_rows``).  Returns
+        the context lengths after the step."""
         self._uploaded.synchronize()  # the last upload has left the pinned buffer
-        h, ps = self.h, cache.page_size
-        S = len(entries)
+        h = self.h
+        S, N, R = len(entries), firsts[-1], len(rows)
         q_lens = [len(e.tokens) for e in entries]
-        N = sum(q_lens)
-        starts = [r.num_computed for r in reqs]
-        ctx_lens = [a + q for a, q in zip(starts, q_lens)]
-        R = sum(len(e.want) for e in entries)
-        h["tokens"][:N] = _flat(e.tokens for e in entries)
-        h["tok_seq"][:N] = np.repeat(np.arange(S, dtype=np.int32), q_lens)
-        q_start = np.zeros(S + 1, dtype=np.int32)
-        np.cumsum(q_lens, out=q_start[1:])
-        h["q_start"][: S + 1] = q_start
-        h["positions"][:N] = np.arange(N) + np.repeat(np.array(starts) - q_start[:S], q_lens)
+        ctx_lens = [r.num_computed + q for r, q in zip(reqs, q_lens)]
+        _write_rows(entries, reqs, firsts, h["tokens"], h["positions"], h["tok_seq"])
+        h["q_start"][: S + 1] = firsts
         h["ctx_lens"][:S] = ctx_lens
-        h["rows"][:R] = wants[0] + np.repeat(q_start[:S], wants[1])
+        h["rows"][:R] = rows
         h["state"][:S] = [r.state_slot if r.state_slot is not None else cache.state.scratch_slot for r in reqs]
-        for g in range(len(cache.groups)):
-            slots, tables, every = h[f"slots{g}"], h[f"tables{g}"], cache.groups[g].every
-            # (a request may hold pages for tokens far beyond this step's: the scheduler reserves a
-            # whole prompt's at admission; the step reads the table up to its context bound only)
-            held = [min(len(r.tables[g]), self.max_blocks) for r in reqs]
-            flat = _flat(r.tables[g][:k] for r, k in zip(reqs, held)).astype(np.int32)
-            tables[:S] = NO_PAGE
-            o = 0
-            for i, r in enumerate(reqs):
-                table = r.tables[g]
-                tables[i, : held[i]] = flat[o : o + held[i]]
-                o += held[i]
-                first, last = starts[i] // every // ps, (ctx_lens[i] - 1) // every // ps
-                pages = table[first : last + 1]
-                if NO_PAGE in pages:
-                    raise RuntimeError(f"request {r.request_id!r}: a token lands in a page that was given back")
-                if q_lens[i] == 1:
-                    slots[q_start[i]] = pages[0] * ps + starts[i] // every % ps
-                else:
-                    pos = np.arange(starts[i], ctx_lens[i], dtype=np.int32) // every
-                    slots[q_start[i] : q_start[i + 1]] = np.array(pages, dtype=np.int32)[pos // ps - first] * ps + pos % ps
+        for g, group in enumerate(cache.groups):
+            _write_pages(reqs, firsts, g, group.every, cache.page_size, h[f"tables{g}"], h[f"slots{g}"])
         self._write_padding(cache, N, S, R)
         single_ctx = [c for q, c in zip(q_lens, ctx_lens) if q == 1]
         for name, rule in self._scalar_rules.items():
@@ -728,7 +727,8 @@ class ModelRunner:
         return made
 
     def _step_with_portion_graph(self, entries: list[StepEntry], key: tuple) -> torch.Tensor | None:
-        wants = _wanted_places(entries)
+        firsts = _firsts(entries)
+        rows = _wanted_rows(entries, firsts)
         reqs = self.builder.requests_of(entries)
         graph = self.portion_graphs.pop(key, None)
         if graph is None:
@@ -737,7 +737,7 @@ class ModelRunner:
                 del self.portion_graphs[next(iter(self.portion_graphs))]
             graph = PortionGraph(self, *key)
         self.portion_graphs[key] = graph  # (the dictionary's order is the order of last use)
-        ctx_lens = graph.fill(self.cache, entries, reqs, wants)
+        ctx_lens = graph.fill(self.cache, entries, reqs, firsts, rows)
         logits = graph.launch()
         self.builder.commit(PreparedStep(None, None, None, reqs, ctx_lens))
         self.graph_kernel_launches += graph.kernels
