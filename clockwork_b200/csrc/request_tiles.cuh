@@ -10,16 +10,17 @@ struct RowTile {
     int rows;
 };
 
-// Tile b, counted from the first request's first tile or (from_end) from the last one's last.  Called by one whole warp;
-// the lanes look at 32 requests at a time, so that their loads are in flight together.
+// Tile b, counted from the first request's first tile or (from_end) from the last one's last; requests of fewer than `from` tokens
+// or of `below` and more have none.  Called by one whole warp; the lanes look at 32 requests at a time, so that their loads are in
+// flight together.
 __device__ __forceinline__ RowTile find_row_tile(int b, bool from_end, const int* __restrict__ q_start, const int* __restrict__ tok_seq,
-                                                 int S, int per_token, int tile_rows) {
+                                                 int S, int per_token, int tile_rows, int from = 1, int below = 0x7fffffff) {
     const int lane = threadIdx.x & 31;
     auto tiles_of = [&](int s, int& first) {
         if (s >= S) return 0;
         first = q_start[s];
         const int len = q_start[s + 1] - first;
-        return len > 0 && tok_seq[first] >= 0 ? (len * per_token + tile_rows - 1) / tile_rows : 0;
+        return len > 0 && len >= from && len < below && tok_seq[first] >= 0 ? (len * per_token + tile_rows - 1) / tile_rows : 0;
     };
     if (from_end) {
         int total = 0, first = 0;

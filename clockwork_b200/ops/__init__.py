@@ -429,14 +429,18 @@ def copy_pages(cache: torch.Tensor, pairs: torch.Tensor, status: torch.Tensor) -
                                   _ptr(status), _stream()), "copy_pages")
 
 
-ATTENTION_ROWS_FROM = 4  # rows per request from which the kernel that shares a request's keys among 16 rows takes a step
+ATTENTION_ROWS_FROM = 4          # rows of a request from which the kernel that shares its keys among 16 rows takes them
+ATTENTION_ROWS_BESIDE = 12288    # rows times contexts of such requests from which they are worth a launch beside shorter requests'
 
 
 def attention_ref(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, block_tables: torch.Tensor,
                   tok_seq: torch.Tensor, positions: torch.Tensor, num_heads: int, num_kv_heads: int,
-                  head_dim: int, scale: float, window: int | None, status: torch.Tensor) -> torch.Tensor:
+                  head_dim: int, scale: float, window: int | None, status: torch.Tensor,
+                  q_start: torch.Tensor | None = None, requests: list[tuple[int, int]] | None = None) -> torch.Tensor:
     """General paged causal attention.  ``q`` is [N, >= nh*hd] with unit column stride (the
-    first nh*hd columns of each row are the query heads); returns [N, nh*hd]."""
+    first nh*hd columns of each row are the query heads); returns [N, nh*hd].  ``q_start`` (int32 [S + 1]: where the requests'
+    rows begin): float32 portions may then run on a kernel whose rows share their request's keys, with the same bits;
+    ``requests``: the rows and the context of each of the S requests, where the host knows them (no padding rows then)."""
     if not q.is_cuda or q.dim() != 2 or q.stride(1) != 1:
         raise ValueError("q must be a 2-d CUDA tensor with unit column stride")
     _need(k_cache, q.dtype, "k_cache", 4)
@@ -451,18 +455,31 @@ def attention_ref(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor,
     if head_dim > 256:
         raise ValueError(f"head_dim {head_dim} is larger than the attention kernels take (256)")
     out = torch.empty((n, num_heads * head_dim), dtype=q.dtype, device=q.device)
-    # float32 steps that are mostly prompts: blocks of 16 rows that share a request's keys (the same bits).  From four rows per
-    # request on; with fewer, blocks of rows of several requests would take them one after the other
-    if (q.dtype == torch.float32 and not window and n >= ATTENTION_ROWS_FROM * block_tables.shape[0] and head_dim % 4 == 0 and head_dim <= 128
+    # float32 portions of four rows or more: blocks of 16 rows of a request that share its keys (12 heads of 128, 8 requests behind
+    # 2,000: of 4 rows 324 us against 766 with a block per row, of 3 rows 378 and 665, but 64 of 2 rows behind 500: 566 and 489).  What
+    # is shorter, single tokens among them, keeps a block per row; a portion of little work then goes with it (20 rows beside 8 single
+    # tokens at 200: 71 us in one launch, 86 in two; 100 rows beside 24 at 2,000: 1,005 and 1,028, but 300 rows behind 200: 1,620 and 1,156)
+    shared, alone, tiles, rows = False, True, 0, 0
+    if (q_start is not None and q.dtype == torch.float32 and not window and head_dim % 4 == 0 and head_dim <= 128
             and q.stride(0) % 4 == 0 and not (q.data_ptr() | k_cache.data_ptr() | v_cache.data_ptr()) % 16):
+        _need(q_start, torch.int32, "q_start", 1)
+        shared = n >= ATTENTION_ROWS_FROM
+        if shared and requests:
+            long = [(m, c) for m, c in requests if m >= ATTENTION_ROWS_FROM]
+            tiles, rows = sum(-(-m // 16) for m, _ in long), n - sum(m for m, _ in long)
+            alone = rows > 0
+            shared = tiles > 0 and (not alone or sum(m * c for m, c in long) > ATTENTION_ROWS_BESIDE)
+            alone = alone or not shared
+    if shared:
         check(library().cw_attention_rows(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
-                                          _ptr(tok_seq), _ptr(positions), n, num_heads, num_kv_heads, head_dim, page_size,
-                                          block_tables.shape[1], pages, float(scale), _ptr(status), _stream()), "attention_rows")
-        return out
-    check(library().cw_attention_ref(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
-                                     _ptr(tok_seq), _ptr(positions), n, num_heads, num_kv_heads, head_dim, page_size,
-                                     block_tables.shape[1], pages, float(scale), int(window or 0),
-                                     dtype_code(q.dtype), _ptr(status), _stream()), "attention_ref")
+                                          _ptr(tok_seq), _ptr(positions), _ptr(q_start), q_start.shape[0] - 1, ATTENTION_ROWS_FROM, tiles, n,
+                                          num_heads, num_kv_heads, head_dim, page_size, block_tables.shape[1], pages, float(scale),
+                                          _ptr(status), _stream()), "attention_rows")
+    if alone:
+        check(library().cw_attention_ref(_ptr(q), q.stride(0), _ptr(out), _ptr(k_cache), _ptr(v_cache), _ptr(block_tables),
+                                         _ptr(tok_seq), _ptr(positions), n, num_heads, num_kv_heads, head_dim, page_size,
+                                         block_tables.shape[1], pages, float(scale), int(window or 0), _ptr(q_start) if shared else None,
+                                         q_start.shape[0] - 1 if shared else 0, ATTENTION_ROWS_FROM if shared else 0, rows, dtype_code(q.dtype), _ptr(status), _stream()), "attention_ref")
     return out
 
 

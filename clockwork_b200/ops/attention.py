@@ -61,7 +61,8 @@ def paged_attention(ctx, qkv: torch.Tensor, view, num_heads: int, num_kv_heads: 
         if not ctx.all_single_token and _prefill is not None and _prefill.accepts(ctx, view, num_heads, num_kv_heads, head_dim, window):
             return _prefill.run(ctx, qkv, view, num_heads, num_kv_heads, head_dim, scale, window)
     return attention_ref(qkv, view.k_cache, view.v_cache, view.block_tables, ctx.tok_seq, ctx.positions,
-                         num_heads, num_kv_heads, head_dim, scale, window, ctx.status)
+                         num_heads, num_kv_heads, head_dim, scale, window, ctx.status,
+                         None if ctx.all_single_token else ctx.q_start, list(zip(ctx.q_lens_host, ctx.ctx_lens_host)))
 
 
 from . import attention_fast as _attention_fast_module  # noqa: E402,F401  (registers the bfloat16 kernels)

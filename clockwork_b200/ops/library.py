@@ -22,8 +22,8 @@ _SIGNATURES: dict[str, list] = {
     "cw_gemm_ref_swiglu": [P, P, P, P, I, I, I, I, P],
     "cw_rope_store": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P],
     "cw_copy_pages": [P, P, I, I, I, LL, P, P],
-    "cw_attention_ref": [P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, I, P, P],
-    "cw_attention_rows": [P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, F, P, P],
+    "cw_attention_ref": [P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, P, I, I, I, I, P, P],
+    "cw_attention_rows": [P, I, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, P, P],
     "cw_argmax": [P, P, I, I, LL, P],
     "cw_sample": [P, P, P, P, P, P, I, I, LL, P],
     "cw_argmax_state": [P, P, I, I, LL, P, P, I, P],

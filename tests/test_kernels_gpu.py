@@ -259,9 +259,9 @@ def test_attention_ref_mixed_batch(ops, status, dtype, nh, nkv, hd, ps, window):
 
 @pytest.mark.parametrize("nh,nkv,hd,ps", [(6, 2, 128, 16), (3, 3, 48, 8), (2, 1, 4, 4), (4, 1, 16, 32)])
 def test_attention_ref_rows_that_share_keys_give_the_plain_kernels_bits(ops, status, monkeypatch, nh, nkv, hd, ps):
-    """Blocks of 16 rows against a block per row: portions that end within a block, single tokens among them, padding rows,
+    """Blocks of 16 rows against a block per row: portions that end within a block, requests of one to four rows among them, padding rows,
     contexts at the edges of a chunk of 128 keys, and values that are not finite behind the keys a row sees."""
-    ctx_lens, q_lens = [128, 333, 1, 129, 41, 300], [23, 1, 1, 129, 41, 17]
+    ctx_lens, q_lens = [128, 333, 1, 129, 41, 300, 140, 260], [23, 1, 1, 129, 41, 17, 3, 4]
     k_cache, v_cache, tables, _, _ = paged_setup(ctx_lens, nkv, hd, ps, torch.float32)
     last = [int(tables[s, (c - 1) // ps]) * ps + (c - 1) % ps for s, c in enumerate(ctx_lens)]
     for s in (0, 3):  # the last token's value is seen by the last row of the request alone
@@ -273,12 +273,48 @@ def test_attention_ref_rows_that_share_keys_give_the_plain_kernels_bits(ops, sta
     tok_seq = torch.cat([torch.full((q,), s, dtype=torch.int32) for s, q in enumerate(q_lens)] + [pad])
     positions = torch.cat([torch.arange(c - q, c, dtype=torch.int32) for c, q in zip(ctx_lens, q_lens)] + [0 * pad])
     args = [t.to(DEV) for t in (wide, k_cache, v_cache, tables, tok_seq, positions)]
-    got = ops.attention_ref(*args, nh, nkv, hd, hd**-0.5, None, status)
+    q_start = torch.tensor([0] + q_lens).cumsum(0).to(torch.int32).to(DEV)
+    got = ops.attention_ref(*args, nh, nkv, hd, hd**-0.5, None, status, q_start)
+    known = ops.attention_ref(wide[:-5].to(DEV), *args[1:4], *(t[:-5] for t in args[4:]), nh, nkv, hd, hd**-0.5, None, status, q_start,
+                              list(zip(q_lens, ctx_lens)))
     monkeypatch.setattr(ops, "ATTENTION_ROWS_FROM", 1 << 30)
-    want = ops.attention_ref(*args, nh, nkv, hd, hd**-0.5, None, status)
+    want = ops.attention_ref(*args, nh, nkv, hd, hd**-0.5, None, status, q_start)
     ops.raise_on_status(status)
+    assert torch.equal(known.nan_to_num(7.0), want[:-5].nan_to_num(7.0))
     assert torch.isinf(want).any() and not torch.isinf(want[: q_lens[0] - 1]).any()
     assert torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0)) and torch.equal(got.isnan(), want.isnan())
+
+
+def test_attention_ref_takes_single_tokens_beside_a_portion_one_by_one(ops, status, monkeypatch):
+    """float32: 32 tokens at contexts of 2,500 beside a portion of 128 rows take no longer than with a block per row each (a block of
+    16 rows of as many requests walked their contexts one after the other, six times as long); nor do requests of six rows."""
+    nh, nkv, hd, ps = 12, 2, 128, 16
+    for ctx_lens, q_lens in (([128] + [2500] * 32, [128] + [1] * 32), ([20] + [200] * 8, [20] + [1] * 8), ([2000] * 8, [6] * 8)):
+        pages = [-(-c // ps) for c in ctx_lens]
+        k_cache, v_cache = torch.randn(sum(pages), ps, nkv, hd, device=DEV), torch.randn(sum(pages), ps, nkv, hd, device=DEV)
+        tables = torch.full((len(pages), max(pages)), -1, dtype=torch.int32)
+        for s, p in enumerate(pages):
+            tables[s, :p] = torch.arange(sum(pages[:s]), sum(pages[:s]) + p)
+        tok_seq = torch.cat([torch.full((q,), s, dtype=torch.int32) for s, q in enumerate(q_lens)]).to(DEV)
+        positions = torch.cat([torch.arange(c - q, c, dtype=torch.int32) for c, q in zip(ctx_lens, q_lens)]).to(DEV)
+        q_start = torch.tensor([0] + q_lens).cumsum(0).to(torch.int32).to(DEV)
+        q, took, outs = torch.randn(sum(q_lens), nh * hd, device=DEV), {}, {}
+        for rows_from in (ops.ATTENTION_ROWS_FROM, 1 << 30):
+            monkeypatch.setattr(ops, "ATTENTION_ROWS_FROM", rows_from)
+            times = []
+            for _ in range(8):
+                begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                begin.record()
+                outs[rows_from] = ops.attention_ref(q, k_cache, v_cache, tables.to(DEV), tok_seq, positions, nh, nkv, hd, hd**-0.5, None, status,
+                                                    q_start, list(zip(q_lens, ctx_lens)))
+                end.record()
+                end.synchronize()
+                times.append(begin.elapsed_time(end))
+            took[rows_from] = min(times)
+        monkeypatch.undo()
+        ops.raise_on_status(status)
+        assert torch.equal(*outs.values())
+        assert took[ops.ATTENTION_ROWS_FROM] <= 1.1 * took[1 << 30], took
 
 
 @pytest.mark.parametrize("dtype", DTYPES)

@@ -38,7 +38,8 @@ def chunk_scan(n):
 def float32_rows(hd):
     ctx, view = one_request(100)
     q, cache = torch.randn(100, 2 * hd, device=DEV), torch.randn(PAGES, PAGE, 1, hd, device=DEV)
-    return lambda: ops.attention_ref(q, cache, cache, view.block_tables, ctx.tok_seq, ctx.positions, 2, 1, hd, 0.1, None, ctx.status)
+    return lambda: ops.attention_ref(q, cache, cache, view.block_tables, ctx.tok_seq, ctx.positions, 2, 1, hd, 0.1, None, ctx.status,
+                                     ctx.q_start)
 
 
 def windowed(d):
