@@ -7,7 +7,7 @@
 // the next group among them, whose results nobody reads); rows that lie scattered (an index says where) by TMA gathers of four
 // rows each, a lane of the producer warp per gather.  An SM gets a gathered row in about 20 cycles, which is enough for the few
 // rows of single tokens and not for a prompt's (gate and up of the sizes below: 385 us): those are copied into the
-// order of their groups first (cw_gather_rows).  A group's rows are cut in tiles of equal width, a multiple of 16, and tiles that share a weight tile are
+// order of their groups first (cw_gather_rows), and only the narrow tiles gather.  A group's rows are cut in tiles of equal width, a multiple of 16, and tiles that share a weight tile are
 // neighbours in the walk, so that it is read from HBM once.  Two accumulators in tensor memory: the epilogue of a tile (eight
 // warps, straight from tensor memory to global memory: a warp's 32 features of a row are one line in float32, and in
 // bfloat16 two lanes swap halves of two rows so that a lane stores two features) runs beside the next tile's MMAs.
@@ -134,16 +134,12 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 
     if (warp == 0) {
         // ---- producer warp: lane 0 the weight tiles, every lane the gathers of its rows ---------------------------
-        constexpr int SETS = (BN + 127) / 128;
-        int next_y[SETS][4];
+        constexpr bool GATHERS = BN == GT_SMALL_ROWS;
+        int next_y[4];
         auto find_rows = [&](const GtTile& x) {  // (rows past the tile's end: its last one again)
+            if (!GATHERS) return;
 #pragma unroll
-            for (int s = 0; s < SETS; ++s)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int r = min(s * 128 + lane * 4 + i, x.rows - 1);
-                    next_y[s][i] = p.a_index != nullptr ? p.a_index[x.row + r] / p.a_div : 0;
-                }
+            for (int i = 0; i < 4; ++i) next_y[i] = p.a_index != nullptr ? p.a_index[x.row + min(lane * 4 + i, x.rows - 1)] / p.a_div : 0;
         };
         int i = 0;
         bool ok = true;
@@ -153,18 +149,16 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             find_rows(x);
         }
         for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-            int y[SETS][4];
+            int y[4];
 #pragma unroll
-            for (int s = 0; s < SETS; ++s)
-#pragma unroll
-                for (int k = 0; k < 4; ++k) y[s][k] = next_y[s][k];
+            for (int k = 0; k < 4; ++k) y[k] = GATHERS ? next_y[k] : 0;
             const GtTile now = x;
             if (t + (int)gridDim.x < tiles) {  // the next tile's rows are looked up while this one's copies are issued
                 x = gt_tile(p, cum, first, ftiles, t + gridDim.x);
                 find_rows(x);
             }
             const int x0 = now.g * p.a_group_off, w0 = now.g * p.Nout + now.f0;
-            const bool gather = p.a_index != nullptr;
+            const bool gather = GATHERS && p.a_index != nullptr;
             const int fetched = gather ? now.width : (now.width + GT_BOX - 1) / GT_BOX * GT_BOX;  // (BN is whole boxes)
             const uint32_t tx = C::W_BYTES + fetched * GT_BK * 2;
             for (int kb = 0; kb < num_kb; ++kb, ++i) {
@@ -184,11 +178,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                         tma_load_2d(w_dst + C::W_BYTES + lane * GT_BOX * GT_BK * 2, &map_x, x0 + kb * GT_BK, now.row + lane * GT_BOX, bar);
                     continue;
                 }
-#pragma unroll
-                for (int q = 0; q < SETS; ++q) {
-                    const int r = q * 128 + lane * 4;
-                    if (r < now.width) gather_rows(w_dst + C::W_BYTES + r * GT_BK * 2, &map_x, x0 + kb * GT_BK, y[q], bar);
-                }
+                if (lane * 4 < now.width) gather_rows(w_dst + C::W_BYTES + lane * 4 * GT_BK * 2, &map_x, x0 + kb * GT_BK, y, bar);
             }
         }
         if (*give_up && lane == 0) {
@@ -334,12 +324,16 @@ static int gt_map(CUtensorMap* map, const void* ptr, long long rows, long long c
     return r == CUDA_SUCCESS ? 0 : -1;
 }
 
+// Rows per group, as far as the host knows (a router spreads them): few of them take the narrow tiles.
+static bool gt_few(const GroupedArgs& p) { return (p.offsets != nullptr ? (p.M + p.G - 1) / p.G : p.M) <= GT_SMALL_ROWS; }
+
 // TMA wants 16-byte rows and bases and all groups' matrices stacked; a group's columns of A must end where a step of 64 does (a
 // step past them would read the next group's); the epilogue stores two features at a time.
 bool grouped_tc_takes(const GroupedArgs& p, int epilogue) {
     if (p.G > GT_MAX_GROUPS || p.K % 8 || p.lda % 8 || p.a_group_off % 8 || ((uintptr_t)p.A | (uintptr_t)p.B | (uintptr_t)p.B2) % 16) return false;
     if (p.b_stride != (long long)p.Nout * p.K || (long long)p.G * p.Nout > 0x7fffffffLL) return false;
     if (p.a_group_off != 0 && p.K % GT_BK) return false;
+    if (p.a_index != nullptr && !gt_few(p)) return false;
     if (p.Nout % 2 || p.ldc % 2 || p.c_group_off % 2 || (uintptr_t)p.C % 8) return false;
     if (epilogue == GG_EPI_SIGMOID_GATE && (p.ldg % 2 || (uintptr_t)p.gate % 4)) return false;
     return true;
@@ -367,9 +361,7 @@ int grouped_tc_run(const GroupedArgs& p, int epilogue, cudaStream_t stream) {
         gt_map(&x, p.A, rows, p.a_group_off != 0 ? (long long)(p.G - 1) * p.a_group_off + p.K : p.K, p.lda,
                p.a_index != nullptr ? 1 : GT_BOX) != 0)
         return CW_ERR_UNSUPPORTED;
-    // rows per group, as far as the host knows: a router spreads them
-    const int per_group = p.offsets != nullptr ? (p.M + p.G - 1) / p.G : p.M;
-    const bool few = per_group <= GT_SMALL_ROWS;
+    const bool few = gt_few(p);
     const int bn = few ? GT_SMALL_ROWS : epilogue == GG_EPI_SILU_MUL ? 128 : 256;
     const long long ftiles = (p.Nout + GT_BM - 1) / GT_BM;
     const long long row_tiles = p.offsets != nullptr ? (long long)(p.M + bn - 1) / bn + (p.M < p.G ? p.M : p.G) : (long long)p.G * ((p.M + bn - 1) / bn);
