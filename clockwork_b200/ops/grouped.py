@@ -10,10 +10,10 @@ from .library import check, library
 EPI_STORE, EPI_STORE_F32, EPI_SILU_MUL, EPI_SIGMOID_GATE, EPI_RELU2, EPI_GROUP_GATE = 0, 1, 2, 3, 4, 5
 
 
-def set_tensor_cores(on: bool) -> None:
+def set_tensor_cores(on: bool | int) -> None:
     """bfloat16 products in groups run on the tensor cores when their sizes allow (the default); ``False`` keeps them
-    on the CUDA-core kernel that float32 runs use (for comparisons)."""
-    library().cw_grouped_gemm_set_mma(1 if on else 0)
+    on the CUDA-core kernel that float32 runs use, 2 on the mma.sync kernel where that takes them (for comparisons)."""
+    library().cw_grouped_gemm_set_mma(int(on))
 
 
 def per_head_product(a: torch.Tensor, a_head_width: int, w: torch.Tensor, out: torch.Tensor, out_head_width: int,

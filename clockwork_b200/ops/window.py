@@ -29,9 +29,10 @@ def _partial_sums(device, heads: int, dv: int, pairs: int = 0) -> torch.Tensor:
     return have
 
 
-def set_tensor_cores(on: bool) -> None:
-    """Whether bfloat16 calls may run the tensor-core form of the attention kernel (the default) or always the CUDA-core one."""
-    library().cw_window_attention_set_mma(1 if on else 0)
+def set_tensor_cores(on: bool | int) -> None:
+    """Whether bfloat16 calls may run the tensor-core forms of the attention kernel (the default) or always the CUDA-core one; 2: the
+    mma.sync form alone where it takes the sizes (for comparisons)."""
+    library().cw_window_attention_set_mma(int(on))
 
 
 def store_rows(src: torch.Tensor, col0: int, width: int, cache_rows: torch.Tensor, slots: torch.Tensor, status: torch.Tensor) -> None:

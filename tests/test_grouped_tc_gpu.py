@@ -41,6 +41,16 @@ def per_group(rows, w, group):
     return want, size
 
 
+def gate_and_up(x, wg, wu, offsets, order, top, a, a_size, b, b_size, k):
+    """The two products that begin an expert, given their sums in float64 (a: gate, b: up) and the sums of magnitudes."""
+    from clockwork_b200.ops import grouped
+
+    silu = torch.nn.functional.silu
+    # |silu'| <= 1.1, |silu(a)| <= |a|: what the two sums' errors become in the product
+    close(grouped.expert_gate_up(x, wg, wu, offsets, order, top), silu(a) * b, 1.1 * a_size * b.abs() + silu(a).abs() * b_size + 1e-6 * (a * b).abs(), 2 * k)
+    close(grouped.expert_up_relu2(x, wu, offsets, order, top), b.clamp(min=0) ** 2, 2 * b.clamp(min=0) * b_size, 2 * k)
+
+
 @pytest.mark.parametrize("sizes", [FEW, MANY], ids=["few", "many"])
 @pytest.mark.parametrize("n,k", [(200, 72), (256, 640)])
 def test_experts(sizes, n, k):
@@ -50,10 +60,7 @@ def test_experts(sizes, n, k):
     x, offsets, order, (wg, wu), group = operands(sizes, top, n, k)
     rows = x[order.long() // top]
     (a, a_size), (b, b_size) = per_group(rows, wg, group), per_group(rows, wu, group)
-    silu = torch.nn.functional.silu
-    # |silu'| <= 1.1, |silu(a)| <= |a|: what the two sums' errors become in the product
-    close(grouped.expert_gate_up(x, wg, wu, offsets, order, top), silu(a) * b, 1.1 * a_size * b.abs() + silu(a).abs() * b_size + 1e-6 * (a * b).abs(), 2 * k)
-    close(grouped.expert_up_relu2(x, wu, offsets, order, top), b.clamp(min=0) ** 2, 2 * b.clamp(min=0) * b_size, 2 * k)
+    gate_and_up(x, wg, wu, offsets, order, top, a, a_size, b, b_size, k)
     act = torch.randn(sum(sizes), k, device=DEV).to(torch.bfloat16)
     y, y_size = per_group(act, wu, group)
     want, size = torch.empty_like(y), torch.empty_like(y)
@@ -99,3 +106,4 @@ def test_takes_and_leaves():
         want, size = per_group(x[order.long()], wg, group)
         act = x[order.long()].contiguous()
         close(grouped.expert_down(act, shifted, offsets, torch.arange(sum(MANY), dtype=torch.int32, device=DEV)), want, size, k)
+        gate_and_up(x, shifted, shifted, offsets, order, 1, want, size, want, size, k)
