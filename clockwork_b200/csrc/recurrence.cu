@@ -247,7 +247,7 @@ recurrence_scan_kernel(const float* __restrict__ q, int ldq, const float* __rest
                        float* __restrict__ state, long long state_stride, long long state_off,
                        const long long* __restrict__ slots, const int* __restrict__ tok_seq,
                        const int* __restrict__ q_start, int Dk, int Dv, int heads_per_group, int ip, int wide, int H,
-                       float* __restrict__ out, int ldo, float q_scale) {
+                       float* __restrict__ out, int ldo, float q_scale, int below) {
     extern __shared__ __align__(16) float rs_smem[];
     __shared__ __align__(16) float nothing[4];  // zeros: what lanes without channels read
     if (threadIdx.x < 4) nothing[threadIdx.x] = 0.f;
@@ -258,7 +258,7 @@ recurrence_scan_kernel(const float* __restrict__ q, int ldq, const float* __rest
     // however many requests of a fixed-shape step bring none)
     const int seq = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
     const int start = q_start[seq], end = q_start[seq + 1];
-    if (end <= start) return;
+    if (end <= start || end - start >= below) return;
     const int ipart = tid % IP, jl = tid / IP, JB = blockDim.x / IP;
     const int j0 = blockIdx.x * JB, j = j0 + jl;
     const bool live = j < Dv;
@@ -432,14 +432,17 @@ recurrence_scan_kernel(const float* __restrict__ q, int ldq, const float* __rest
     }
 }
 
-// rows: the rows of the step (all requests'), which only sizes the blocks.
+// rows: the rows of the step (all requests'), which only sizes the blocks.  below > 0: requests of as many tokens and more are left
+// alone (cw_chunk_scan takes them).
 // pre: the coefficients that cw_recurrence_coefficients made (form 0: a [N, H*Dk]; form 1: [a | dt] [N, 2H]).
 extern "C" int cw_recurrence_scan(int form, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
                                   const float* pre, int ldp, const float* p0, const float* p1, const float* p2,
                                   float* state, long long state_stride, long long state_off, const long long* slots,
                                   const int* tok_seq, const int* q_start, int S, int H, int Dk, int Dv, int heads_per_group, float* out, int ldo,
-                                  float q_scale, int rows, cudaStream_t stream) {
+                                  float q_scale, int below, int rows, cudaStream_t stream) {
     if (S == 0) return CW_OK;
+    if (below <= 0) below = 0x7fffffff;
+    rows = min(rows, below);
     if (S < 0 || H <= 0 || Dk <= 0 || Dv <= 0 || heads_per_group <= 0 || H % heads_per_group) return CW_ERR_BAD_SIZE;
     if (Dk > 32 * RS || H > 65535 || S > 65535) return CW_ERR_UNSUPPORTED;
     int IP = 1, log_ip = 0;
@@ -463,7 +466,7 @@ extern "C" int cw_recurrence_scan(int form, const float* q, int ldq, const float
     static size_t allowed[5][7] = {};
     using Kernel = void (*)(const float*, int, const float*, int, const float*, int, const float*, int, const float*, const float*,
                             const float*, float*, long long, long long, const long long*, const int*, const int*, int, int, int, int, int, int,
-                            float*, int, float);
+                            float*, int, float, int);
 #define CW_FORM(f)                                                                                                              \
     {recurrence_scan_kernel<f, 1>, recurrence_scan_kernel<f, 2>, recurrence_scan_kernel<f, 4>, recurrence_scan_kernel<f, 8>,     \
      recurrence_scan_kernel<f, 16>, recurrence_scan_kernel<f, 32>, recurrence_scan_kernel<f, 0>}
@@ -475,7 +478,7 @@ extern "C" int cw_recurrence_scan(int form, const float* q, int ldq, const float
         allowed[form][which] = smem;
     }
     return cw_launch_ordered(kernels[form][which], grid, dim3(threads), smem, stream, q, ldq, k, ldk, v, ldv, pre, ldp, p0, p1, p2, state,
-                     state_stride, state_off, slots, tok_seq, q_start, Dk, Dv, heads_per_group, IP, wide, H, out, ldo, q_scale);
+                     state_stride, state_off, slots, tok_seq, q_start, Dk, Dv, heads_per_group, IP, wide, H, out, ldo, q_scale, below);
 }
 
 // Decays of a gated linear-attention layer from the pre-activations of its decay product, in place (float32):

@@ -38,6 +38,7 @@ struct ChunkArgs {
     const long long* slots;
     const int *tok_seq, *q_start;
     int S, H, Dk, Dv, heads_per_group;
+    int from;                // requests of fewer tokens are left alone (the token-by-token scans take them)
     float* out;              // [N, H Dv]
     float* gram;             // [N, H, CK_WORDS]
     // rows of `carry` [N, ldc] (C columns) whose last R of every portion go to the request's state at carry_off (null: none)
@@ -56,7 +57,7 @@ __global__ void __launch_bounds__(CK * CK) chunk_gram_kernel(const ChunkArgs p, 
     const int h0 = group * p.heads_per_group + blockIdx.y % splits * CK_HEADS, heads = min(CK_HEADS, (group + 1) * p.heads_per_group - h0);
     const int tid = threadIdx.x, Dk = p.Dk, ld = Dk + 4;
     if (tid < 32) {
-        const RowTile tile = find_row_tile(blockIdx.x, false, p.q_start, p.tok_seq, p.S, 1, CK);
+        const RowTile tile = find_row_tile(blockIdx.x, false, p.q_start, p.tok_seq, p.S, 1, CK, p.from);
         if (tid == 0) tile_row = tile.row0, tile_rows = tile.seq < 0 ? 0 : tile.rows;
     }
     __syncthreads();
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(Dk) chunk_scan_kernel(const ChunkArgs p) {
     float* ws = us + CK * CK;                // [token] W
     const int seq = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int start = p.q_start[seq], end = p.q_start[seq + 1];
-    if (end <= start) return;
+    if (end <= start || end - start < p.from) return;
     const int Dv = p.Dv, c = (tid & 7) * 2, grp = tid >> 3, j0 = blockIdx.x * CK, j = j0 + c;
     const bool live[2] = {j < Dv, j + 1 < Dv};
     const int ldo = p.H * Dv;
@@ -359,13 +360,13 @@ static int launch_chunks(const ChunkArgs& p, long long rows, cudaStream_t stream
     return cw_launch_ordered(chunk_scan_kernel<Dk, DELTA>, grid, dim3(Dk), smem, stream, p);
 }
 
-// rows: the rows of the step.  delta: the second form above (no skip, q_scale 1, no column of ones).  Heads of 32, 64 or 128
+// rows: the rows of the step.  from: requests of fewer tokens are left alone.  delta: the second form above (no skip, q_scale 1, no column of ones).  Heads of 32, 64 or 128
 // channels, rows of q and k whole 16-byte pieces at 16-byte addresses (CW_ERR_UNSUPPORTED otherwise).  gram: rows * H * 36
 // floats of scratch.
 extern "C" int cw_chunk_scan(int delta, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* a, int lda,
                              const float* b, int ldb, const float* skip, float q_scale, int ones, float* state, long long state_stride,
                              long long state_off, const long long* slots, const int* tok_seq, const int* q_start, int S, int H, int Dk,
-                             int Dv, int heads_per_group, float* out, float* gram, const float* carry, int ldc, int C, int R,
+                             int Dv, int heads_per_group, int from, float* out, float* gram, const float* carry, int ldc, int C, int R,
                              long long carry_off, int rows, cudaStream_t stream) {
     if (S == 0 || rows == 0) return CW_OK;
     if (S < 0 || rows < 0 || H <= 0 || Dk <= 0 || Dv <= (ones ? 1 : 0) || heads_per_group <= 0 || H % heads_per_group) return CW_ERR_BAD_SIZE;
@@ -374,7 +375,7 @@ extern "C" int cw_chunk_scan(int delta, const float* q, int ldq, const float* k,
     if ((Dk != 32 && Dk != 64 && Dk != 128) || ldq % 4 || ldk % 4 || (((uintptr_t)q | (uintptr_t)k | (uintptr_t)gram) & 15) || H > 65535 || S > 65535)
         return CW_ERR_UNSUPPORTED;
     const ChunkArgs p = {q, k, v, ldq, ldk, ldv, a, b, lda, ldb, skip, q_scale, ones, state, state_stride, state_off, slots, tok_seq, q_start,
-                         S, H, Dk, Dv, heads_per_group, out, gram, R > 0 ? carry : nullptr, ldc, C, R, carry_off};
+                         S, H, Dk, Dv, heads_per_group, from, out, gram, R > 0 ? carry : nullptr, ldc, C, R, carry_off};
     const int chunks = (rows + CK - 1) / CK + (rows < S ? rows : S);
     const int err = cw_launch_ordered(chunk_gram_kernel, dim3(chunks, H / heads_per_group * ((heads_per_group + CK_HEADS - 1) / CK_HEADS)), dim3(CK * CK), sizeof(float) * 2 * CK * (Dk + 4), stream, p, delta);
     if (err != CW_OK) return err;

@@ -225,8 +225,8 @@ extern "C" int cw_delta_prepare(const float* x, int ldx, const float* weight, in
 // Blocks: (request, head, slice of JB value columns); IP threads share a value column.  The operands of DC tokens at a time
 // are staged in shared memory by cp.async (the next chunk while the current one runs).  Per token the column's S^T k is
 // summed over the IP lanes by shuffles (the update needs it); the read-out sums wait until the chunk is through.  Every sum
-// has a fixed order, so a row's result does not depend on how the request's tokens were cut into steps or on what else the
-// step holds.
+// has a fixed order, so a row's result from this kernel does not depend on how the request's tokens were cut into steps or on
+// what else the step holds (bfloat16 steps may bring portions to the kernels of recurrence_chunks.cu instead, whose sums do).
 // IPT > 0: IP known at compile time and heads of whole groups of eight channels at 16-byte addresses: a thread owns channels
 // 4 ipart .. 4 ipart + 3 and the same four in the upper half of the head (two 16-byte words per operand and token), and the
 // read-out sums of the chunk's tokens are added up over the lanes with the tokens spread over them.  IPT = 0: any head size,
@@ -262,6 +262,7 @@ struct DeltaScanArgs {
     const int* tok_seq;
     const int* q_start;
     int Dk, Dv, heads_per_group, IP, wide;
+    int below;  // requests of as many tokens and more are left alone
     float* out;  // [N, ldo]
     int ldo;
     // the rows of `carry` [N, ldc] (C columns) that the next step's convolutions read again: the last R of each portion go to
@@ -282,7 +283,7 @@ delta_scan_kernel(const DeltaScanArgs g) {
     // however many requests of a fixed-shape step bring none)
     const int seq = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
     const int start = g.q_start[seq], end = g.q_start[seq + 1];
-    if (end <= start) return;
+    if (end <= start || end - start >= g.below) return;
     constexpr bool VEC = IPT > 0;
     const int IP = VEC ? IPT : g.IP, Dk = g.Dk, Dv = g.Dv;
     const int ipart = tid % IP, jl = tid / IP, JB = blockDim.x / IP;
@@ -454,12 +455,15 @@ delta_scan_kernel(const DeltaScanArgs g) {
 
 // q, k [N, groups*Dk] (head h reads group h / heads_per_group), v [N, H*Dv], beta [N, H], decays a [N, H*Dk] or, with
 // head_decay, [N, H]: float32, unit column stride, any row stride.  out [N, H*Dv].  rows: N, which only sizes the blocks.
+// below > 0: requests of as many tokens and more are left alone (cw_chunk_scan takes them).
 extern "C" int cw_delta_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* a, int lda,
                              int head_decay, const float* beta, int ldb, float* state, long long state_stride, long long state_off,
                              const long long* slots, const int* tok_seq, const int* q_start, int S, int H, int Dk, int Dv,
                              int heads_per_group, float* out, int ldo, const float* carry, int ldc, int C, int R, long long carry_off,
-                             int rows, cudaStream_t stream) {
+                             int below, int rows, cudaStream_t stream) {
     if (S == 0) return CW_OK;
+    if (below <= 0) below = 0x7fffffff;
+    rows = min(rows, below);
     if (S < 0 || H <= 0 || Dk <= 0 || Dv <= 0 || heads_per_group <= 0 || H % heads_per_group) return CW_ERR_BAD_SIZE;
     if (carry != nullptr && (C <= 0 || R < 0 || ldc < C)) return CW_ERR_BAD_SIZE;
     if (Dk > 32 * DS || H > 65535 || S > 65535) return CW_ERR_UNSUPPORTED;
@@ -491,7 +495,7 @@ extern "C" int cw_delta_scan(const float* q, int ldq, const float* k, int ldk, c
         allowed[by_head][which] = smem;
     }
     const DeltaScanArgs args = {q, ldq, k, ldk, v, ldv, a, lda, beta, ldb, state, state_stride, state_off, slots, tok_seq, q_start, Dk, Dv,
-                                heads_per_group, IP, wide, out, ldo, R > 0 ? carry : nullptr, ldc, C, R, carry_off};
+                                heads_per_group, IP, wide, below, out, ldo, R > 0 ? carry : nullptr, ldc, C, R, carry_off};
     return cw_launch_ordered(kernels[by_head][which], grid, dim3(threads), smem, stream, args);
 }
 

@@ -74,13 +74,14 @@ def chunks_take(dk: int, q, k) -> bool:
 
 
 def recurrence_scan(form: int, q, k, v, pre, p0, p1, p2, view, offset: int, ctx, heads: int, dk: int, dv: int,
-                    heads_per_group: int = 1, q_scale: float = 1.0, chunks: bool = False) -> torch.Tensor:
+                    heads_per_group: int = 1, q_scale: float = 1.0, chunks: int = 0) -> torch.Tensor:
     """float32 [N, heads*dv].  ``q``, ``k`` [N, groups*dk], ``v`` [N, heads*dv], ``pre`` [N, heads*dk] (forms 0 and 2) or
     [N, heads] (form 1) or None (form 3): float32, unit column stride, any row stride.  The state piece at ``offset``
     holds heads*dk*dv numbers.  Form 0 turns ``pre`` into the decays in place (it is a product's output that nothing
     else reads); form 2 takes ``pre`` as the decays themselves (``sigmoid_power_decay``); form 3 takes a constant
     decay per head in ``p0``.  ``q_scale`` multiplies the outputs of forms 2 and 3.  ``chunks``: in the forms with one decay
-    per head a portion's tokens may be taken 16 at a time: the same sums in an order that depends on where the portion begins."""
+    per head the tokens of requests that bring at least so many are taken 16 at a time (0: of none): the same sums in an order that
+    depends on where the portion begins."""
     for name, t in (("q", q), ("k", k), ("v", v), ("pre", pre)):
         if t is None and name == "pre" and form == FORM_HEAD_DECAY:
             continue
@@ -109,12 +110,15 @@ def recurrence_scan(form: int, q, k, v, pre, p0, p1, p2, view, offset: int, ctx,
                                       None if constant else _ptr(pre[:, heads:]), 0 if constant else ld(pre),
                                       _ptr(p2) if form == FORM_STEP_SIZE else None, 1.0 if form == FORM_STEP_SIZE else float(q_scale),
                                       1 if form == FORM_GATED_WITH_KEY_SUM else 0, state, stride, offset, slots, _ptr(ctx.tok_seq), _ptr(ctx.q_start),
-                                      ctx.num_seqs, heads, dk, dv, heads_per_group, _ptr(out), _ptr(gram), None, 0, 0, 0, 0, n, _stream()),
-              "chunk_scan")
-        return out
+                                      ctx.num_seqs, heads, dk, dv, heads_per_group, int(chunks), _ptr(out), _ptr(gram), None, 0, 0, 0, 0, n,
+                                      _stream()), "chunk_scan")
+        if chunks <= 1:
+            return out
+    else:
+        chunks = 0
     check(library().cw_recurrence_scan(form, _ptr(q), ld(q), _ptr(k), ld(k), _ptr(v), ld(v), _ptr(pre), 0 if pre is None else ld(pre),
                                        _ptr(p0), _ptr(p1), _ptr(p2), state, stride, offset, slots, _ptr(ctx.tok_seq), _ptr(ctx.q_start),
-                                       ctx.num_seqs, heads, dk, dv, heads_per_group, _ptr(out), heads * dv, float(q_scale), n, _stream()),
+                                       ctx.num_seqs, heads, dk, dv, heads_per_group, _ptr(out), heads * dv, float(q_scale), int(chunks), n, _stream()),
           "recurrence_scan")
     return out
 
@@ -154,20 +158,20 @@ def delta_scan(q, k, v, pre, beta, dt_bias, a_log, view, offset: int, ctx, heads
           "delta_coefficients")
     check(library().cw_delta_scan(_ptr(q), ld(q), _ptr(k), ld(k), _ptr(v), ld(v), _ptr(pre), ld(pre), 0, _ptr(beta), ld(beta), state, stride,
                                   offset, slots, _ptr(ctx.tok_seq), _ptr(ctx.q_start), ctx.num_seqs, heads, dk, dv, heads_per_group,
-                                  _ptr(out), heads * dv, None, 0, 0, 0, 0, n, _stream()), "delta_scan")
+                                  _ptr(out), heads * dv, None, 0, 0, 0, 0, 0, n, _stream()), "delta_scan")
     return out
 
 
 def head_delta(x, conv_weight, beta, decay, dt_bias, a_log, view, scan_offset: int, conv_offset: int, ctx, groups: int, heads: int,
-               dk: int, dv: int, unit_eps: float, q_scale: float, chunks: bool = False) -> torch.Tensor:
+               dk: int, dv: int, unit_eps: float, q_scale: float, chunks: int = 0) -> torch.Tensor:
     """float32 [N, heads*dv]: everything between a delta layer's joint product and its output norm, for one decay per head.
     ``x`` [N, >= 2*groups*dk + heads*dv] holds ``[q | k | v | ..]``; these columns pass a causal convolution of ``taps`` taps per
     channel (``conv_weight`` [channels, taps], the current token's last) and SiLU; q and k heads are divided by
     ``sqrt(sum of squares + unit_eps)``, q also multiplied by ``q_scale``; ``beta = sigmoid(beta)`` and
     ``g = exp(-exp(a_log) softplus(decay + dt_bias))`` per head; per head ``S <- g S; u = beta (v - S^T k); S <- S + k u^T; y = S^T q``.
     The state piece at ``scan_offset`` holds S, the one at ``conv_offset`` the convolutions' last taps-1 inputs (both are
-    carried on).  Two kernels.  ``chunks``: a portion's tokens may be taken 16 at a time (three kernels): the same sums in an order
-    that depends on where the portion begins."""
+    carried on).  ``chunks``: the tokens of requests that bring at least so many are taken 16 at a time (0: of none): the same sums in an
+    order that depends on where the portion begins."""
     for name, t in (("x", x), ("beta", beta), ("decay", decay)):
         if t.dtype != torch.float32 or t.dim() != 2 or t.stride(1) != 1:
             raise ValueError(f"{name} must be float32 [N, *] with unit column stride")
@@ -196,13 +200,16 @@ def head_delta(x, conv_weight, beta, decay, dt_bias, a_log, view, scan_offset: i
         gram = torch.empty((n, heads, CHUNK_GRAM_WORDS), dtype=torch.float32, device=x.device)
         check(library().cw_chunk_scan(1, _ptr(qkv), channels, _ptr(qkv[:, qk:]), channels, _ptr(qkv[:, 2 * qk :]), channels, _ptr(coef), 2 * heads,
                                       _ptr(coef[:, heads:]), 2 * heads, None, 1.0, 0, state, stride, scan_offset, slots, _ptr(ctx.tok_seq),
-                                      _ptr(ctx.q_start), ctx.num_seqs, heads, dk, dv, heads // groups, _ptr(out), _ptr(gram), _ptr(x), ld(x),
+                                      _ptr(ctx.q_start), ctx.num_seqs, heads, dk, dv, heads // groups, int(chunks), _ptr(out), _ptr(gram), _ptr(x), ld(x),
                                       channels, taps - 1, conv_offset, n, _stream()), "chunk_scan")
-        return out
+        if chunks <= 1:
+            return out
+    else:
+        chunks = 0
     check(library().cw_delta_scan(_ptr(qkv), channels, _ptr(qkv[:, qk:]), channels, _ptr(qkv[:, 2 * qk :]), channels, _ptr(coef), 2 * heads, 1,
                                   _ptr(coef[:, heads:]), 2 * heads, state, stride, scan_offset, slots, _ptr(ctx.tok_seq), _ptr(ctx.q_start),
                                   ctx.num_seqs, heads, dk, dv, heads // groups, _ptr(out), heads * dv, _ptr(x), ld(x), channels, taps - 1,
-                                  conv_offset, n, _stream()), "delta_scan")
+                                  conv_offset, int(chunks), n, _stream()), "delta_scan")
     return out
 
 

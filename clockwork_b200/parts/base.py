@@ -195,6 +195,8 @@ class Part:
     # kernels on the current stream and takes what it needs about the portions from device memory (the
     # step's arrays and ``step_arrays`` below), never from the host-side lists: such a step may be captured too
 
+    long_portions_from = 0  # > 0: forward launches other kernels when the step's longest portion has this many tokens
+
     def step_arrays(self, max_tokens: int, max_seqs: int, page_size: int, max_portions: int | None = None,
                     max_ctx: int | None = None) -> dict:
         """int32 arrays that the part's kernels read from device memory in a step of prompt portions and
@@ -203,8 +205,9 @@ class Part:
         step of up to ``max_tokens`` tokens of up to ``max_seqs`` requests with contexts up to ``max_ctx``
         (None: any), of which at most ``max_portions`` (None: all) bring more than one token, keeps ``words`` words per key
         in its input buffer, fills them before every replay and hands ``present(view)`` to the parts as
-        ``ctx.extras[key]``; ``ctx.extras["captured_portions"]`` then holds ``{"singles": bool}``
-        (whether the steps that replay this graph hold requests that bring a single token).  In an
+        ``ctx.extras[key]``; ``ctx.extras["captured_portions"]`` then holds ``{"singles": bool, "long": bool}``
+        (whether the steps that replay this graph hold requests that bring a single token, and whether their longest portion has
+        ``long_portions_from`` tokens).  In an
         uncaptured step the key is absent and the part builds the array from the step's host-side
         lists."""
         return {}

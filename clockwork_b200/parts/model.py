@@ -70,6 +70,10 @@ class DecoderModel:
         """Whether a step of this model that holds prompt portions may be captured in a CUDA graph."""
         return all(part.graph_safe_portions for part in self.all_parts())
 
+    def long_portions_from(self) -> int:
+        """From how many tokens of a step's longest portion on the model's parts launch other kernels (0: they never do)."""
+        return max(part.long_portions_from for part in self.all_parts())
+
     def all_parts(self):
         """Every part of every block, and the final norm."""
         for block in self.blocks:

@@ -54,6 +54,7 @@ class SideBySide(Mixer):
         self.right = build_part("mixer", p["right"], self.name("right"), dtype, device)
         self.graph_safe = bool(self.left.graph_safe and self.right.graph_safe)
         self.graph_safe_portions = bool(self.left.graph_safe_portions and self.right.graph_safe_portions)
+        self.long_portions_from = max(self.left.long_portions_from, self.right.long_portions_from)
         self.left_weight = self.right_weight = None
         needs = [m.cache_need() for m in (self.left, self.right)]
         if any(isinstance(n, tuple) for n in needs):

@@ -80,13 +80,32 @@ from .registry import register_mixer
 from .rotary import check_rotary, rotary_tables
 
 
-def takes_chunks(mixer: Mixer, ctx: StepContext) -> bool:
-    """Whether a scan may take a portion's tokens a chunk at a time: in bfloat16 steps that hold portions.  (A float32 run's bits do
-    not depend on how a prompt was cut into steps; a chunk of one token costs what sixteen do.)"""
-    return mixer.dtype == torch.bfloat16 and not ctx.all_single_token
+CHUNKS_FROM = 96         # tokens of a step's longest portion from which its scans take chunks
+CHUNKS_BESIDE_FROM = 256  # tokens of a step that holds single tokens from which its portions do
+
+
+def takes_chunks(mixer: Mixer, ctx: StepContext) -> int:
+    """From how many tokens of a request on a scan takes them a chunk at a time (0: never), in bfloat16 steps that hold portions.  (A
+    float32 run's bits do not depend on how a prompt was cut into steps.)  Single tokens beside a portion keep to the scan of
+    steps that hold nothing else, a launch of its own: a chunk of one token costs what sixteen do, and their bits do not change with
+    what else the step holds.
+
+    Measured (B200, us, token by token and in chunks; delta rule of 16 heads of 128 x 128, state space of 64 heads of 128 x 64,
+    retention of 16 of 128 x 128): one portion of 64 tokens 25 and 27, 25 and 27, 15 and 17; of 96 35 and 33, 35 and 32, 21 and 21; of 128
+    43 and 39, 45 and 37, 26 and 25; of 1,024 224 and 152, 228 and 144, 119 and 108; eight of 16 27 and 30, 34 and 34, 16 and 19.  24 single
+    tokens beside 200 71 and 84, 82 and 100, 43 and 60; beside 391 and 130 164 and 119 (171 with the single tokens in chunks as well), 163 and 136 (153), 108
+    and 94 (117): a step of 256 tokens and more spreads its blocks over the SMs one by one, which single tokens have no use for."""
+    if mixer.dtype != torch.bfloat16 or ctx.all_single_token:
+        return 0
+    captured = ctx.extras.get("captured_portions")
+    long, singles = (captured["long"], captured["singles"]) if captured is not None else (ctx.max_q_len >= CHUNKS_FROM, 1 in ctx.q_lens_host)
+    if not long or (singles and ctx.num_tokens < CHUNKS_BESIDE_FROM):
+        return 0
+    return 2 if singles else 1
 
 
 class Mamba2Mixer(Mixer):
+    long_portions_from = CHUNKS_FROM
     graph_safe = True
     graph_safe_portions = True
 
@@ -272,6 +291,7 @@ class GatedLinearMixer(_LinearAttention):
 
 
 class DecayLinearMixer(_LinearAttention):
+    long_portions_from = CHUNKS_FROM
     def __init__(self, spec, prefix, dtype, device) -> None:
         super().__init__(spec, prefix, dtype, device)
         decay = [float(d) for d in spec["decay"]]
@@ -296,6 +316,7 @@ class DecayLinearMixer(_LinearAttention):
 
 
 class RetentionMixer(_LinearAttention):
+    long_portions_from = CHUNKS_FROM
     def __init__(self, spec, prefix, dtype, device) -> None:
         super().__init__(spec, prefix, dtype, device)
         decay = [float(d) for d in spec["decay"]]
@@ -428,6 +449,7 @@ class _DeltaRule(Mixer):
 
 
 class HeadDeltaMixer(_DeltaRule):
+    long_portions_from = CHUNKS_FROM
     def tensor_decls(self):
         yield from self._shared_decls()
         yield TensorDecl(self.name("a"), (self.heads, self.hidden_size), "matrix", "linear")
@@ -487,6 +509,7 @@ class ChannelDeltaMixer(_DeltaRule):
 
 
 class MatrixMemoryMixer(Mixer):
+    long_portions_from = CHUNKS_FROM
     graph_safe = True
     graph_safe_portions = True
 

@@ -166,3 +166,36 @@ def test_a_token_that_is_not_finite_does_not_reach_earlier_ones(form, operand, b
     assert not torch.isfinite(outs[1][at:end]).all()  # (it does reach its own output or later ones)
     others = [s for s in range(len(LENS)) if s != spoiled]
     assert torch.equal(states[1][others], states[0][others])
+
+
+@pytest.mark.parametrize("form", ["delta", "step size", "constant", "gated"])
+def test_single_tokens_beside_portions_keep_their_bits(form):
+    """With chunks from two tokens on, a request of one token gets the bits of the scan that takes tokens one by one, as in a step
+    of single tokens, and every other request those of the chunks; nobody's state is moved on twice."""
+    groups, heads, dk, dv = 2, 4, 64, 48
+    g = torch.Generator().manual_seed(6)
+    qk, ones = groups * dk, form == "gated"
+    x = torch.randn(N, 2 * qk + heads * (dv - ones), generator=g)
+    conv, coef = torch.randn(x.shape[1], TAPS, generator=g) * 0.5, torch.rand(N, 3 * heads, generator=g)
+    decays = torch.linspace(0.5, 0.99, heads)
+    state = torch.randn(len(LENS) + 1, heads * dk * dv + (TAPS - 1) * x.shape[1], generator=g) * 0.3
+    on = lambda t: None if t is None else t.clone().to(DEV)  # noqa: E731
+    ctx, outs, states = Context(), {}, {}
+    for chunks in (0, 1, 2):
+        w, view = on(x), View(on(state))
+        if form == "delta":
+            out = rec.head_delta(w, on(conv), on(coef[:, :heads]), on(coef[:, heads : 2 * heads]), on(decays - 2), on(decays - 1), view, 0,
+                                 heads * dk * dv, ctx, groups, heads, dk, dv, 1e-6, 1.0, chunks=chunks)
+        else:
+            number, args = {"step size": (rec.FORM_STEP_SIZE, dict(pre=coef[:, :heads].contiguous(), p0=decays, p1=decays, p2=decays)),
+                            "constant": (rec.FORM_HEAD_DECAY, dict(pre=None, p0=decays, p1=None, p2=None)),
+                            "gated": (rec.FORM_GATED_WITH_KEY_SUM, dict(pre=coef, p0=None, p1=None, p2=None))}[form]
+            out = rec.recurrence_scan(number, w[:, :qk], w[:, qk : 2 * qk], w[:, 2 * qk :], view=view, offset=0, ctx=ctx, heads=heads, dk=dk, dv=dv,
+                                      heads_per_group=heads // groups, chunks=chunks, **{name: on(t) for name, t in args.items()})
+        outs[chunks], states[chunks] = out.cpu(), view.state.cpu()
+    at = 0
+    for s, m in enumerate(LENS):
+        right = 0 if m == 1 else 1
+        assert torch.equal(outs[2][at : at + m], outs[right][at : at + m]) and torch.equal(states[2][s], states[right][s]), (s, m)
+        at += m
+    assert not torch.equal(outs[0], outs[1])
