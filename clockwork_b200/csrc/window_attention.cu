@@ -33,8 +33,10 @@
 // further down when that does; the CUDA-core kernel is the float32 path and the fallback.
 //
 // Scores, weights, the softmax statistics and the weighted sums are float32 in both run precisions; T names
-// the type of the product's output and of the cache.  A token's result depends on its position alone: keys
-// are taken in tiles that start at the window's first position, in order, whatever else the step holds.
+// the type of the product's output and of the cache.  In float32 a token's result depends on its position alone: keys
+// are taken in tiles that start at the window's first position, in order, whatever else the step holds.  In bfloat16 the step's
+// rows decide which kernel runs and whether keys are cut in parts, and the tcgen05 kernel's tiles begin at multiples of 64
+// positions: the order of the sums, and with it the last bits, may change from step to step.
 #include "window_attention.cuh"
 #include "rotation.cuh"
 
@@ -947,8 +949,9 @@ window_attention_mma_kernel(const WindowMmaArgs args) {
 }
 
 static int g_window_mma = 1;
-// 1 (the default): the tensor-core kernels where they take the sizes; 2: the mma.sync kernel alone; 0: the CUDA-core kernel alone.
-extern "C" int cw_window_attention_set_mma(int on) { g_window_mma = on < 0 || on > 2 ? 1 : on; return CW_OK; }
+// 1 (the default): the tensor-core kernels where they take the sizes; 2: the mma.sync kernel alone; 3: the tcgen05 kernel also where
+// the mma.sync kernel is faster; 0: the CUDA-core kernel alone.
+extern "C" int cw_window_attention_set_mma(int on) { g_window_mma = on < 0 || on > 3 ? 1 : on; return CW_OK; }
 
 // The tensor-core form if it takes the sizes (returns 1 and launches), else 0; negative or positive: an error.
 static int window_attention_mma(const WindowAttentionArgs& base, const int* q_start, int S, int N, cudaStream_t stream, int* launched) {
@@ -1023,7 +1026,8 @@ extern "C" int cw_window_attention(const void* q, int ldq, const void* cache, co
                                           window, scale, head_scale, talk, head_bias, sigmoid_weights, blocked, sink, out, WM_BN, parts, 0,
                                           partial, status, softcap, slopes, temp_coef, temp_every, gate, ldg, pool, pool_cache, pool_tables,
                                           pool_max_blocks, pool_pages, keep, voff, gate_entries};
-        if (g_window_mma == 1 && q_start != nullptr && window_tc_takes(base, N)) return window_tc_run(base, q_start, S, N, stream);
+        const bool tc = (g_window_mma & 1) && q_start != nullptr && window_tc_takes(base);
+        if (tc && (g_window_mma == 3 || window_tc_pays(base, N, S))) return window_tc_run(base, q_start, S, N, stream);
         int launched = 0;
         const int rc = window_attention_mma(base, q_start, S, N, stream, &launched);
         if (rc != 0) return rc;
@@ -1032,6 +1036,7 @@ extern "C" int cw_window_attention(const void* q, int ldq, const void* cache, co
             return cw_launch_ordered(window_merge_kernel<bf16>, dim3(N, H), dim3(merge_threads), 0, stream, (const float*)partial, positions, tok_seq, H,
                                      dv, window, parts, 0, sigmoid_weights, 1, blocked, sink, (bf16*)out, pool, keep, gate, ldg, gate_entries);
         }
+        if (tc && parts <= WC_MAX_PARTS) return window_tc_run(base, q_start, S, N, stream);  // (sizes that the mma.sync form does not take)
     }
     int threads = 128;
     while (threads < 1024 && threads * 4 < HV) threads *= 2;      // about four output columns a thread

@@ -43,6 +43,9 @@ __device__ __forceinline__ float wa_query_temperature(int p, float coef, int eve
     return every > 0 ? 1.f + coef * logf((float)((p + 1) / every + 1)) : 1.f;
 }
 
-// Whether the tcgen05 kernel takes these switches, sizes and rows; and the launch (a.parts is not looked at: rows are not cut).
-bool window_tc_takes(const WindowAttentionArgs& a, int N);
+// Whether the tcgen05 kernel takes these switches, sizes and addresses; whether it is faster than the mma.sync kernel for a step of N
+// rows of S requests; and the launch (a.parts is not looked at there: rows are not cut).
+#define WC_MAX_PARTS 4
+bool window_tc_takes(const WindowAttentionArgs& a);
+bool window_tc_pays(const WindowAttentionArgs& a, int N, int S);
 int window_tc_run(const WindowAttentionArgs& a, const int* q_start, int S, int N, cudaStream_t stream);

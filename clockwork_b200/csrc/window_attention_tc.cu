@@ -11,11 +11,8 @@
 // Two CTAs share an SM, one's loads and exponentials beside the other's products.  A tile's pages that no row sees (given back,
 // or between the kept positions and the window) are not read; rows of a value tile that were not fetched, or lie behind the
 // context, are set to zero in shared memory.  Switches that change a score by more than a factor and an addend per row (mixed
-// heads, sigmoid weights, a cap, a distance bias, pooled blocks) stay with the mma.sync kernel.  So do steps of few rows over many
-// keys, which that kernel cuts in parts (and this one walks in one chain, 1.9 us for 64 keys): 64 tokens behind 8,000 on an open
-// window, 15 parts, take 134 us there and 236 here; 32 of them, 4 parts, 316 and 238; 512, 16 parts on 64 row tiles, 481 and 258;
-// 8 behind 1,000 in a window of 1,024, 8 parts, 39 and 43; uncut keys are slower there at every size (64 single tokens at 1,000:
-// 193 and 52; 256: 502 and 185; a window of 128: equal).
+// heads, sigmoid weights, a cap, a distance bias, pooled blocks) stay with the mma.sync kernel, and so do the steps that it is
+// faster for (window_tc_pays).
 // What bounds it: the softmax warps (64 exponentials and their split in halves a thread and tile) and the latency of a tile's chain.
 // Measured (B200, prompts of 1,500, 421 and 127 tokens, 16 heads of 128 on 4, window 1,024): mma.sync kernel and merge 223 us, this
 // one 55 us.
@@ -33,7 +30,7 @@
 #define WC_TMEM 256                   // O in columns 0 .. 127, two S buffers
 #define WC_SMEM (112 * 1024)          // two CTAs to an SM
 #define WC_MIN_TILES 64               // row tiles from which keys cut in more than WC_MAX_PARTS parts run here as well
-#define WC_MAX_PARTS 4
+#define WC_AT_ONCE 296                // CTAs that run side by side on 148 SMs
 
 struct WindowTc {
     WindowAttentionArgs a;
@@ -348,16 +345,36 @@ static int wc_stages(int kb, int vb) {
     return room > WC_MAX_STAGES ? WC_MAX_STAGES : room;
 }
 
+// Whether this kernel is the faster one.  Its time is that of a row tile's chain, about 13 us and 1.5 to 1.8 for 64 keys, times the
+// rounds of WC_AT_ONCE CTAs; single tokens fill a row tile with `per` rows of 128, so many of them take several rounds.  The
+// mma.sync kernel takes 4 to 5 us and 6 to 11 for 64 keys (24 with one head per key/value head of 128 + 128), in blocks of 16
+// rows of which four to eight share an SM, and cuts the keys of few rows in parts.  Measured there and here (us, B200):
+//   cut keys: 64 tokens behind 8,000 on an open window, 15 parts, 134 and 236; 32 of them, 4 parts, 316 and 238; 512, 16 parts on 64
+//   row tiles, 481 and 258; 8 behind 1,000 in a window of 1,024, 8 parts, 39 and 43; 4 parts of 512 keys, 32 heads of 64 + 64 on 8:
+//   8 single tokens 22 and 24, a portion of 32 24 and 27, 24 single tokens 41 and 28; with heads of 128 + 128 equal or faster here;
+//   uncut, 16 heads of 128 + 128 on 4: 64 single tokens in a window of 64 17 and 22, of 128 28 and 23; 256 of them, four rounds, 43 and
+//   80, 72 and 92, of 192 104 and 101; 32 heads of 64 + 64 on 8, 128 single tokens: 27 and 59, 44 and 67, 61 and 74, of 256 77 and 81;
+//   a portion of 300 in a window of 16 13 and 21, of 64 23 and 21 (heads of 64 + 64: 16 and 18).
+bool window_tc_pays(const WindowAttentionArgs& a, int N, int S) {
+    const int per = a.H / a.G, width = a.dk + a.dv;
+    const long long keys = (long long)a.window + a.keep;
+    const bool singles = N < 2LL * S;  // (fewer than two tokens a request: as good as all of them)
+    if (a.parts > WC_MAX_PARTS) return ((long long)N * per + WC_ROWS - 1) / WC_ROWS * a.G >= WC_MIN_TILES;
+    if (a.parts > 1) return !(a.parts == WC_MAX_PARTS && width <= 128 && per > 1 && N <= 32 && (N <= 8 || !singles));
+    if (!singles) return keys * width > (N >= 32 ? 8192 : 4096);
+    if ((long long)min(N, S) * a.G <= WC_AT_ONCE) return keys > (per > 1 ? 64 : 16);
+    return keys > (per >= 8 || (per == 1 && width > 128) ? 64 : 32768 / width);
+}
+
 // Key and value sizes of whole steps of 16 up to 128; query heads per key/value head that divide the 128 rows; rows, strides and
 // bases of whole 16-byte pieces; pages of 8, 16 or 32 tokens or a multiple of 64 (a box of keys lies in one page).
-bool window_tc_takes(const WindowAttentionArgs& a, int N) {
+bool window_tc_takes(const WindowAttentionArgs& a) {
     if (a.talk != nullptr || a.sigmoid_weights || a.softcap > 0.f || a.slopes != nullptr || a.pool > 0) return false;
     if (a.dk % 16 || a.dv % 16 || a.dk > WC_MAX_DIM || a.dv > WC_MAX_DIM) return false;
     const int per = a.H / a.G, width = a.voff + a.dv;
     if (per > WC_ROWS || (per & (per - 1)) || width % 8 || a.voff % 8 || a.ldq % 8) return false;
     if (a.page_size != 8 && a.page_size != 16 && a.page_size != 32 && a.page_size % WC_KEYS) return false;
-    if (((uintptr_t)a.q | (uintptr_t)a.cache | (uintptr_t)a.out) % 16 || (long long)a.num_pages * a.page_size > 0x7fffffffLL) return false;
-    return a.parts <= WC_MAX_PARTS || ((long long)N * per + WC_ROWS - 1) / WC_ROWS * a.G >= WC_MIN_TILES;
+    return ((uintptr_t)a.q | (uintptr_t)a.cache | (uintptr_t)a.out) % 16 == 0 && (long long)a.num_pages * a.page_size <= 0x7fffffffLL;
 }
 
 int window_tc_run(const WindowAttentionArgs& a, const int* q_start, int S, int N, cudaStream_t stream) {

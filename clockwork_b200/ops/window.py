@@ -31,7 +31,7 @@ def _partial_sums(device, heads: int, dv: int, pairs: int = 0) -> torch.Tensor:
 
 def set_tensor_cores(on: bool | int) -> None:
     """Whether bfloat16 calls may run the tensor-core forms of the attention kernel (the default) or always the CUDA-core one; 2: the
-    mma.sync form alone where it takes the sizes (for comparisons)."""
+    mma.sync form alone where it takes the sizes, 3: the tcgen05 form also where the mma.sync form is faster (for comparisons)."""
     library().cw_window_attention_set_mma(int(on))
 
 

@@ -1,7 +1,8 @@
 """Windowed attention on tcgen05 against the same attention in float64: windows of one position, shorter and longer than a tile of
 keys and than the contexts, kept first positions in the window's tile and before it, blocks of positions, pages shorter and
 longer than a tile, values that are their keys, one to sixteen query heads per key/value head, sizes that fill part of a block of 64
-columns, and each switch on the scores and the output.  Keys are not cut, so that every step runs on this kernel.  Pages that no token
+columns, and each switch on the scores and the output.  Keys are not cut, and the kernel is asked
+for whatever the step.  Pages that no token
 sees are gone from the tables and the cache holds NaN wherever no token was stored.  Bound: sums of bfloat16 operands in float32,
 weights in two bfloat16 halves (2^-16), the result rounded to bfloat16 (2^-8)."""
 
@@ -63,9 +64,14 @@ def test_portions(H, G, dk, dv, voff, window, keep, blocked, page, extras):
     scale = dk**-0.5
     on = lambda t: None if t is None else t.to(DEV)  # noqa: E731
     status = ops.new_status(DEV)
-    got = window_ops.window_attention(q.to(DEV), cache.to(DEV), tables.to(DEV), positions, tok_seq, q_start, H, G, dk, dv, window, scale,
-                                      on(head_scale), None, on(head_bias), False, status, 1, blocked=blocked, sink=on(sink), temperature=temperature,
-                                      gate=on(gate), keep_first=keep, value_offset=voff, gate_entries=entries).double().cpu()
+    window_ops.set_tensor_cores(3)  # (this kernel, where another would be faster as well)
+    try:
+        got = window_ops.window_attention(q.to(DEV), cache.to(DEV), tables.to(DEV), positions, tok_seq, q_start, H, G, dk, dv, window, scale,
+                                          on(head_scale), None, on(head_bias), False, status, 1, blocked=blocked, sink=on(sink),
+                                          temperature=temperature, gate=on(gate), keep_first=keep, value_offset=voff,
+                                          gate_entries=entries).double().cpu()
+    finally:
+        window_ops.set_tensor_cores(True)
     ops.raise_on_status(status)
     assert (got[-3:] == 0).all()
     at = 0
@@ -97,3 +103,47 @@ def test_portions(H, G, dk, dv, voff, window, keep, blocked, page, extras):
         off = (mine - want).abs()
         assert (off <= 2.0**-8 * want.abs() + 2 * slack * total + 1e-6).all(), (s, float((off / (total + 1e-9)).max()))
         at += m
+
+
+@pytest.mark.parametrize("H, G, d, window, behind, new, here", [
+    # uncut: windows and counts of single tokens on both sides of the rule
+    (16, 4, 128, 64, 1500, [1] * 64, False), (16, 4, 128, 128, 1500, [1] * 64, True), (16, 4, 128, 128, 1500, [1] * 128, False),
+    (32, 8, 64, 256, 1500, [1] * 128, False), (32, 8, 64, 320, 1500, [1] * 128, True), (16, 16, 64, 64, 1500, [1] * 8, True),
+    (8, 8, 128, 64, 1500, [1] * 48, False), (64, 8, 64, 128, 1500, [1] * 64, True),
+    # portions in narrow windows
+    (16, 4, 128, 32, 0, [300], False), (16, 4, 128, 64, 0, [300], True), (16, 4, 64, 64, 500, [40], False),
+    # cut in up to four parts, and in more on few and on many row tiles
+    (32, 8, 64, 512, 1500, [1] * 8, False), (32, 8, 64, 512, 1500, [1] * 24, True), (32, 8, 64, 512, 1500, [32], False),
+    (16, 4, 128, 512, 1500, [1] * 8, True), (16, 4, 128, 1024, 1500, [1] * 8, False), (16, 4, 128, 1 << 30, 8000, [64], False),
+    (16, 4, 128, 1 << 30, 8000, [512], True),
+    # query heads that the mma.sync kernel does not take
+    (32, 1, 64, 64, 500, [1] * 4, True),
+])
+def test_the_rule_between_the_kernels(H, G, d, window, behind, new, here):
+    """Steps on both sides of every line of the rule that chooses between the two tensor-core kernels: the default gives the bits of
+    the kernel that the rule names, and the two agree (weights in two bfloat16 halves and sums in float32 in both, the results rounded
+    to bfloat16: 2^-8 of the value from each, and 2^-15 of the sum of magnitudes)."""
+    page, n = 16, sum(new)
+    pages = -(-(behind + max(new)) // page)
+    g = torch.Generator(device=DEV).manual_seed(window % 997 + n)
+    cache = torch.randn(pages, page, G, 2 * d, device=DEV, generator=g).bfloat16()  # (the requests share their pages)
+    tables = torch.arange(pages, dtype=torch.int32, device=DEV).expand(len(new), pages).contiguous()
+    tok_seq = torch.repeat_interleave(torch.arange(len(new), dtype=torch.int32), torch.tensor(new)).to(DEV)
+    positions = torch.cat([torch.arange(behind, behind + m, dtype=torch.int32) for m in new]).to(DEV)
+    q_start = torch.tensor([0] + new).cumsum(0).to(torch.int32).to(DEV)
+    q, status = torch.randn(n, H * d, device=DEV, generator=g).bfloat16(), ops.new_status(DEV)
+    parts = window_ops.window_parts(n, window, torch.bfloat16, behind + max(new))
+    outs = {}
+    try:
+        for mode in (1, 2, 3):
+            window_ops.set_tensor_cores(mode)
+            outs[mode] = window_ops.window_attention(q, cache, tables, positions, tok_seq, q_start, H, G, d, d, window, d**-0.5, None, None, None,
+                                                     False, status, parts)
+    finally:
+        window_ops.set_tensor_cores(True)
+    ops.raise_on_status(status)
+    assert torch.equal(outs[1], outs[3 if here else 2])
+    assert not torch.equal(outs[2], outs[3]) or window == 1
+    size = float(cache.float().abs().mean()) + 1
+    off = (outs[2].double() - outs[3].double()).abs()
+    assert (off <= 2 * 2.0**-8 * outs[3].double().abs() + 2.0**-13 * size).all(), float(off.max())
