@@ -663,7 +663,7 @@ class ModelRunner:
     PORTION_LONG_WASTE = 0.04
     PORTION_SEQ_BUCKETS = (8, 64)
     PORTION_MAX_LOGITS = 1 << 28  # float32 logits that a captured step may keep (1 GiB)
-    PORTION_MAX_GRAPHS = 32       # captured steps kept at a time
+    PORTION_MAX_GRAPHS = 40       # captured steps kept at a time: a little over three for every bucket of tokens
     PORTION_MAX_PORTIONS = 8      # requests with more than one token in a captured step that also holds single tokens
 
     def _portion_token_bucket(self, tokens: int) -> int | None:

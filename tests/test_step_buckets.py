@@ -38,3 +38,8 @@ def test_long_steps_are_padded_by_four_percent_at_most():
     assert captured > 1000
     assert bucket(2048) == 2048 and bucket(4096) == 4096 and bucket(2000) == 2048
     assert bucket(1100) is None and bucket(4097) is None  # (16 % of padding; beyond the longest captured step)
+
+
+def test_captured_steps_kept_at_a_time_follow_the_buckets():
+    """(32 with ten buckets: more buckets under the same limit would put steps out, and capture them again, sooner.)"""
+    assert ModelRunner.PORTION_MAX_GRAPHS >= 3.2 * len(ModelRunner.PORTION_TOKEN_BUCKETS)
