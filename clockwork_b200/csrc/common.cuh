@@ -123,8 +123,11 @@ __device__ __forceinline__ int sum_tokens_over_lanes(float (&part)[TOKENS], int 
 // Dynamic shared memory that a scan over a long portion asks for so that its blocks spread evenly: a request that has a block
 // for at most every SM gets no two of them on one (a step of `rows` rows whose grid holds blocks for requests that bring none
 // would otherwise put two of the blocks that do work side by side while other SMs idle); a request with up to two for every SM
-// gets no three (64 heads of 128 x 64 over 900, 333 and 65 tokens, token by token: 337 us in rounds of one per SM, 257 in one
-// round of two, 290 without a bound).  Short steps keep what they need.
+// gets no three; more blocks than that fill the SMs by themselves.  Short steps keep what they need.
+// Measured (B200, token by token): 64 heads of 128 x 64 over 900, 333 and 65 tokens, state space, 337 us in rounds of one per SM, 257
+// in one round of two, 290 without a bound.  One per SM and this, one request of 512 tokens, decays per key channel: 24 heads of
+// 128 x 128 (192 blocks) 171 and 139, 48 of them (384) 257 and 222, 64 (512) 342 and 276; the delta rule 235 and 172, 350 (40 heads) and
+// 241, 471 and 353; four requests of 512 no slower at any of these.  The same times with up to 148 blocks.
 #define CW_SCAN_ALONE (120 << 10)
 static inline size_t cw_scan_smem(size_t needed, long long rows, long long blocks_per_request) {
     const size_t want = blocks_per_request <= 148 ? CW_SCAN_ALONE : blocks_per_request <= 296 ? 76u << 10 : 0;
