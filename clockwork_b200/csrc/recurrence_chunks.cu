@@ -10,8 +10,8 @@
 //   S  <- A_last S + sum of W_t k_t u_t
 // with c_ts the product of the decays s + 1 .. t, A_t that of all up to t and W_t that of all behind t.  What stands beside S and u
 // belongs to a head and not to a value column: chunk_gram_kernel makes it for all chunks side by side.  The scan is then bound
-// by its reads of q and k from shared memory (a 16-byte read takes the pipe four cycles, whatever the lanes share) and its
-// multiply-adds, two or three per token, channel and column: a thread owns two value columns and eight key channels, so that a
+// by what its four warps, one a scheduler, issue: reads of q and k from shared memory (a 16-byte read takes the pipe four cycles,
+// whatever the lanes share; the pipe 44 % busy) and multiply-adds, two or three per token, channel and column (37 %; issue slots 54 %): a thread owns two value columns and eight key channels, so that a
 // read serves eight multiply-adds, and the sums over the channels meet once per chunk.  With one column and 16 channels a thread
 // it ran 148 us instead of the 113 below.  The token-by-token scans read q and k once per column (the pipe 70 % busy in the delta
 // rule), which besides waits for four shuffles per token.

@@ -205,7 +205,8 @@ extern "C" int cw_sample(const float* logits, const float* temperature, const in
 // which blocks and threads add them up, so a row's token is the same on every run whatever the
 // scheduling (floating-point atomics would not give that), and the final walk along the row in index
 // order compares exact cumulative sums with u * total.
-// What bounds it: the instructions of the first passes (37 keys a thread), then the latency of the barriers.
+// What bounds it: the instructions of the first passes (37 keys a thread; issue slots 48 % busy over the launch), then the latency of
+// the barriers, the first of its stalls.
 // Measured (B200, 64 rows of 151,936 with top-k 50 and top-p 0.9): 62 us; a chain of eight kernels that
 // re-read the row from L2 and kept its histograms in global memory took 224; one row: 21 and 68.
 // Rows of more than SR_CTAS * SR_STAGED logits are read again from global memory on each pass.
