@@ -24,7 +24,7 @@ import torch
 from .. import ops
 from ..cache.manager import NO_PAGE, CacheManager
 from ..ops.library import launch_count
-from ..parts.base import StepContext
+from ..parts.base import StepContext, portions_class
 from ..parts.model import DecoderModel
 
 
@@ -407,10 +407,9 @@ class PortionGraph:
     arrays (``Part.step_arrays``).  Unused token rows carry token 0 at position 0 with no cache slot,
     belong to no request, and are computed and ignored; unused requests have no tokens.  ``singles``:
     whether the steps that replay this graph hold requests that bring one token (parts may serve those
-    apart from the portions, as attention does with its decode kernel); ``long``: whether their longest portion has the model's
-    ``long_portions_from`` tokens."""
+    apart from the portions, as attention does with its decode kernel); ``long``: their ``portions_class``."""
 
-    def __init__(self, runner: "ModelRunner", tokens: int, seqs: int, rows: int, max_ctx: int, singles: bool, long: bool = False) -> None:
+    def __init__(self, runner: "ModelRunner", tokens: int, seqs: int, rows: int, max_ctx: int, singles: bool, long: int = 0) -> None:
         cache, model = runner.cache, runner.model
         self.tokens, self.seqs, self.rows, self.max_ctx, self.singles = tokens, seqs, rows, max_ctx, singles
         self.max_blocks = (max_ctx + cache.page_size - 1) // cache.page_size
@@ -547,7 +546,7 @@ class ModelRunner:
         self.long_portions_from = model.long_portions_from()
         self.graph_kernel_launches = 0  # kernels replayed through graphs (for accounting)
         self.last_graph: DecodeGraph | None = None  # the graph of the last captured step that ran
-        self.portion_graphs: dict[tuple, PortionGraph] = {}  # (tokens, requests, rows, context tier, singles apart, long portions)
+        self.portion_graphs: dict[tuple, PortionGraph] = {}  # (tokens, requests, rows, context tier, singles apart, portions_class)
         self.portion_graph_steps = 0  # steps with prompt portions that replayed a captured graph
         self.last_upload_bytes = 0
         self.uploaded_bytes = 0  # host-to-device bytes of all steps so far
@@ -696,10 +695,7 @@ class ModelRunner:
         singles = any(len(e.tokens) == 1 for e in entries)
         if singles and sum(1 for e in entries if len(e.tokens) > 1) > self.PORTION_MAX_PORTIONS:
             return None  # (a captured step with single tokens has work lists for this many portions)
-        return bucket, seqs, rows, tier, singles, self._long(max(len(e.tokens) for e in entries))
-
-    def _long(self, tokens: int) -> bool:
-        return 0 < self.long_portions_from <= tokens
+        return bucket, seqs, rows, tier, singles, portions_class(max(len(e.tokens) for e in entries), bucket, self.long_portions_from)
 
     def capture_ahead(self, decode_batches=(), prompt_tokens=(), max_ctx: int = 1024, greedy: bool = True) -> int:
         """Captures, before any request needs them, the graphs of single-token steps of these batch sizes
@@ -725,7 +721,7 @@ class ModelRunner:
             bucket = self._portion_token_bucket(tokens) if self.portions_captured else None
             if bucket is None:
                 continue
-            key = (bucket, self.PORTION_SEQ_BUCKETS[0], self.PORTION_SEQ_BUCKETS[0], tier, False, self._long(tokens))
+            key = (bucket, self.PORTION_SEQ_BUCKETS[0], self.PORTION_SEQ_BUCKETS[0], tier, False, portions_class(tokens, bucket, self.long_portions_from))
             if key not in self.portion_graphs and len(self.portion_graphs) < self.PORTION_MAX_GRAPHS:
                 self.portion_graphs[key] = PortionGraph(self, *key)
                 made += 1

@@ -195,7 +195,7 @@ class Part:
     # kernels on the current stream and takes what it needs about the portions from device memory (the
     # step's arrays and ``step_arrays`` below), never from the host-side lists: such a step may be captured too
 
-    long_portions_from = 0  # > 0: forward launches other kernels when the step's longest portion has this many tokens
+    long_portions_from = 0  # > 0: what forward launches depends on the step's ``portions_class`` under this number
 
     def step_arrays(self, max_tokens: int, max_seqs: int, page_size: int, max_portions: int | None = None,
                     max_ctx: int | None = None) -> dict:
@@ -205,9 +205,8 @@ class Part:
         step of up to ``max_tokens`` tokens of up to ``max_seqs`` requests with contexts up to ``max_ctx``
         (None: any), of which at most ``max_portions`` (None: all) bring more than one token, keeps ``words`` words per key
         in its input buffer, fills them before every replay and hands ``present(view)`` to the parts as
-        ``ctx.extras[key]``; ``ctx.extras["captured_portions"]`` then holds ``{"singles": bool, "long": bool}``
-        (whether the steps that replay this graph hold requests that bring a single token, and whether their longest portion has
-        ``long_portions_from`` tokens).  In an
+        ``ctx.extras[key]``; ``ctx.extras["captured_portions"]`` then holds ``{"singles": bool, "long": int}``
+        (whether the steps that replay this graph hold requests that bring a single token, and their ``portions_class``).  In an
         uncaptured step the key is absent and the part builds the array from the step's host-side
         lists."""
         return {}
@@ -216,6 +215,12 @@ class Part:
         """Called once before steps are captured: set up whatever scratch memory a single-token step
         of up to ``max_seqs`` requests with contexts up to ``max_ctx`` needs, so that no buffer a
         captured graph points at is replaced later."""
+
+
+def portions_class(longest: int, tokens: int, long_from: int) -> int:
+    """What a step of prompt portions is to parts that take long portions by other kernels: 2 when its longest portion has
+    ``long_from`` tokens, 1 when it has 256 tokens in shorter ones, else 0 (and 0 when ``long_from`` is)."""
+    return 0 if not long_from else 2 if longest >= long_from else 1 if tokens >= 256 else 0
 
 
 class Norm(Part):

@@ -71,7 +71,7 @@ class DecoderModel:
         return all(part.graph_safe_portions for part in self.all_parts())
 
     def long_portions_from(self) -> int:
-        """From how many tokens of a step's longest portion on the model's parts launch other kernels (0: they never do)."""
+        """The number of tokens that divides the model's steps of portions by ``portions_class`` (0: nothing depends on it)."""
         return max(part.long_portions_from for part in self.all_parts())
 
     def all_parts(self):

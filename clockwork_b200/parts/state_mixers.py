@@ -74,34 +74,38 @@ import torch
 from ..ops import gemm as gemm_ops
 from ..ops import recurrence as rec_ops
 from ..weights.decl import TensorDecl
-from .base import Mixer, ResidualStream, SlotStateNeed, StateView, StepContext
+from .base import Mixer, ResidualStream, SlotStateNeed, StateView, StepContext, portions_class
 from .linear import Linear
 from .registry import register_mixer
 from .rotary import check_rotary, rotary_tables
 
 
-CHUNKS_FROM = 96         # tokens of a step's longest portion from which its scans take chunks
+CHUNKS_FROM = 80          # tokens of a step's longest portion from which its scans take chunks
 CHUNKS_BESIDE_FROM = 256  # tokens of a step that holds single tokens from which its portions do
 
 
-def takes_chunks(mixer: Mixer, ctx: StepContext) -> int:
+def takes_chunks(mixer: Mixer, ctx: StepContext, short_portions: bool = False) -> int:
     """From how many tokens of a request on a scan takes them a chunk at a time (0: never), in bfloat16 steps that hold portions.  (A
     float32 run's bits do not depend on how a prompt was cut into steps.)  Single tokens beside a portion keep to the scan of
     steps that hold nothing else, a launch of its own: a chunk of one token costs what sixteen do, and their bits do not change with
-    what else the step holds.
+    what else the step holds.  ``short_portions``: also in steps of 256 tokens whose portions are all shorter.
 
     Measured (B200, us, token by token and in chunks; delta rule of 16 heads of 128 x 128, state space of 64 heads of 128 x 64,
-    retention of 16 of 128 x 128): one portion of 64 tokens 25 and 27, 25 and 27, 15 and 17; of 96 35 and 33, 35 and 32, 21 and 21; of 128
-    43 and 39, 45 and 37, 26 and 25; of 1,024 224 and 152, 228 and 144, 119 and 108; eight of 16 27 and 30, 34 and 34, 16 and 19.  24 single
-    tokens beside 200 71 and 84, 82 and 100, 43 and 60; beside 391 and 130 164 and 119 (171 with the single tokens in chunks as well), 163 and 136 (153), 108
-    and 94 (117): a step of 256 tokens and more spreads its blocks over the SMs one by one, which single tokens have no use for."""
+    retention of 16 of 128 x 128): one portion of 64 tokens 25 and 27, 25 and 27, 15 and 17; of 80 30 and 30, 30 and 29, 18 and 19; of 128
+    43 and 39, 45 and 37, 26 and 25; of 1,024 224 and 152, 228 and 144, 119 and 108; eight of 16 27 and 30, 34 and 34, 16 and 19; four of 64
+    65 and 54, 58 and 53, 35 and 38; eight of 32 63 and 61, 60 and 57, 35 and 41.  24 single tokens beside 200 71 and 84, 82 and 100, 43 and
+    60; beside 391 and 130 164 and 119 (171 with the single tokens in chunks as well), 163 and 136 (153), 108 and 94 (117): a step of 256
+    tokens and more spreads its blocks over the SMs one by one, which short requests have no use for."""
     if mixer.dtype != torch.bfloat16 or ctx.all_single_token:
         return 0
     captured = ctx.extras.get("captured_portions")
-    long, singles = (captured["long"], captured["singles"]) if captured is not None else (ctx.max_q_len >= CHUNKS_FROM, 1 in ctx.q_lens_host)
-    if not long or (singles and ctx.num_tokens < CHUNKS_BESIDE_FROM):
-        return 0
-    return 2 if singles else 1
+    if captured is not None:
+        portions, singles = captured["long"], captured["singles"]
+    else:
+        portions, singles = portions_class(ctx.max_q_len, ctx.num_tokens, CHUNKS_FROM), 1 in ctx.q_lens_host
+    if singles:
+        return 2 if portions == 2 and ctx.num_tokens >= CHUNKS_BESIDE_FROM else 0
+    return 1 if portions == 2 or (portions == 1 and short_portions) else 0
 
 
 class Mamba2Mixer(Mixer):
@@ -159,7 +163,7 @@ class Mamba2Mixer(Mixer):
             rec_ops.FORM_STEP_SIZE, q=xbc[:, inner + gn :], k=xbc[:, inner : inner + gn], v=xbc[:, :inner],
             pre=proj[:, inner + self.channels :], p0=self.dt_bias, p1=self.a_log, p2=self.skip, view=view,
             offset=self.scan_offset, ctx=ctx, heads=self.heads, dk=self.state_size, dv=self.vdim,
-            heads_per_group=self.heads // self.groups, chunks=takes_chunks(self, ctx))
+            heads_per_group=self.heads // self.groups, chunks=takes_chunks(self, ctx, short_portions=True))
         out = rec_ops.gated_group_norm(y, proj[:, :inner], self.norm_w, self.norm_groups, self.eps, True, self.dtype)
         return self.o.add_or_defer(out, stream)
 
@@ -464,7 +468,7 @@ class HeadDeltaMixer(_DeltaRule):
         proj = self.w_in.to_float32(x)  # [N, q | k | v | gate | beta | decay], float32
         o = rec_ops.head_delta(proj, self.conv_w, proj[:, c + i : c + i + h], proj[:, c + i + h :], self.dt_bias, self.a_log, view,
                                self.scan_offset, self.conv_offset, ctx, self.kv_heads, h, self.dim, self.vdim, self.UNIT_EPS,
-                               self.dim ** -0.5, chunks=takes_chunks(self, ctx))
+                               self.dim ** -0.5, chunks=takes_chunks(self, ctx, short_portions=True))
         return rec_ops.gated_group_norm(o, proj[:, c : c + i], self.norm_w, h, self.eps, False, self.dtype, gate=rec_ops.GATE_SILU,
                                         shared_weight=True)
 
