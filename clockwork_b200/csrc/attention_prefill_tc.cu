@@ -259,7 +259,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
             }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---- MMA issuer --------------------------------------------------------------------------------
         constexpr uint32_t idesc_s = instr_desc(AQ, AK);
         constexpr uint32_t idesc_o = instr_desc(AQ, HD) | (1u << 16);  // B (= V) is MN-major

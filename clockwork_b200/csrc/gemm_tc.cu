@@ -22,7 +22,7 @@
 //                              also few tokens against three rounds of weight tiles or more (the logits)
 //   gemm_tc_pair_kernel        the same on CTA pairs (cta_group::2), in gemm_tc_pair.cuh
 //
-// Warp roles of gemm_tc_kernel (128 threads): warp 0 lane 0 issues TMA loads, warp 1 lane 0 issues the
+// Warp roles of gemm_tc_kernel (128 threads): a lane of warp 0 issues TMA loads, a lane of warp 1 the
 // MMAs, warp 2 allocates and frees TMEM; all four warps run the epilogue (warp w reads TMEM lanes
 // 32w..32w+31).  Epilogues: 0 store bf16; 1 add into the float32 residual; 2 store float32; SWIGLU
 // computes silu(X Wg^T) * (X Wu^T) from two accumulators; an RMSNorm can be split over the two products
@@ -167,14 +167,16 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (p.splits > 1) cluster_sync();
 
     int issued = 0;
-    if (warp == 0 && lane == 0) {
+    const bool elected = elect_one();
+    if (warp == 0 && elected) {
         // ---- TMA producer ----------------------------------------------------------------------
         // Weight tiles of the first stages go out before the wait on the preceding kernel: no
         // kernel of the step writes weights, so they stream while that kernel finishes.  The
         // activation tiles (which it may still be writing) follow after the wait.
         const int early = min(my_kb, C::STAGES);
+        const uint32_t smem0 = smem_u32(smem);
         for (int i = 0; i < early; ++i) {
-            const uint32_t a_dst = smem_u32(smem + i * C::STAGE_BYTES);
+            const uint32_t a_dst = smem0 + i * C::STAGE_BYTES;
             const uint32_t bar = full0 + 8 * i;
             mbar_expect_tx(bar, C::STAGE_BYTES);
             const int kx = (kb0 + i) * BK;
@@ -182,16 +184,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (SWIGLU) tma_load_2d(a_dst + C::A_BYTES, &map_w2, kx, m0, bar);
         }
         pdl_wait();
-        for (int i = 0; i < early; ++i) {
-            const uint32_t a_dst = smem_u32(smem + i * C::STAGE_BYTES);
-            tma_load_2d(a_dst + C::A_BYTES * (SWIGLU ? 2 : 1), &map_x, (kb0 + i) * BK, n0, full0 + 8 * i);
-            ++issued;
-        }
+        for (int i = 0; i < early; ++i)
+            tma_load_2d(smem0 + i * C::STAGE_BYTES + C::A_BYTES * (SWIGLU ? 2 : 1), &map_x, (kb0 + i) * BK, n0, full0 + 8 * i);
+        issued = early;
+        int s = 0;            // the stage, and the parity of its barriers' phase, counted along (no division per k-block)
+        uint32_t parity = 0;
         for (int i = early; i < my_kb; ++i) {
-            const int s = i % C::STAGES;
-            const uint32_t parity = ((i / C::STAGES) & 1) ^ 1;
             if (!mbar_wait(empty0 + 8 * s, parity, give_up)) break;
-            const uint32_t a_dst = smem_u32(smem + s * C::STAGE_BYTES);
+            const uint32_t a_dst = smem0 + s * C::STAGE_BYTES;
             const uint32_t bar = full0 + 8 * s;
             mbar_expect_tx(bar, C::STAGE_BYTES);
             const int kx = (kb0 + i) * BK;
@@ -199,21 +199,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
             if (SWIGLU) tma_load_2d(a_dst + C::A_BYTES, &map_w2, kx, m0, bar);
             tma_load_2d(a_dst + C::A_BYTES * (SWIGLU ? 2 : 1), &map_x, kx, n0, bar);
             ++issued;
+            if (++s == C::STAGES) {
+                s = 0;
+                parity ^= 1;
+            }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elected) {
         // ---- MMA issuer ------------------------------------------------------------------------
         pdl_wait();  // blocked here a thread costs nothing; polling a barrier takes issue slots
         constexpr uint32_t idesc = instr_desc(BM, BN);
+        const uint64_t desc0 = smem_desc_sw128(smem_u32(smem));
+        uint64_t adesc = desc0;  // (16-byte units: a stage further is STAGE_BYTES / 16)
+        int s = 0;
+        uint32_t parity = 0;
         bool ok = true;
-        for (int i = 0; i < my_kb && ok; ++i) {
-            const int s = i % C::STAGES;
-            ok = mbar_wait(full0 + 8 * s, (i / C::STAGES) & 1, give_up);
+        for (int i = 0; i < my_kb; ++i) {
+            ok = mbar_wait(full0 + 8 * s, parity, give_up);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-            const uint64_t adesc = smem_desc_sw128(a_addr);
-            const uint64_t a2desc = smem_desc_sw128(a_addr + C::A_BYTES);
-            const uint64_t bdesc = smem_desc_sw128(a_addr + C::A_BYTES * (SWIGLU ? 2 : 1));
+            const uint64_t a2desc = adesc + C::A_BYTES / 16;
+            const uint64_t bdesc = adesc + C::A_BYTES * (SWIGLU ? 2 : 1) / 16;
 #pragma unroll
             for (int k = 0; k < BK / 16; ++k) {
                 // 16 bf16 = 32 bytes further along K inside the swizzle atom: +2 in 16-byte units
@@ -222,6 +227,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
                 if (SWIGLU) umma_bf16(tmem_base + BN, a2desc + 2 * k, bdesc + 2 * k, idesc, acc);
             }
             umma_commit(empty0 + 8 * s);  // frees the stage when these MMAs have read it
+            adesc += C::STAGE_BYTES / 16;
+            if (++s == C::STAGES) {
+                s = 0;
+                parity ^= 1;
+                adesc = desc0;
+            }
         }
         if (ok) umma_commit(acc_bar);
     }
@@ -451,7 +462,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     // ---- teardown ---------------------------------------------------------------------------------
     if (*give_up) {
         if (tid == 0) cw_report(p.status, CW_ST_WAIT_TIMEOUT, blockIdx.x, blockIdx.z);
-        if (warp == 0 && lane == 0) {
+        if (warp == 0 && elected) {
             // wait, bounded, for the copies still in flight before the CTA's shared memory goes away
             for (int i = max(0, issued - C::STAGES); i < issued; ++i) {
                 const uint32_t bar = full0 + 8 * (i % C::STAGES);
@@ -539,7 +550,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- TMA producer: runs ahead over tiles, bounded by the ring only ----------------------------
         const int my_tiles = (int)blockIdx.x < tiles ? (tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
         const int total = my_tiles * p.num_kb;  // k-blocks of all this CTA's tiles, in order
@@ -563,20 +574,25 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                 }
             }
         }
-        // the rest runs ahead over tiles, bounded by the ring only
-        int kb = early % p.num_kb;
+        // the rest runs ahead over tiles, bounded by the ring only; the stage and its phase are counted along
+        int kb = early % p.num_kb, s = early % C::STAGES;
+        uint32_t parity = early < C::STAGES ? 1 : 0;
+        const uint32_t smem0 = smem_u32(smem);
         for (int tile = blockIdx.x + (early / p.num_kb) * gridDim.x; tile < tiles && ok; tile += gridDim.x, kb = 0) {
             const int m0 = (tile / n_tiles) * BM, n0 = (tile % n_tiles) * bn;
             for (; kb < p.num_kb; ++kb, ++i) {
-                const int s = i % C::STAGES;
-                ok = mbar_wait(empty0 + 8 * s, ((i / C::STAGES) & 1) ^ 1, give_up);
+                ok = mbar_wait(empty0 + 8 * s, parity, give_up);
                 if (!ok) break;
-                const uint32_t a_dst = smem_u32(smem + s * C::STAGE_BYTES);
+                const uint32_t a_dst = smem0 + s * C::STAGE_BYTES;
                 const uint32_t bar = full0 + 8 * s;
                 mbar_expect_tx(bar, stage_tx);
                 tma_load_2d(a_dst, &map_w, kb * BK, m0, bar);
                 if (SWIGLU) tma_load_2d(a_dst + C::A_BYTES, &map_w2, kb * BK, m0, bar);
                 tma_load_2d(a_dst + C::A_BYTES * (SWIGLU ? 2 : 1), &map_x, kb * BK, n0, bar);
+                if (++s == C::STAGES) {
+                    s = 0;
+                    parity ^= 1;
+                }
             }
         }
         if (*give_up) {
@@ -588,11 +604,14 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                 }
             }
         }
-    } else if (warp == 1 && lane == 0) {
+    } else if (warp == 1 && elect_one()) {
         // ---- MMA issuer: tile `it` accumulates into TMEM buffer it & 1 -------------------------------
         pdl_wait();  // (nothing to do before the producer's activations arrive; parked here a thread polls no barrier)
         const uint32_t idesc = instr_desc(BM, bn);
-        int i = 0, it = 0;
+        const uint64_t desc0 = smem_desc_sw128(smem_u32(smem));
+        uint64_t adesc = desc0;  // (16-byte units: a stage further is STAGE_BYTES / 16)
+        int it = 0, s = 0;
+        uint32_t parity = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++it) {
             const int buf = it & 1;
@@ -600,15 +619,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = tmem_base + buf * C::ACC_COLS;
-            for (int kb = 0; kb < p.num_kb; ++kb, ++i) {
-                const int s = i % C::STAGES;
-                ok = mbar_wait(full0 + 8 * s, (i / C::STAGES) & 1, give_up);
+            for (int kb = 0; kb < p.num_kb; ++kb) {
+                ok = mbar_wait(full0 + 8 * s, parity, give_up);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-                const uint64_t adesc = smem_desc_sw128(a_addr);
-                const uint64_t a2desc = smem_desc_sw128(a_addr + C::A_BYTES);
-                const uint64_t bdesc = smem_desc_sw128(a_addr + C::A_BYTES * (SWIGLU ? 2 : 1));
+                const uint64_t a2desc = adesc + C::A_BYTES / 16;
+                const uint64_t bdesc = adesc + C::A_BYTES * (SWIGLU ? 2 : 1) / 16;
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k) {
                     const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
@@ -616,6 +632,12 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                     if (SWIGLU) umma_bf16(acc + BN, a2desc + 2 * k, bdesc + 2 * k, idesc, accumulate);
                 }
                 umma_commit(empty0 + 8 * s);
+                adesc += C::STAGE_BYTES / 16;
+                if (++s == C::STAGES) {
+                    s = 0;
+                    parity ^= 1;
+                    adesc = desc0;
+                }
             }
             if (ok) umma_commit(accf0 + 8 * buf);
         }

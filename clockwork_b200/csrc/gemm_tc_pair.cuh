@@ -135,18 +135,17 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && elect_one()) {
         // ---- TMA producer (both CTAs): own rows of W, own half of the token tile ------------------------
         const uint32_t stage_tx = B_OFF + half_bn * BK * 2;
         const int my_tiles = pair < tiles ? (tiles - pair + pairs - 1) / pairs : 0;
         const int total = my_tiles * nkb;  // k-blocks of all this pair's units, in order
         const int early = min(total, C::STAGES);
         bool ok = true;
-        int i = 0;
         // the first stages: weight tiles before the wait, their activation tiles after it
         for (int phase = 0; phase < 2; ++phase) {
             if (phase == 1) pdl_wait();
-            for (i = 0; i < early; ++i) {
+            for (int i = 0; i < early; ++i) {
                 const int ts = i / nkb, unit = pair + ts * pairs, tile = unit / splits;
                 const int kb = (unit - tile * splits) * nkb + (i - ts * nkb);  // k-block within K
                 const int m0 = (tile % m_tiles) * 2 * BM + (int)rank * BM;
@@ -162,22 +161,27 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
                 }
             }
         }
-        // the rest runs ahead over tiles, bounded by the ring only
-        int kb = early % nkb;
+        // the rest runs ahead over tiles, bounded by the ring only; the stage and its phase are counted along
+        int kb = early % nkb, s = early % C::STAGES;
+        uint32_t parity = early < C::STAGES ? 1 : 0;
+        const uint32_t smem0 = smem_u32(smem), leader_full0 = dsmem_addr(full0, 0);
         for (int unit = pair + (early / nkb) * pairs; unit < tiles && ok; unit += pairs, kb = 0) {
             const int tile = unit / splits, kb0 = (unit - tile * splits) * nkb;
             const int m0 = (tile % m_tiles) * 2 * BM + (int)rank * BM;
             const int n0 = (tile / m_tiles) * bn + (int)rank * half_bn;
-            for (; kb < nkb; ++kb, ++i) {
-                const int s = i % C::STAGES;
-                ok = mbar_wait(empty0 + 8 * s, ((i / C::STAGES) & 1) ^ 1, give_up);
+            for (; kb < nkb; ++kb) {
+                ok = mbar_wait(empty0 + 8 * s, parity, give_up);
                 if (!ok) break;
-                const uint32_t a_dst = smem_u32(smem + s * C::STAGE_BYTES);
-                const uint32_t bar = dsmem_addr(full0 + 8 * s, 0);  // the leader's barrier
+                const uint32_t a_dst = smem0 + s * C::STAGE_BYTES;
+                const uint32_t bar = leader_full0 + 8 * s;
                 mbar_expect_tx_cluster(bar, stage_tx);
                 tma_load_2d_pair(a_dst, &map_w, (kb0 + kb) * BK, m0, bar);
                 if (SWIGLU) tma_load_2d_pair(a_dst + C::A_BYTES, &map_w2, (kb0 + kb) * BK, m0, bar);
                 tma_load_2d_pair(a_dst + B_OFF, &map_x, (kb0 + kb) * BK, n0, bar);
+                if (++s == C::STAGES) {
+                    s = 0;
+                    parity ^= 1;
+                }
             }
         }
         if (*give_up) {
@@ -187,11 +191,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             while (clock64() - t0 < 2000000LL) {
             }
         }
-    } else if (warp == 1 && lane == 0 && rank == 0) {
+    } else if (warp == 1 && rank == 0 && elect_one()) {
         // ---- MMA issuer (leader only): tile `it` accumulates into TMEM buffer it & 1 of both CTAs ---------
         pdl_wait();  // (parked here a thread polls no barrier)
         const uint32_t idesc = instr_desc(2 * BM, bn);
-        int i = 0, it = 0;
+        const uint64_t desc0 = smem_desc_sw128(smem_u32(smem));
+        uint64_t adesc = desc0;  // (16-byte units: a stage further is STAGE_BYTES / 16)
+        int it = 0, s = 0;
+        uint32_t parity = 0;
         bool ok = true;
         for (int tile = pair; tile < tiles && ok; tile += pairs, ++it) {
             const int buf = it & 1;
@@ -199,24 +206,26 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = tmem_base + buf * C::ACC_STRIDE;
-            for (int kb = 0; kb < nkb; ++kb, ++i) {
-                const int s = i % C::STAGES;
-                ok = mbar_wait(full0 + 8 * s, (i / C::STAGES) & 1, give_up);
+            for (int kb = 0; kb < nkb; ++kb) {
+                ok = mbar_wait(full0 + 8 * s, parity, give_up);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t a_addr = smem_u32(smem + s * C::STAGE_BYTES);
-                const uint64_t adesc = smem_desc_sw128(a_addr);
-                const uint64_t bdesc = smem_desc_sw128(a_addr + B_OFF);
+                const uint64_t udesc = adesc + C::A_BYTES / 16, bdesc = adesc + B_OFF / 16;
 #pragma unroll
                 for (int k = 0; k < BK / 16; ++k)
                     umma_bf16_pair(acc, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                 if (SWIGLU) {
-                    const uint64_t udesc = smem_desc_sw128(a_addr + C::A_BYTES);
 #pragma unroll
                     for (int k = 0; k < BK / 16; ++k)
                         umma_bf16_pair(acc + C::ACC_STRIDE / 2, udesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
                 }
                 umma_commit_pair(empty0 + 8 * s);  // the stage is free in both CTAs
+                adesc += C::STAGE_BYTES / 16;
+                if (++s == C::STAGES) {
+                    s = 0;
+                    parity ^= 1;
+                    adesc = desc0;
+                }
             }
             if (ok) umma_commit_pair(accf0 + 8 * buf);
         }

@@ -190,9 +190,12 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMA issuer: the walk's tile `it` accumulates into buffer it & 1 ---------------------------------
-            int i = 0, it = 0;
+            const uint64_t desc0 = smem_desc_sw128(smem_u32(smem));
+            uint64_t adesc = desc0;  // (16-byte units: a stage further is STAGE_BYTES / 16)
+            int it = 0, s = 0;
+            uint32_t parity = 0;
             bool ok = true;
             for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x, ++it) {
                 const uint32_t idesc = instr_desc(GT_BM, gt_tile(p, cum, first, ftiles, t).width);
@@ -201,14 +204,11 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc = tmem_base + buf * C::ACC_COLS;
-                for (int kb = 0; kb < num_kb; ++kb, ++i) {
-                    const int s = i % C::STAGES;
-                    ok = mbar_wait(full0 + 8 * s, (i / C::STAGES) & 1, give_up);
+                for (int kb = 0; kb < num_kb; ++kb) {
+                    ok = mbar_wait(full0 + 8 * s, parity, give_up);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t w_addr = smem_u32(smem + s * C::STAGE_BYTES);
-                    const uint64_t adesc = smem_desc_sw128(w_addr), a2desc = smem_desc_sw128(w_addr + C::W_BYTES / 2);
-                    const uint64_t bdesc = smem_desc_sw128(w_addr + C::W_BYTES);
+                    const uint64_t a2desc = adesc + C::W_BYTES / 2 / 16, bdesc = adesc + C::W_BYTES / 16;
 #pragma unroll
                     for (int k = 0; k < GT_BK / 16; ++k) {
                         const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
@@ -216,6 +216,12 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                         if (TWO) umma_bf16(acc + BN, a2desc + 2 * k, bdesc + 2 * k, idesc, accumulate);
                     }
                     umma_commit(empty0 + 8 * s);
+                    adesc += C::STAGE_BYTES / 16;
+                    if (++s == C::STAGES) {
+                        s = 0;
+                        parity ^= 1;
+                        adesc = desc0;
+                    }
                 }
                 if (ok) umma_commit(accf0 + 8 * buf);
             }

@@ -176,7 +176,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMA issuer ---------------------------------------------------------------------------------------
             constexpr uint32_t idesc_s = instr_desc(LC_ROWS, LC_KEYS);
             const uint32_t idesc_o = instr_desc(LC_ROWS, cols) | (1u << 16);  // B is MN-major

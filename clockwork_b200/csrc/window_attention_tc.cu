@@ -182,7 +182,7 @@ window_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             settle(aux, partial & 1);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             // ---- MMA issuer ---------------------------------------------------------------------------------------
             constexpr uint32_t idesc_s = instr_desc(WC_ROWS, WC_KEYS);
             const uint32_t idesc_o = instr_desc(WC_ROWS, dv) | (1u << 16);  // B is MN-major
