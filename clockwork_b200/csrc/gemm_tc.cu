@@ -33,6 +33,7 @@
 // the status words, the producer waits (bounded again) for the copies it has in flight, TMEM is
 // freed and the kernel returns.
 #include "tc_common.cuh"
+#include <atomic>
 #include <type_traits>
 
 #define BM 128
@@ -92,7 +93,8 @@ __device__ __forceinline__ float gated_act(float g, float u, float limit) {
 
 #include "gemm_tc_pair.cuh"
 
-template <int BN, bool SWIGLU>
+// PER_SM: how many CTAs an SM is meant to hold (2: up to 64 tokens without SwiGLU, with as many stages as half of the shared memory has room for).
+template <int BN, bool SWIGLU, int PER_SM = 1>
 struct Cfg {
     static constexpr int A_BYTES = BM * BK * 2;                     // 16 KB
     static constexpr int B_BYTES = BN * BK * 2;
@@ -107,19 +109,20 @@ struct Cfg {
     // tiles in flight from HBM
     // Small token tiles without SwiGLU (the decode products around attention) leave room for a CTA of
     // the decode attention kernel beside them, so that its prologue runs while this kernel finishes.
-    static constexpr int BUDGET = (BN <= 64 && !SWIGLU) ? 140 * 1024 : 200 * 1024;
+    static constexpr int BUDGET = PER_SM == 2 ? 110 * 1024 : (BN <= 64 && !SWIGLU) ? 140 * 1024 : 200 * 1024;
     static constexpr int MAX_STAGES = (BUDGET - INBOX_BYTES) / STAGE_BYTES;
     static constexpr int STAGES = MAX_STAGES > 8 ? 8 : MAX_STAGES;
     static constexpr int TMEM_COLS = ACC_COLS <= 32 ? 32 : (ACC_COLS <= 64 ? 64 : (ACC_COLS <= 128 ? 128 : (ACC_COLS <= 256 ? 256 : 512)));
     static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + INBOX_BYTES + 1024 /*alignment*/ + 1024 /*barriers*/;
+    static_assert(PER_SM == 1 || (BN <= 64 && !SWIGLU && 2 * (SMEM_BYTES + 1024) <= 228 * 1024), "two CTAs share an SM");
 };
 
-template <int BN, bool SWIGLU>
+template <int BN, bool SWIGLU, int PER_SM = 1>
 __global__ void __launch_bounds__(THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2,
                const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_c,
                const GemmParams p) {
-    using C = Cfg<BN, SWIGLU>;
+    using C = Cfg<BN, SWIGLU, PER_SM>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t* bars = (uint64_t*)(smem + C::STAGES * C::STAGE_BYTES);
@@ -751,6 +754,7 @@ static int make_map_c(CUtensorMap* map, const void* ptr, int T, int N, long long
 
 struct Plan {
     int bn, splits, kb_per_split, tiles;
+    int per_sm;       // CTAs an SM is to hold (gemm_tc_kernel with splits)
     bool persistent;  // bn is then any multiple of 16 and the persistent kernel runs
     bool pair;        // ... on CTA pairs: tiles of 256 features
     bool stream;      // few tokens, many rounds of weight tiles (a vocabulary): the persistent kernel with narrow tiles
@@ -895,6 +899,37 @@ extern "C" int cw_gemm_tc_set_persistent_from(int tokens) {
     return CW_OK;
 }
 
+// How many clusters of `size` CTAs of gemm_tc_kernel the GPU holds at a time, with one CTA or two to an SM.  A cluster lies
+// within one group of SMs (GPC), so that the counts are well below SMs / size and differ from part to part: the driver is asked
+// once per size (148 SMs, one CTA to an SM: 74, 45, 33, 26, 22, 15 and 15 clusters of 2 to 8; two: 148, 93, 71, 56, 45, 37 and 33).
+// It is asked about an empty kernel with the same threads and shared memory: of kernels that allocate tensor memory the
+// occupancy calculator says one CTA to an SM whatever they hold.
+__global__ void __launch_bounds__(THREADS) cluster_places_kernel() {}
+static int clusters_at_once(int size, int per_sm, int sm_count) {
+    static std::atomic<int> known[2][MAX_SPLITS + 1];
+    if (size <= 1) return per_sm * sm_count;
+    int n = known[per_sm - 1][size].load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    const int smem = per_sm == 2 ? Cfg<64, false, 2>::SMEM_BYTES : MAX_SMEM_BYTES;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = cluster.val.clusterDim.y = 1;
+    cluster.val.clusterDim.z = size;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1, 1, size);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(cluster_places_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM_BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, cluster_places_kernel, &cfg) != cudaSuccess || n <= 0) {
+        (void)cudaGetLastError();
+        return per_sm * sm_count / size;  // (no answer: as if clusters could lie anywhere)
+    }
+    known[per_sm - 1][size].store(n, std::memory_order_relaxed);
+    return n;
+}
+
 static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_tma = true, bool adds = false) {
     Plan pl;
     pl.persistent = T >= g_persistent_from && sm_count > 0 && c_by_tma;  // its epilogue has no other way out than TMA
@@ -914,6 +949,7 @@ static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_
     const int num_kb = (K + BK - 1) / BK;
     int splits = 1;
     const bool can_split = pl.bn <= 64 || (pl.bn == 128 && !swiglu);  // Cfg::CAN_SPLIT
+    pl.per_sm = 1;
     if (!pl.persistent && can_split && pl.tiles * 2 <= sm_count) {
         // One wave: as many CTAs as SMs at most, each with as much of K as possible.  A CTA costs a
         // few microseconds of set-up and epilogue whatever it streams, so fewer, longer CTAs win
@@ -923,6 +959,17 @@ static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_
         if (splits > max_by_k) splits = max_by_k;
         if (splits > MAX_SPLITS) splits = MAX_SPLITS;
         if (splits < 1) splits = 1;
+        // Where the clusters do not find a place each at once (see clusters_at_once), two CTAs share an SM; what has no form for
+        // that is cut in fewer parts.  Measured (B200, N x K: us a product in two waves -> so): 8 tokens, 2048 x 2048 8.2 ->
+        // 4.3, 2048 x 5632 12.1 -> 7.2, 3584 x 3584 9.7 -> 7.4, 4608 x 3584 13.1 -> 8.5, 3584 x 18944 33.0 -> 25.1; 64 tokens,
+        // the last three 17.7, 18.2 and 50.0 -> 10.9, 11.8 and 32.2; 128 tokens 23.9, 23.5 and 57.4 -> 14.1, 14.4 and 36.6.  Fewer parts
+        // with one CTA to an SM are about as fast (8 tokens: 4.4, 6.9, 6.9, 8.5, 24.2), but add up in another order.
+        if (pl.tiles > clusters_at_once(splits, 1, sm_count)) {
+            if (pl.bn <= 64 && !swiglu && pl.tiles <= clusters_at_once(splits, 2, sm_count))
+                pl.per_sm = 2;
+            else
+                while (splits > 1 && pl.tiles > clusters_at_once(splits, 1, sm_count)) --splits;
+        }
     }
     pl.kb_per_split = (num_kb + splits - 1) / splits;
     pl.splits = (num_kb + pl.kb_per_split - 1) / pl.kb_per_split;  // no empty split
@@ -938,21 +985,21 @@ static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_
     return pl;
 }
 
-template <int BN, bool SWIGLU>
+template <int BN, bool SWIGLU, int PER_SM = 1>
 static int launch(const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensorMap& mx, const CUtensorMap& mc,
                   const GemmParams& p, dim3 grid, cudaStream_t stream) {
-    using C = Cfg<BN, SWIGLU>;
+    using C = Cfg<BN, SWIGLU, PER_SM>;
     static_assert(C::ACC_COLS * BM * 4 <= C::STAGES * C::STAGE_BYTES, "a staged tile must fit in the operand stages");
     static_assert(C::STAGES >= 2, "too few operand stages");
     if (grid.z > 1 && !C::CAN_SPLIT) return CW_ERR_UNSUPPORTED;
     static bool configured = false;
     if (!configured) {
-        if (cudaFuncSetAttribute(gemm_tc_kernel<BN, SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        if (cudaFuncSetAttribute(gemm_tc_kernel<BN, SWIGLU, PER_SM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  C::SMEM_BYTES) != cudaSuccess)
             return (int)cudaGetLastError();
         configured = true;
     }
-    return cw_launch(gemm_tc_kernel<BN, SWIGLU>, grid, dim3(THREADS), C::SMEM_BYTES, stream, grid.z, mw, mw2, mx, mc, p);
+    return cw_launch(gemm_tc_kernel<BN, SWIGLU, PER_SM>, grid, dim3(THREADS), C::SMEM_BYTES, stream, grid.z, mw, mw2, mx, mc, p);
 }
 
 template <bool SWIGLU>
@@ -1091,6 +1138,10 @@ static int gemm_tc_run(const void* X, const void* W, const void* W2, const float
     case bn:                                                                              \
         return swiglu ? launch<bn, true>(mw, mw2, mx, mc, p, grid, stream)                \
                       : launch<bn, false>(mw, mw2, mx, mc, p, grid, stream);
+    if (pl.per_sm == 2)
+        return pl.bn == 16   ? launch<16, false, 2>(mw, mw2, mx, mc, p, grid, stream)
+               : pl.bn == 32 ? launch<32, false, 2>(mw, mw2, mx, mc, p, grid, stream)
+                             : launch<64, false, 2>(mw, mw2, mx, mc, p, grid, stream);
     switch (pl.bn) {
         CW_CASE(16)
         CW_CASE(32)

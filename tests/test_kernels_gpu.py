@@ -691,6 +691,14 @@ def test_gemm_tc_few_tokens_over_many_weight_tiles(ops, gemm_tc, t, n, k):
     assert torch.equal(walked, per_tile)
 
 
+@pytest.mark.parametrize("t,n,k", [(1, 2048, 2048), (16, 3584, 1544), (17, 2000, 2056), (32, 4608, 1032), (33, 3500, 1288), (64, 2048, 2104),
+                                   (64, 3584, 1288), (65, 3584, 1288), (128, 2048, 2048)])
+def test_gemm_tc_splits_beyond_one_cta_per_sm(ops, gemm_tc, t, n, k):
+    """Weight tiles times splits that no single wave of clusters holds with a CTA to an SM: two share one up to 64 tokens,
+    more tokens are cut in fewer parts."""
+    test_gemm_tc_against_float64(ops, gemm_tc, t, n, k)
+
+
 @pytest.mark.parametrize("t,n,k", TC_SHAPES)
 def test_gemm_tc_against_float64(ops, gemm_tc, t, n, k):
     x, w, bias = rand(t, k, dtype=torch.bfloat16), rand(n, k, dtype=torch.bfloat16, scale=0.1, seed=1), rand(n, seed=2)
