@@ -68,7 +68,7 @@ struct GemmParams {
     const float* emit_g;      // [N] or null
     bf16* emit_x;             // [T, N]
     float* emit_part;         // [T, gridDim.x]
-    int* split_flags;         // CTA-pair kernel with splits > 1: two words per tile, zero between launches
+    int* split_flags;         // CTA-pair kernel with splits > 1: sixteen words per tile (one per epilogue warp), zero between launches
     float act_limit;          // SWIGLU only.  0: silu(gate) * up.  Positive: the clamped form (gated_act)
     int squared_relu;         // not SWIGLU, epilogue 0: max(v, 0)^2 of v = product + bias is stored instead of v
 };
@@ -760,18 +760,41 @@ struct Plan {
     bool stream;      // few tokens, many rounds of weight tiles (a vocabulary): the persistent kernel with narrow tiles
 };
 
-// Token-tile width for CTA pairs: per k-block a pair-tile costs about max(2 bn, 256 + bn) cycles (MMA
-// time, shared-memory traffic) and the pairs run ceil(tiles / pairs) rounds.
-static int balanced_bn_pair(int T, int N, int sm_count, bool swiglu = false) {
+// About how long a CTA-pair product takes with token tiles of bn and K cut in `splits` (in ns, without its set-up): a k-block 1.3
+// bn for the MMAs and at least 180 for a stage's round trip, (60 + bn) of the share of pairs at work for what they draw from L2
+// together, and 600 a round.  Fitted to 2,140 timings (B200, 150 to 3,000 tokens, the products of the named shapes, every
+// width): the widths that it picks are 1.8 % slower than the best on average.
+static long long pair_cost(int bn, int T, int N, int num_kb, int splits, int sm_count) {
+    const long long pairs = sm_count / 2, units = (long long)((N + 2 * BM - 1) / (2 * BM)) * ((T + bn - 1) / bn) * splits;
+    const long long rounds = (units + pairs - 1) / pairs;
+    long long kb = 13 * bn / 10;
+    if (kb < 180) kb = 180;
+    const long long drawn = (60 + bn) * units / (rounds * pairs);
+    if (kb < drawn) kb = drawn;
+    return rounds * (num_kb / splits * kb + 600);
+}
+// Token-tile width for CTA pairs, K being cut in `splits`: the least time, the wider tile on a tie.  (The width decides nothing
+// about the result: every output's sum runs over the k-blocks of its split in order.)
+static int balanced_bn_pair(int T, int N, int num_kb, int splits, int sm_count) {
+    long long best_cost = -1;
+    int best = 256;
+    for (int bn = 256; bn >= 64; bn -= 16) {
+        const long long cost = pair_cost(bn, T, N, num_kb, splits, sm_count);
+        if (best_cost < 0 || cost < best_cost) {
+            best_cost = cost;
+            best = bn;
+        }
+    }
+    return best;
+}
+// The same for SwiGLU on CTA pairs (two accumulators per tile, two weight tiles per k-block): a k-block about max(4 bn, 512 + bn) cycles.
+static int balanced_bn_pair_swiglu(int T, int N, int sm_count) {
     const int m_tiles = (N + 2 * BM - 1) / (2 * BM), pairs = sm_count / 2;
     long long best_cost = -1;
-    const int cap = swiglu ? 128 : 256;  // (SwiGLU: two accumulators per tile, two weight tiles per k-block)
-    int best = cap;
-    for (int bn = cap; bn >= 64; bn -= 16) {
-        const long long tiles = (long long)m_tiles * ((T + bn - 1) / bn);
-        const long long rounds = (tiles + pairs - 1) / pairs;
-        const long long cost = swiglu ? rounds * (4 * bn > 512 + bn ? 4 * bn : 512 + bn)
-                                      : rounds * (2 * bn > 256 + bn ? 2 * bn : 256 + bn);
+    int best = 128;
+    for (int bn = 128; bn >= 64; bn -= 16) {
+        const long long rounds = ((long long)m_tiles * ((T + bn - 1) / bn) + pairs - 1) / pairs;
+        const long long cost = rounds * (4 * bn > 512 + bn ? 4 * bn : 512 + bn);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
             best = bn;
@@ -821,21 +844,20 @@ extern "C" int cw_gemm_tc_set_split_flags(int* words, int n) {
 // as leave no pair idle, dividing the k-blocks evenly, at least 16 k-blocks each, at most 8.
 static int pair_splits(int tiles, int num_kb, int sm_count) {
     const int pairs = sm_count / 2;
-    if (g_split_flags == nullptr || 2 * tiles > g_split_flags_n || tiles * 2 > pairs) return 1;
+    if (g_split_flags == nullptr || 2 * PAIR_EPI_WARPS * tiles > g_split_flags_n || tiles * 2 > pairs) return 1;
     int best = 1;
     for (int d = 2; d <= 8 && d * tiles <= pairs; ++d)
         if (num_kb % d == 0 && num_kb / d >= 16) best = d;
     return best;
 }
 
-// Token-tile width for a CTA-pair product that may be split over K.  Measured: a pair's k-block costs
-// about 330 + 0.2 bn nanoseconds whatever the tile's width (the stages in flight bound it), and the
-// splits of a tile store one after the other, each taking about 1000 + 25 bn nanoseconds (a turn of
-// the flag, bn / 16 chunks of stores).
-static int balanced_bn_pair_split(int T, int N, int num_kb, int sm_count) {
+// How many ways a CTA-pair product that adds into its output is cut over K.  The number decides the order of an output's sum, so
+// it follows from a rule of its own, in which a k-block of any width counts 330 + 0.2 bn ns and a split's turn to add 1000 + 25
+// bn, and does not move with the widths that the tiles then get (balanced_bn_pair).
+static int add_splits(int T, int N, int num_kb, int sm_count) {
     const int m_tiles = (N + 2 * BM - 1) / (2 * BM), pairs = sm_count / 2;
     long long best_cost = -1;
-    int best = 256;
+    int best = 1;
     for (int bn = 256; bn >= 64; bn -= 16) {
         const int tiles = m_tiles * ((T + bn - 1) / bn);
         const int splits = pair_splits(tiles, num_kb, sm_count);
@@ -843,7 +865,7 @@ static int balanced_bn_pair_split(int T, int N, int num_kb, int sm_count) {
         const long long cost = rounds * (num_kb / splits) * (330 + bn / 5) + splits * (1000LL + 25 * bn);
         if (best_cost < 0 || cost < best_cost) {
             best_cost = cost;
-            best = bn;
+            best = splits;
         }
     }
     return best;
@@ -851,9 +873,9 @@ static int balanced_bn_pair_split(int T, int N, int num_kb, int sm_count) {
 // A product whose splits over K are kept apart (epilogue 3): every split stores its partial tile in a
 // slab of its own and whoever reads the result next adds the slabs, in split order (the RMSNorm that
 // follows a product into the residual reads the residual anyway).  Nothing takes turns, so splits may
-// outnumber the pairs and run in rounds.  Cost as measured for the CTA-pair kernel: a k-block about
-// 330 + 0.2 bn ns, a tile's store 1000 + 25 bn ns once, and each further slab costs its reader about
-// T N / 500 ns (its bytes, written and read again).
+// outnumber the pairs and run in rounds.  The number of splits (which decides the order of the sums) follows from
+// a rule of its own as in add_splits: a k-block 330 + 0.2 bn ns, a tile's store 1000 + 25 bn ns once, and each
+// further slab costs its reader about T N / 500 ns (its bytes, written and read again).
 // Measured in the step (Qwen2.5-1.5B sizes, K = 8,960): 15 % of a 256-token prompt's time, 10 % at 512, 4 % at
 // 1,024; from 1,056 tokens on the slabs cost what the splits save (a mixed step of 1,056 tokens 5 % slower),
 // so longer products add into their output with splits that take turns, as before.
@@ -861,7 +883,7 @@ static int balanced_bn_pair_split(int T, int N, int num_kb, int sm_count) {
 static void parts_plan(int T, int N, int K, int sm_count, int* splits_out, int* bn_out) {
     const int m_tiles = (N + 2 * BM - 1) / (2 * BM), pairs = sm_count / 2, num_kb = (K + BK - 1) / BK;
     long long best_cost = -1;
-    int best_d = 1, best_bn = 256;
+    int best_d = 1;
     for (int bn = 256; bn >= 64; bn -= 16) {
         const int tiles = m_tiles * ((T + bn - 1) / bn);
         for (int d = 1; d <= 8; ++d) {
@@ -871,12 +893,11 @@ static void parts_plan(int T, int N, int K, int sm_count, int* splits_out, int* 
             if (best_cost < 0 || cost < best_cost) {
                 best_cost = cost;
                 best_d = d;
-                best_bn = bn;
             }
         }
     }
     *splits_out = best_d;
-    *bn_out = best_bn;
+    *bn_out = balanced_bn_pair(T, N, num_kb, best_d, sm_count);
 }
 
 // Forces the token-tile width of the prompt-portion kernels (0: chosen automatically); for measurements.
@@ -943,10 +964,13 @@ static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_
     pl.stream = !pl.persistent && !swiglu && T <= 64 && sm_count > 0 && c_by_tma &&
                 (long long)((N + BM - 1) / BM) >= 3LL * sm_count && g_stream_enabled;
     if (pl.stream) pl.persistent = true;
-    if (pl.persistent && !pl.stream) pl.bn = pl.pair ? balanced_bn_pair(T, N, sm_count, swiglu) : balanced_bn(T, N, swiglu, sm_count);
+    const int num_kb = (K + BK - 1) / BK;
+    if (pl.persistent && !pl.stream)
+        pl.bn = !pl.pair ? balanced_bn(T, N, swiglu, sm_count)
+                : swiglu ? balanced_bn_pair_swiglu(T, N, sm_count)
+                         : balanced_bn_pair(T, N, num_kb, 1, sm_count);
     if (pl.persistent && !pl.stream && g_forced_bn != 0 && (!swiglu || g_forced_bn <= 128)) pl.bn = g_forced_bn;
     pl.tiles = pl.pair ? ((N + 2 * BM - 1) / (2 * BM)) * ((T + pl.bn - 1) / pl.bn) : ((N + BM - 1) / BM) * ((T + pl.bn - 1) / pl.bn);
-    const int num_kb = (K + BK - 1) / BK;
     int splits = 1;
     const bool can_split = pl.bn <= 64 || (pl.bn == 128 && !swiglu);  // Cfg::CAN_SPLIT
     pl.per_sm = 1;
@@ -973,13 +997,16 @@ static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_
     }
     pl.kb_per_split = (num_kb + splits - 1) / splits;
     pl.splits = (num_kb + pl.kb_per_split - 1) / pl.kb_per_split;  // no empty split
-    if (pl.pair && adds && g_forced_bn == 0) {
-        // products that add into their output may be split over K when the tiles leave pairs idle
-        pl.bn = balanced_bn_pair_split(T, N, num_kb, sm_count);
-        pl.tiles = ((N + 2 * BM - 1) / (2 * BM)) * ((T + pl.bn - 1) / pl.bn);
-    }
     if (pl.pair && adds) {
-        pl.splits = pair_splits(pl.tiles, num_kb, sm_count);
+        // products that add into their output may be split over K when the tiles leave pairs idle
+        if (g_forced_bn == 0) {
+            pl.splits = add_splits(T, N, num_kb, sm_count);
+            pl.bn = balanced_bn_pair(T, N, num_kb, pl.splits, sm_count);
+            pl.tiles = ((N + 2 * BM - 1) / (2 * BM)) * ((T + pl.bn - 1) / pl.bn);
+        } else {
+            pl.splits = pair_splits(pl.tiles, num_kb, sm_count);
+        }
+        if (2 * PAIR_EPI_WARPS * pl.tiles > g_split_flags_n) pl.splits = 1;
         pl.kb_per_split = num_kb / pl.splits;
     }
     return pl;
@@ -1003,8 +1030,8 @@ static int launch(const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensorM
 }
 
 template <bool SWIGLU>
-static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensorMap& mx, const CUtensorMap& mc,
-                       const GemmParams& p, int pairs, cudaStream_t stream) {
+static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mw2, const CUtensorMap& mx, const GemmParams& p, int pairs,
+                       cudaStream_t stream) {
     using C = PairCfgT<SWIGLU>;
     static bool configured = false;
     if (!configured) {
@@ -1012,7 +1039,7 @@ static int launch_pair(const CUtensorMap& mw, const CUtensorMap& mw2, const CUte
             return (int)cudaGetLastError();
         configured = true;
     }
-    return cw_launch(gemm_tc_pair_kernel<SWIGLU>, dim3(2 * pairs), dim3(PAIR_THREADS), C::SMEM_BYTES, stream, 1, mw, mw2, mx, mc, p);
+    return cw_launch(gemm_tc_pair_kernel<SWIGLU>, dim3(2 * pairs), dim3(PAIR_THREADS), C::SMEM_BYTES, stream, 1, mw, mw2, mx, p);
 }
 
 template <int BN, bool SWIGLU>
@@ -1110,7 +1137,7 @@ static int gemm_tc_run(const void* X, const void* W, const void* W2, const float
     // prompt portions: the persistent kernel, whose epilogue overlaps the next tile's MMAs
     const bool persistent = pl.persistent;
     CUtensorMap mc = mx;
-    if (tma_store && make_map_c(&mc, C, T, N, ldc, persistent ? P_CHUNK : pl.bn, c_f32) != 0) return CW_ERR_UNSUPPORTED;
+    if (tma_store && !pl.pair && make_map_c(&mc, C, T, N, ldc, persistent ? P_CHUNK : pl.bn, c_f32) != 0) return CW_ERR_UNSUPPORTED;
     GemmParams p;
     p.tma_store = tma_store ? 1 : 0;
     p.T = T; p.N = N; p.K = K; p.ldc = ldc; p.epilogue = epilogue;
@@ -1126,7 +1153,7 @@ static int gemm_tc_run(const void* X, const void* W, const void* W2, const float
     if (pl.pair) {
         const int units = pl.tiles * pl.splits;
         const int pairs = units < sm_count / 2 ? units : sm_count / 2;
-        return swiglu ? launch_pair<true>(mw, mw2, mx, mc, p, pairs, stream) : launch_pair<false>(mw, mw2, mx, mc, p, pairs, stream);
+        return swiglu ? launch_pair<true>(mw, mw2, mx, p, pairs, stream) : launch_pair<false>(mw, mw2, mx, p, pairs, stream);
     }
     if (persistent) {
         const int ctas = pl.tiles < sm_count ? pl.tiles : sm_count;
@@ -1164,8 +1191,7 @@ extern "C" int cw_gemm_tc_parts_plan(int T, int N, int K, int sm_count, int* spl
 }
 
 // parts[ks][t][n] = the part of X W^T that split ks of K contributes (float32, [splits][part_rows][N],
-// part_rows >= T a multiple of 16; rows from T on are written too, with what the tile's last store
-// holds).  `splits` as cw_gemm_tc_parts_plan gave it.
+// part_rows >= T a multiple of 16; rows from T on are not written).  `splits` as cw_gemm_tc_parts_plan gave it.
 extern "C" int cw_gemm_tc_parts(const void* X, const void* W, float* parts, int T, int N, int K, int ldx, int part_rows,
                                 int splits, int sm_count, int* status, cudaStream_t stream) {
     if (T == 0 || N == 0) return CW_OK;
@@ -1179,10 +1205,9 @@ extern "C" int cw_gemm_tc_parts(const void* X, const void* W, float* parts, int 
     if (splits != want || splits < 1) return CW_ERR_BAD_SIZE;
     if (g_forced_bn != 0) bn = g_forced_bn;
     const int num_kb = (K + BK - 1) / BK;
-    CUtensorMap mw, mx, mc;
+    CUtensorMap mw, mx;
     if (make_map(&mw, W, N, K, K, BM) != 0) return CW_ERR_UNSUPPORTED;
     if (make_map(&mx, X, T, K, ldx, bn / 2) != 0) return CW_ERR_UNSUPPORTED;
-    if (make_map_c(&mc, parts, splits * part_rows, N, N, P_CHUNK, true) != 0) return CW_ERR_UNSUPPORTED;
     GemmParams p = {};
     p.tma_store = 1;
     p.T = T; p.N = N; p.K = K; p.ldc = N; p.epilogue = 3; p.part_rows = part_rows;
@@ -1192,7 +1217,7 @@ extern "C" int cw_gemm_tc_parts(const void* X, const void* W, float* parts, int 
     const int tiles = ((N + 2 * BM - 1) / (2 * BM)) * ((T + bn - 1) / bn);
     const int units = tiles * splits;
     const int pairs = units < sm_count / 2 ? units : sm_count / 2;
-    return launch_pair<false>(mw, mw, mx, mc, p, pairs, stream);
+    return launch_pair<false>(mw, mw, mx, p, pairs, stream);
 }
 
 CW_TRACE_TU(gemm_tc)
