@@ -32,8 +32,8 @@
 // Every wait on an mbarrier is bounded: when it runs out the kernel records CW_ST_WAIT_TIMEOUT in
 // the status words, the producer waits (bounded again) for the copies it has in flight, TMEM is
 // freed and the kernel returns.
+#include "cluster_places.cuh"
 #include "tc_common.cuh"
-#include <atomic>
 #include <type_traits>
 
 #define BM 128
@@ -918,37 +918,6 @@ extern "C" int cw_gemm_tc_set_persistent_from(int tokens) {
     if (tokens < 129) return CW_ERR_BAD_SIZE;
     g_persistent_from = tokens;
     return CW_OK;
-}
-
-// How many clusters of `size` CTAs of gemm_tc_kernel the GPU holds at a time, with one CTA or two to an SM.  A cluster lies
-// within one group of SMs (GPC), so that the counts are well below SMs / size and differ from part to part: the driver is asked
-// once per size (148 SMs, one CTA to an SM: 74, 45, 33, 26, 22, 15 and 15 clusters of 2 to 8; two: 148, 93, 71, 56, 45, 37 and 33).
-// It is asked about an empty kernel with the same threads and shared memory: of kernels that allocate tensor memory the
-// occupancy calculator says one CTA to an SM whatever they hold.
-__global__ void __launch_bounds__(THREADS) cluster_places_kernel() {}
-static int clusters_at_once(int size, int per_sm, int sm_count) {
-    static std::atomic<int> known[2][MAX_SPLITS + 1];
-    if (size <= 1) return per_sm * sm_count;
-    int n = known[per_sm - 1][size].load(std::memory_order_relaxed);
-    if (n > 0) return n;
-    const int smem = per_sm == 2 ? Cfg<64, false, 2>::SMEM_BYTES : MAX_SMEM_BYTES;
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = cluster.val.clusterDim.y = 1;
-    cluster.val.clusterDim.z = size;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1, 1, size);
-    cfg.blockDim = dim3(THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.attrs = &cluster;
-    cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(cluster_places_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM_BYTES) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, cluster_places_kernel, &cfg) != cudaSuccess || n <= 0) {
-        (void)cudaGetLastError();
-        return per_sm * sm_count / size;  // (no answer: as if clusters could lie anywhere)
-    }
-    known[per_sm - 1][size].store(n, std::memory_order_relaxed);
-    return n;
 }
 
 static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_tma = true, bool adds = false) {

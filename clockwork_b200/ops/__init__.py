@@ -347,7 +347,8 @@ EPILOGUE_RELU2 = 4  # store max(v, 0)^2 of v = product + bias, in the operands' 
 
 def gemm_ref(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, *,
              out: torch.Tensor | None = None, epilogue: int = EPILOGUE_STORE) -> torch.Tensor:
-    """``a [M,K] @ w[N,K]^T (+ bias)`` on the CUDA cores with float32 accumulation.
+    """``a [M,K] @ w[N,K]^T (+ bias)``: float32 operands as exactly as chains of float32 multiply-adds give it (``gemm_f32.cu``),
+    bfloat16 ones on the CUDA cores with float32 accumulation.
     ``a`` may be a column slice of a wider matrix (row stride > K).  Epilogues: store in
     ``a``'s dtype; add into the float32 ``out``; store float32; ``EPILOGUE_RELU2``."""
     if not a.is_cuda or a.dim() != 2 or a.stride(1) != 1:
@@ -371,7 +372,7 @@ def gemm_ref(a: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None,
         raise ValueError(f"out has shape {tuple(out.shape)}, expected {(m, n)}")
     lda = a.stride(0) if m > 1 else max(a.stride(0), k)
     check(library().cw_gemm_ref(_ptr(a), _ptr(w), _ptr(bias), _ptr(out), m, n, k, lda, n, epilogue,
-                                dtype_code(a.dtype), _stream()), "gemm_ref")
+                                dtype_code(a.dtype), _ptr(device_status(a.device)), _stream()), "gemm_ref")
     return out
 
 
@@ -385,7 +386,7 @@ def gemm_ref_swiglu(a: torch.Tensor, w_gate: torch.Tensor, w_up: torch.Tensor) -
         raise ValueError("gate and up weights must both be [N, K] with a's K")
     out = torch.empty((m, n), dtype=a.dtype, device=a.device)
     check(library().cw_gemm_ref_swiglu(_ptr(a), _ptr(w_gate), _ptr(w_up), _ptr(out), m, n, k,
-                                       dtype_code(a.dtype), _stream()), "gemm_ref_swiglu")
+                                       dtype_code(a.dtype), _ptr(device_status(a.device)), _stream()), "gemm_ref_swiglu")
     return out
 
 

@@ -1,6 +1,6 @@
 """Matrix products of the product path, chosen by run precision.
 
-float32: ``cw_gemm_ref`` (CUDA cores, fmaf, float32 throughout).
+float32: ``cw_gemm_ref`` (every operand as three bfloat16 numbers on the tensor cores, compensated float32 sums).
 bfloat16: the tcgen05 tensor-core kernel when it takes the sizes (``cw_gemm_tc``), else the
 plain kernel on bfloat16 operands."""
 

@@ -18,8 +18,8 @@ _SIGNATURES: dict[str, list] = {
     "cw_silu_mul": [P, P, I, I, I, P],
     "cw_add_to_residual": [P, P, I, I, I, P],
     "cw_add_parts_rmsnorm": [P, P, I, I, P, P, I, I, F, I, I, P, P, P],
-    "cw_gemm_ref": [P, P, P, P, I, I, I, I, I, I, I, P],
-    "cw_gemm_ref_swiglu": [P, P, P, P, I, I, I, I, P],
+    "cw_gemm_ref": [P, P, P, P, I, I, I, I, I, I, I, P, P],
+    "cw_gemm_ref_swiglu": [P, P, P, P, I, I, I, I, P, P],
     "cw_rope_store": [P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, P],
     "cw_copy_pages": [P, P, I, I, I, LL, P, P],
     "cw_attention_ref": [P, I, P, P, P, P, P, P, I, I, I, I, I, I, I, F, I, P, I, I, I, I, P, P],

@@ -18,7 +18,7 @@ import torch
 
 from .library import check, library
 
-_TUS = ("attention_decode", "attention_decode_large", "attention_decode_mid", "attention_prefill", "attention_prefill_tc", "attention_ref", "embed_norm", "gemm_ref",
+_TUS = ("attention_decode", "attention_decode_large", "attention_decode_mid", "attention_prefill", "attention_prefill_tc", "attention_ref", "embed_norm", "gemm_f32", "gemm_ref",
         "gemm_tc", "grouped_gemm", "grouped_gemm_tc", "latent_attention", "latent_attention_tc", "recurrence", "recurrence_chunks", "recurrence_gated", "rope_cache", "sampling", "window_attention", "window_attention_tc")
 _WORDS = 8
 _buf: torch.Tensor | None = None

@@ -143,6 +143,28 @@ def test_gemm_ref_float32_cut_inner_dimension(ops, n, k):
     torch.testing.assert_close(both.cpu(), want, rtol=4e-6, atol=1e-6)  # (two exponentials and a division apart)
 
 
+@pytest.mark.parametrize("m", [1, 16, 17, 32, 33, 64, 65, 200])
+@pytest.mark.parametrize("n,k", [(31, 4), (33, 60), (127, 64), (129, 68), (260, 1792), (64, 1796)])
+def test_gemm_ref_float32_operands_in_three_parts(ops, m, n, k):
+    """Edges of the float32 tiles, operands whose sizes spread over many powers of two and beyond what a rounded first part
+    holds: the sums within the bound of the chains (see above), aligned or not; a number that is not finite stays in
+    its row."""
+    a, w = rand(m, k) * torch.exp(3 * rand(m, k, seed=5)), rand(n, k, scale=0.1, seed=1)
+    a[0, 0], w[0, 0] = 3.4028e38, 2.0**-120
+    ad, wd = a.to(DEV), w.to(DEV)
+    got = ops.gemm_ref(ad, wd).cpu()
+    want, bound = a.double() @ w.double().T, 19 * 2.0**-24 * (a.double().abs() @ w.double().abs().T)
+    # (the first row's sums may leave float32, but not become anything that is no number unless the others' magnitudes do too)
+    fits = bound < 3e38 * 19 * 2.0**-24
+    assert ((got.double() - want).abs() <= bound)[fits].all() and fits[1:].all() and fits[0, 0]
+    odd = torch.zeros(m + 1, k + 1, device=DEV)[:m, :k].copy_(ad)
+    assert torch.equal(ops.gemm_ref(odd, wd).cpu()[1:], got[1:])
+    if m > 1:
+        ad[1, k - 1] = float("inf")
+        spoilt = ops.gemm_ref(ad, wd).cpu()
+        assert not torch.isfinite(spoilt[1]).any() and torch.equal(spoilt[2:], got[2:]) and torch.equal(spoilt[0, 0], got[0, 0])
+
+
 def test_gemm_ref_is_true_float32(ops):
     """Operands that need 13 mantissa bits, chosen so that every product and every partial sum is
     exact in float32 (22 bits at most) whatever the order of summation: the result must equal the
