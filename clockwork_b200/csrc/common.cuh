@@ -240,6 +240,15 @@ __device__ __forceinline__ void pdl_launch_dependents() {
     cw_trace(0);
 }
 
+// For kernels with nothing to do before their predecessor has finished: waits for it, then lets the successor's blocks come, whose
+// launch so costs no time of its own.  In this order, so that no more than one kernel's blocks ever sit on the SMs waiting.
+// Measured against launches in plain stream order (B200): 8 single tokens of a layer with experts 224.4 -> 219.4 us, a retention
+// layer's 2 88.5 -> 85.6, prompts within 1 %; the windowed attention of prompts, two CTAs to an SM, was 1 % slower so and stays ordered.
+__device__ __forceinline__ void pdl_enter() {
+    pdl_wait();
+    pdl_launch_dependents();
+}
+
 // 1: launch with the attribute (default); 0: plain launches.  Set through cw_set_pdl().
 extern "C" int cw_pdl_enabled();
 

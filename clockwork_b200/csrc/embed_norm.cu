@@ -431,7 +431,7 @@ extern "C" int cw_sum_rmsnorm_add(float* resid, const float* a, const float* b, 
 // ---- logits scaled and bent towards a bound ---------------------------------------------------------------
 // x <- cap tanh(scale x / cap), in place, float32 (cap 0: x <- scale x).
 __global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ x, long long n, float cap, float scale) {
-    pdl_wait();
+    pdl_enter();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float z = x[i] * scale;  // (scale 1: the logit as it is)
         x[i] = cap > 0.f ? cap * tanhf(z / cap) : z;
@@ -442,7 +442,7 @@ extern "C" int cw_softcap(float* x, long long n, float cap, float scale, cudaStr
     if (n == 0) return CW_OK;
     if (n < 0 || !(cap >= 0.f)) return CW_ERR_BAD_SIZE;
     const int blocks = (int)min((long long)148 * 8, (n + 255) / 256);
-    return cw_launch_ordered(softcap_kernel, dim3(blocks), dim3(256), 0, stream, x, n, cap, scale);
+    return cw_launch(softcap_kernel, dim3(blocks), dim3(256), 0, stream, 1, x, n, cap, scale);
 }
 
 // ---- a second table read by a hash of (previous token, token) -------------------------------------------

@@ -395,7 +395,7 @@ moe_choose_kernel(const float* __restrict__ logits, const float* __restrict__ b,
                   int* __restrict__ sel, float* __restrict__ wt, int N, int E, int top, int mode, int groups, int keep,
                   const float* __restrict__ correction, float weight_scale, int group_rank, int renormalize) {
     extern __shared__ float choose_s[];  // per warp: [E] logits or scores, [top] chosen ones, [groups] the runs' best, [E] plain scores
-    pdl_wait();
+    pdl_enter();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int row = blockIdx.x * 4 + warp;
     if (row >= N) return;
@@ -521,7 +521,7 @@ extern "C" int cw_moe_choose(const float* logits, const float* b, const int* tok
     if (group_rank < 1 || group_rank > 4 || group_rank > E / groups) return CW_ERR_BAD_SIZE;
     const size_t smem = 4 * (size_t)(2 * E + top + groups) * sizeof(float);
     if (smem > (48 << 10)) return CW_ERR_UNSUPPORTED;
-    return cw_launch_ordered(moe_choose_kernel, dim3((N + 3) / 4), dim3(128), smem, stream, logits, b, tok_seq, sel, wt, N, E, top,
+    return cw_launch(moe_choose_kernel, dim3((N + 3) / 4), dim3(128), smem, stream, 1, logits, b, tok_seq, sel, wt, N, E, top,
                              mode, groups, keep, correction, weight_scale, group_rank, renormalize);
 }
 
@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(1024)
 moe_group_kernel(const int* __restrict__ sel, int* __restrict__ offsets, int* __restrict__ order, int* __restrict__ rank,
                  int P, int E) {
     extern __shared__ int count_s[];  // [E + 1]
-    pdl_wait();
+    pdl_enter();
     for (int e = threadIdx.x; e <= E; e += blockDim.x) count_s[e] = 0;
     __syncthreads();
     for (int p = threadIdx.x; p < P; p += blockDim.x) {
@@ -560,7 +560,7 @@ moe_group_kernel(const int* __restrict__ sel, int* __restrict__ offsets, int* __
 
 extern "C" int cw_moe_group(const int* sel, int* offsets, int* order, int* rank, int P, int E, cudaStream_t stream) {
     if (P < 0 || E <= 0 || E > 8191) return CW_ERR_BAD_SIZE;
-    return cw_launch_ordered(moe_group_kernel, dim3(1), dim3(1024), (size_t)(E + 1) * sizeof(int), stream, sel, offsets, order, rank, P, E);
+    return cw_launch(moe_group_kernel, dim3(1), dim3(1024), (size_t)(E + 1) * sizeof(int), stream, 1, sel, offsets, order, rank, P, E);
 }
 
 // resid[n] += sum_t wt[n, t] * y[n * top + t] over the choices in order; with `assign` the sum replaces resid[n] (rows of no
@@ -569,7 +569,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 moe_combine_kernel(float* __restrict__ resid, const float* __restrict__ y, const int* __restrict__ sel,
                    const float* __restrict__ wt, const T* __restrict__ x, int experts, int W, int top, int assign) {
-    pdl_wait();
+    pdl_enter();
     const int row = blockIdx.x;
     if (sel[(size_t)row * top] < 0) {
         if (assign)
@@ -592,7 +592,7 @@ template <typename T>
 __global__ void __launch_bounds__(128)
 moe_combine_vec_kernel(float* __restrict__ resid, const float* __restrict__ y, const int* __restrict__ sel,
                        const float* __restrict__ wt, const T* __restrict__ x, int experts, int W, int top, int assign) {
-    pdl_wait();
+    pdl_enter();
     const int row = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * 4;
     if (c >= W) return;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -631,8 +631,8 @@ template <typename T>
 static int launch_moe_combine(float* resid, const float* y, const int* sel, const float* wt, const T* x, int experts, int N, int W, int top,
                               int assign, cudaStream_t stream) {
     if (W % 4 == 0 && (((uintptr_t)resid | (uintptr_t)y | (uintptr_t)x) & 15) == 0)
-        return cw_launch_ordered(moe_combine_vec_kernel<T>, dim3(N, (W + 511) / 512), dim3(128), 0, stream, resid, y, sel, wt, x, experts, W, top, assign);
-    return cw_launch_ordered(moe_combine_kernel<T>, dim3(N), dim3(256), 0, stream, resid, y, sel, wt, x, experts, W, top, assign);
+        return cw_launch(moe_combine_vec_kernel<T>, dim3(N, (W + 511) / 512), dim3(128), 0, stream, 1, resid, y, sel, wt, x, experts, W, top, assign);
+    return cw_launch(moe_combine_kernel<T>, dim3(N), dim3(256), 0, stream, 1, resid, y, sel, wt, x, experts, W, top, assign);
 }
 
 // x null: every choice has its y.  dtype: of x.

@@ -105,6 +105,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
+    pdl_enter();
     if (warp == 0) {
         int run = 0;
         for (int g0 = 0; g0 < p.G; g0 += 32) {
@@ -303,6 +304,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 // out[r] = a[index[r] / div] for the offsets[G] rows that belong to a group; a block per row, 16 bytes a thread.
 __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ a, uint4* __restrict__ out, const int* __restrict__ index,
                                                           const int* __restrict__ rows, int div, int pieces) {
+    pdl_enter();
     if ((int)blockIdx.x >= *rows) return;
     const uint4* from = a + (size_t)(index[blockIdx.x] / div) * pieces;
     for (int c = threadIdx.x; c < pieces; c += 256) out[(size_t)blockIdx.x * pieces + c] = from[c];
@@ -315,7 +317,7 @@ extern "C" int cw_gather_rows(const void* a, void* out, const int* index, const 
     if (M == 0) return CW_OK;
     if (M < 0 || div <= 0 || row_bytes <= 0) return CW_ERR_BAD_SIZE;
     if (row_bytes % 16 || row_bytes / 16 > 0x7fffffffLL || ((uintptr_t)a | (uintptr_t)out) % 16) return CW_ERR_UNSUPPORTED;
-    return cw_launch_ordered(gather_rows_kernel, dim3(M), dim3(256), 0, stream, (const uint4*)a, (uint4*)out, index, rows, div, (int)(row_bytes / 16));
+    return cw_launch(gather_rows_kernel, dim3(M), dim3(256), 0, stream, 1, (const uint4*)a, (uint4*)out, index, rows, div, (int)(row_bytes / 16));
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------
@@ -352,7 +354,7 @@ static int gt_launch(const GroupedArgs& p, const CUtensorMap& w, const CUtensorM
     const int smem = C::smem(p.G);
     const cudaError_t e = cudaFuncSetAttribute(grouped_gemm_tc_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::smem(GT_MAX_GROUPS));
     if (e != cudaSuccess) return (int)e;
-    return cw_launch_ordered(grouped_gemm_tc_kernel<BN, EPI>, dim3(grid), dim3(GT_THREADS), (size_t)smem, stream, w, w2, x, p);
+    return cw_launch(grouped_gemm_tc_kernel<BN, EPI>, dim3(grid), dim3(GT_THREADS), (size_t)smem, stream, 1, w, w2, x, p);
 }
 
 int grouped_tc_run(const GroupedArgs& p, int epilogue, cudaStream_t stream) {

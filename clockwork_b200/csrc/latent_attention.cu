@@ -31,7 +31,7 @@ latent_prepare_kernel(const float* __restrict__ down, int ldd, const QT* __restr
                       float eps, int write_cache, int vec, int* status) {
     extern __shared__ float lp_table[];  // cosines, then sines, of the token's pairs
     __shared__ float scratch[33];
-    pdl_wait();
+    pdl_enter();
     const int row = blockIdx.x, tid = threadIdx.x;
     const int D = rank + rot.dims, half = rot.dims >> 1;
     float *cs = lp_table, *sn = lp_table + half;
@@ -98,12 +98,12 @@ extern "C" int cw_latent_prepare(const float* down, int ldd, const void* q, int 
     const dim3 grid(N), block(H * (dim + rot_dims) > 1024 ? 256 : 128);
     const size_t smem = sizeof(float) * (size_t)rot_dims;
     if (dtype == 0)
-        return cw_launch_ordered(latent_prepare_kernel<float, float>, grid, block, smem, stream, down, ldd, (const float*)q, ldq, (float*)q_plain,
+        return cw_launch(latent_prepare_kernel<float, float>, grid, block, smem, stream, 1, down, ldd, (const float*)q, ldq, (float*)q_plain,
                                  (float*)qa, (float*)cache, norm_w, rot, positions, slots, H, dim, rank, num_slots, eps, write_cache, vec, status);
     if (wide_q)
-        return cw_launch_ordered(latent_prepare_kernel<bf16, float>, grid, block, smem, stream, down, ldd, (const float*)q, ldq, (bf16*)q_plain,
+        return cw_launch(latent_prepare_kernel<bf16, float>, grid, block, smem, stream, 1, down, ldd, (const float*)q, ldq, (bf16*)q_plain,
                                  (bf16*)qa, (bf16*)cache, norm_w, rot, positions, slots, H, dim, rank, num_slots, eps, write_cache, vec, status);
-    return cw_launch_ordered(latent_prepare_kernel<bf16, bf16>, grid, block, smem, stream, down, ldd, (const bf16*)q, ldq, (bf16*)q_plain,
+    return cw_launch(latent_prepare_kernel<bf16, bf16>, grid, block, smem, stream, 1, down, ldd, (const bf16*)q, ldq, (bf16*)q_plain,
                              (bf16*)qa, (bf16*)cache, norm_w, rot, positions, slots, H, dim, rank, num_slots, eps, write_cache, vec, status);
 }
 
@@ -316,7 +316,7 @@ latent_attention_mma_kernel(const LatentArgs a) {
     float* alpha_s = row_sum + KW * ROWS;                 // [ROWS] what the sums so far are multiplied by when the maximum moves
     float* inv_s = alpha_s + ROWS;                        // [ROWS] what they are multiplied by at the end
     int* slot_s = (int*)(inv_s + ROWS);                   // [2][KT]
-    pdl_wait();
+    pdl_enter();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, part = blockIdx.y;
     const long long total_rows = (long long)a.N * H;
     if (part == 0) {  // rows of no request (padding of a fixed-shape step) come out as zeros
@@ -586,7 +586,7 @@ __global__ void __launch_bounds__(256)
 latent_merge_kernel(const float* __restrict__ partial, const int* __restrict__ tok_seq, const float* __restrict__ sink,
                     bf16* __restrict__ out, int H, int rank, int parts, long long total_rows) {
     __shared__ float factor[LT_MAX_PARTS];
-    pdl_wait();
+    pdl_enter();
     const long long row = blockIdx.x;
     if (tok_seq[row / H] < 0) return;  // (the attention kernel wrote the zeros)
     const float* stats = partial + (size_t)parts * total_rows * rank;
@@ -648,11 +648,11 @@ static int launch_latent_mma(const LatentArgs& a, cudaStream_t stream) {
     }
     const long long rows = (long long)a.N * a.H;
     const dim3 grid((unsigned)((rows + L::ROWS - 1) / L::ROWS + a.S), a.parts);
-    const int rc = cw_launch_ordered(latent_attention_mma_kernel<MT>, grid, dim3(256), bytes, stream, a);
+    const int rc = cw_launch(latent_attention_mma_kernel<MT>, grid, dim3(256), bytes, stream, 1, a);
     if (rc != 0 || a.parts == 1) return rc;
     int threads = 32;
     while (threads < 256 && threads * 2 < a.rank) threads *= 2;
-    return cw_launch_ordered(latent_merge_kernel, dim3((unsigned)rows), dim3(threads), 0, stream, (const float*)a.partial, a.tok_seq, a.sink,
+    return cw_launch(latent_merge_kernel, dim3((unsigned)rows), dim3(threads), 0, stream, 1, (const float*)a.partial, a.tok_seq, a.sink,
                              a.out, a.H, a.rank, a.parts, rows);
 }
 

@@ -69,6 +69,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const int split = blockIdx.x % p.splits, block = blockIdx.x / p.splits;
     const long long total_rows = (long long)a.N * H;
 
+    pdl_enter();
     if (split == 0) {  // rows of no request (padding of a fixed-shape step) come out as zeros
         const long long first = (long long)block * LC_ROWS, last = min(total_rows, first + LC_ROWS);
         for (long long t = first / H; t * H < last; ++t)
@@ -381,7 +382,7 @@ int latent_tc_run(const LatentArgs& a, cudaStream_t stream) {
     const size_t smem = (size_t)(p.blocks - p.held) * LC_Q_BLOCK + (size_t)p.blocks * p.stages * LC_K_BLOCK + 2048;
     const cudaError_t e = cudaFuncSetAttribute(latent_attention_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LC_SMEM);
     if (e != cudaSuccess) return (int)e;
-    return cw_launch_ordered(latent_attention_tc_kernel, dim3((unsigned)blocks), dim3(LC_THREADS), smem, stream, q, c, p);
+    return cw_launch(latent_attention_tc_kernel, dim3((unsigned)blocks), dim3(LC_THREADS), smem, stream, 1, q, c, p);
 }
 
 CW_TRACE_TU(latent_attention_tc)

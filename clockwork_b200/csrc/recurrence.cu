@@ -98,7 +98,7 @@ causal_conv4_kernel(const float* __restrict__ x, int ldx, const float* __restric
                     const float* __restrict__ state, long long state_stride, long long state_off,
                     const long long* __restrict__ slots, const int* __restrict__ tok_seq, const int* __restrict__ q_start,
                     float* __restrict__ out, int C) {
-    pdl_wait();
+    pdl_enter();
     const int row = blockIdx.y, c = (blockIdx.x * blockDim.x + threadIdx.x) * 4;
     if (c >= C) return;
     float4* to = (float4*)(out + (size_t)row * C + c);
@@ -132,7 +132,7 @@ extern "C" int cw_causal_conv(const float* x, int ldx, const float* weight, cons
     if (N < 0 || C <= 0 || taps <= 0 || ldx < C) return CW_ERR_BAD_SIZE;
     if (taps == 4 && C % 4 == 0 && ldx % 4 == 0 && state_stride % 4 == 0 && state_off % 4 == 0 && N <= 65535 &&
         (((uintptr_t)x | (uintptr_t)weight | (uintptr_t)bias | (uintptr_t)state | (uintptr_t)out) & 15) == 0)
-        return cw_launch_ordered(causal_conv4_kernel, dim3((C / 4 + 255) / 256, N), dim3(256), 0, stream, x, ldx, weight, bias, state,
+        return cw_launch(causal_conv4_kernel, dim3((C / 4 + 255) / 256, N), dim3(256), 0, stream, 1, x, ldx, weight, bias, state,
                                  state_stride, state_off, slots, tok_seq, q_start, out, C);
     return cw_launch_ordered(causal_conv_kernel, dim3(N), dim3(256), 0, stream, x, ldx, weight, bias, state, state_stride, state_off,
                      slots, tok_seq, q_start, out, C, taps);
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256)
 carry_rows_kernel(const T* __restrict__ x, int ldx, float* __restrict__ state, long long state_stride,
                   long long state_off, const long long* __restrict__ slots, const int* __restrict__ tok_seq,
                   const int* __restrict__ q_start, int C, int R) {
-    pdl_wait();
+    pdl_enter();
     const int seq = blockIdx.x;
     const int start = q_start[seq], end = q_start[seq + 1];
     const int n = end - start;
@@ -165,10 +165,10 @@ extern "C" int cw_carry_rows(const void* x, int ldx, float* state, long long sta
     if (S < 0 || C <= 0 || R < 0 || ldx < C) return CW_ERR_BAD_SIZE;
     dim3 grid(S, min(64, (C + 255) / 256));
     if (dtype == 0)
-        return cw_launch_ordered(carry_rows_kernel<float>, grid, dim3(256), 0, stream, (const float*)x, ldx, state, state_stride,
+        return cw_launch(carry_rows_kernel<float>, grid, dim3(256), 0, stream, 1, (const float*)x, ldx, state, state_stride,
                          state_off, slots, tok_seq, q_start, C, R);
     if (dtype == 1)
-        return cw_launch_ordered(carry_rows_kernel<bf16>, grid, dim3(256), 0, stream, (const bf16*)x, ldx, state, state_stride,
+        return cw_launch(carry_rows_kernel<bf16>, grid, dim3(256), 0, stream, 1, (const bf16*)x, ldx, state, state_stride,
                          state_off, slots, tok_seq, q_start, C, R);
     return CW_ERR_BAD_DTYPE;
 }
@@ -196,7 +196,7 @@ extern "C" int cw_carry_rows(const void* x, int ldx, float* state, long long sta
 __global__ void __launch_bounds__(256)
 recurrence_coefficients_kernel(int form, float* __restrict__ pre, int ldp, const float* __restrict__ p0,
                                const float* __restrict__ p1, float* __restrict__ out, int N, int C) {
-    pdl_wait();
+    pdl_enter();
     const long long total = (long long)N * C;
     for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (long long)gridDim.x * blockDim.x) {
         const int t = (int)(idx / C), c = (int)(idx - (long long)t * C);
@@ -218,7 +218,7 @@ extern "C" int cw_recurrence_coefficients(int form, float* pre, int ldp, const f
     if (N < 0 || C <= 0 || ldp < C || (form != 0 && form != 1)) return CW_ERR_BAD_SIZE;
     const long long total = (long long)N * C;
     const int blocks = (int)min((long long)148 * 8, (total + 255) / 256);
-    return cw_launch_ordered(recurrence_coefficients_kernel, dim3(blocks), dim3(256), 0, stream, form, pre, ldp, p0, p1, out, N, C);
+    return cw_launch(recurrence_coefficients_kernel, dim3(blocks), dim3(256), 0, stream, 1, form, pre, ldp, p0, p1, out, N, C);
 }
 
 #define RS 8    // key channels per thread
@@ -251,7 +251,7 @@ recurrence_scan_kernel(const float* __restrict__ q, int ldq, const float* __rest
     extern __shared__ __align__(16) float rs_smem[];
     __shared__ __align__(16) float nothing[4];  // zeros: what lanes without channels read
     if (threadIdx.x < 4) nothing[threadIdx.x] = 0.f;
-    pdl_wait();
+    pdl_enter();
     constexpr bool VEC = IPT > 0;
     const int IP = VEC ? IPT : ip;
     // (the request is the slowest index: the blocks of a request that brings tokens then start side by side on as many SMs,
@@ -477,7 +477,7 @@ extern "C" int cw_recurrence_scan(int form, const float* q, int ldq, const float
         if (e != cudaSuccess) return (int)e;
         allowed[form][which] = smem;
     }
-    return cw_launch_ordered(kernels[form][which], grid, dim3(threads), smem, stream, q, ldq, k, ldk, v, ldv, pre, ldp, p0, p1, p2, state,
+    return cw_launch(kernels[form][which], grid, dim3(threads), smem, stream, 1, q, ldq, k, ldk, v, ldv, pre, ldp, p0, p1, p2, state,
                      state_stride, state_off, slots, tok_seq, q_start, Dk, Dv, heads_per_group, IP, wide, H, out, ldo, q_scale, below);
 }
 
@@ -544,7 +544,7 @@ __global__ void __launch_bounds__(256)
 gated_group_norm_kernel(const float* __restrict__ y, const float* __restrict__ z, int ldz, const float* __restrict__ weight,
                         T* __restrict__ out, int C, int parts, float eps, int mode) {
     __shared__ float scratch[33];
-    pdl_wait();
+    pdl_enter();
     const bool ungated = mode & 8;
     const int gate_first = ungated ? 0 : (mode & 1);
     const bool plain_sigmoid = mode & 2;
@@ -580,7 +580,7 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(256)
 gated_group_norm_warp_kernel(const float* __restrict__ y, const float* __restrict__ z, int ldz, const float* __restrict__ weight,
                              T* __restrict__ out, int N, int C, int parts, float eps, int mode) {
-    pdl_wait();
+    pdl_enter();
     const bool ungated = mode & 8, gate_first = !ungated && (mode & 1), plain_sigmoid = mode & 2;
     const int lane = threadIdx.x & 31;
     const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -636,11 +636,11 @@ static int launch_gated_group_norm(const float* y, const float* z, int ldz, cons
                             : width <= 256 ? gated_group_norm_warp_kernel<T, 2>
                             : width <= 512 ? gated_group_norm_warp_kernel<T, 4>
                                            : gated_group_norm_warp_kernel<T, 8>;
-        return cw_launch_ordered(kernel, grid, dim3(256), 0, stream, y, z, ldz, weight, out, N, C, parts, eps, mode);
+        return cw_launch(kernel, grid, dim3(256), 0, stream, 1, y, z, ldz, weight, out, N, C, parts, eps, mode);
     }
     int threads = 32;
     while (threads < 256 && threads * 4 < width) threads *= 2;
-    return cw_launch_ordered(gated_group_norm_kernel<T>, dim3(N, parts), dim3(threads), 0, stream, y, z, ldz, weight, out, C, parts, eps, mode);
+    return cw_launch(gated_group_norm_kernel<T>, dim3(N, parts), dim3(threads), 0, stream, 1, y, z, ldz, weight, out, C, parts, eps, mode);
 }
 
 extern "C" int cw_gated_group_norm(const float* y, const float* z, int ldz, const float* weight, void* out, int N, int C,
@@ -659,7 +659,7 @@ extern "C" int cw_gated_group_norm(const float* y, const float* z, int ldz, cons
 __global__ void __launch_bounds__(256)
 rotate_heads_kernel(float* __restrict__ x, int ld, const int* __restrict__ positions, Rotation rot, int heads, int dk) {
     extern __shared__ float rh_table[];
-    pdl_wait();
+    pdl_enter();
     const int n = blockIdx.x, half = rot.dims >> 1;
     float* cs = rh_table;
     float* sn = rh_table + half;
@@ -684,7 +684,7 @@ extern "C" int cw_rotate_heads(float* x, int ld, const int* positions, const flo
     if (rot_dims > 8192) return CW_ERR_UNSUPPORTED;
     int threads = 64;
     while (threads < 256 && threads < heads * (rot_dims >> 1)) threads *= 2;
-    return cw_launch_ordered(rotate_heads_kernel, dim3(N), dim3(threads), sizeof(float) * (size_t)rot_dims, stream, x, ld, positions, rot,
+    return cw_launch(rotate_heads_kernel, dim3(N), dim3(threads), sizeof(float) * (size_t)rot_dims, stream, 1, x, ld, positions, rot,
                              heads, dk);
 }
 
@@ -698,7 +698,7 @@ __device__ __forceinline__ float activation_of(int kind, float z) {
 
 template <typename T>
 __global__ void __launch_bounds__(256) activation_kernel(T* __restrict__ x, long long n, int kind) {
-    pdl_wait();
+    pdl_enter();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         x[i] = from_f<T>(activation_of(kind, to_f(x[i])));
 }
@@ -729,8 +729,8 @@ extern "C" int cw_activation(void* x, long long n, int kind, int dtype, cudaStre
     if (n == 0) return CW_OK;
     if (n < 0 || kind < 0 || kind > 3) return CW_ERR_BAD_SIZE;
     const int blocks = (int)min((long long)148 * 8, (n + 255) / 256);
-    if (dtype == 0) return cw_launch_ordered(activation_kernel<float>, dim3(blocks), dim3(256), 0, stream, (float*)x, n, kind);
-    if (dtype == 1) return cw_launch_ordered(activation_kernel<bf16>, dim3(blocks), dim3(256), 0, stream, (bf16*)x, n, kind);
+    if (dtype == 0) return cw_launch(activation_kernel<float>, dim3(blocks), dim3(256), 0, stream, 1, (float*)x, n, kind);
+    if (dtype == 1) return cw_launch(activation_kernel<bf16>, dim3(blocks), dim3(256), 0, stream, 1, (bf16*)x, n, kind);
     return CW_ERR_BAD_DTYPE;
 }
 

@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(CK * CK) chunk_gram_kernel(const ChunkArgs p, 
     const int splits = (p.heads_per_group + CK_HEADS - 1) / CK_HEADS, group = blockIdx.y / splits;
     const int h0 = group * p.heads_per_group + blockIdx.y % splits * CK_HEADS, heads = min(CK_HEADS, (group + 1) * p.heads_per_group - h0);
     const int tid = threadIdx.x, Dk = p.Dk, ld = Dk + 4;
+    pdl_enter();
     if (tid < 32) {
         const RowTile tile = find_row_tile(blockIdx.x, false, p.q_start, p.tok_seq, p.S, 1, CK, p.from);
         if (tid == 0) tile_row = tile.row0, tile_rows = tile.seq < 0 ? 0 : tile.rows;
@@ -136,6 +137,7 @@ __global__ void __launch_bounds__(Dk) chunk_scan_kernel(const ChunkArgs p) {
     float* us = sums + NW * SUMS * CK * CK;  // [token][column]: what a token writes, before what the chunk's earlier ones take off
     float* ws = us + CK * CK;                // [token] W
     const int seq = blockIdx.z, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_enter();
     const int start = p.q_start[seq], end = p.q_start[seq + 1];
     if (end <= start || end - start < p.from) return;
     const int Dv = p.Dv, c = (tid & 7) * 2, grp = tid >> 3, j0 = blockIdx.x * CK, j = j0 + c;
@@ -357,7 +359,7 @@ static int launch_chunks(const ChunkArgs& p, long long rows, cudaStream_t stream
     const size_t smem = cw_scan_smem(need, rows, (long long)grid.x * grid.y);
     const cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<Dk, DELTA>, cudaFuncAttributeMaxDynamicSharedMemorySize, CK_SMEM);
     if (e != cudaSuccess) return (int)e;
-    return cw_launch_ordered(chunk_scan_kernel<Dk, DELTA>, grid, dim3(Dk), smem, stream, p);
+    return cw_launch(chunk_scan_kernel<Dk, DELTA>, grid, dim3(Dk), smem, stream, 1, p);
 }
 
 // rows: the rows of the step.  from: requests of fewer tokens are left alone.  delta: the second form above (no skip, q_scale 1, no column of ones).  Heads of 32, 64 or 128
@@ -377,7 +379,7 @@ extern "C" int cw_chunk_scan(int delta, const float* q, int ldq, const float* k,
     const ChunkArgs p = {q, k, v, ldq, ldk, ldv, a, b, lda, ldb, skip, q_scale, ones, state, state_stride, state_off, slots, tok_seq, q_start,
                          S, H, Dk, Dv, heads_per_group, from, out, gram, R > 0 ? carry : nullptr, ldc, C, R, carry_off};
     const int chunks = (rows + CK - 1) / CK + (rows < S ? rows : S);
-    const int err = cw_launch_ordered(chunk_gram_kernel, dim3(chunks, H / heads_per_group * ((heads_per_group + CK_HEADS - 1) / CK_HEADS)), dim3(CK * CK), sizeof(float) * 2 * CK * (Dk + 4), stream, p, delta);
+    const int err = cw_launch(chunk_gram_kernel, dim3(chunks, H / heads_per_group * ((heads_per_group + CK_HEADS - 1) / CK_HEADS)), dim3(CK * CK), sizeof(float) * 2 * CK * (Dk + 4), stream, 1, p, delta);
     if (err != CW_OK) return err;
 #define CK_GO(D) return delta ? launch_chunks<D, true>(p, rows, stream) : launch_chunks<D, false>(p, rows, stream)
     switch (Dk) {

@@ -109,7 +109,7 @@ struct DeltaPrepareArgs {
 template <bool VEC>
 __global__ void __launch_bounds__(256)
 delta_prepare_kernel(const DeltaPrepareArgs a) {
-    pdl_wait();
+    pdl_enter();
     const int row = blockIdx.x, tid = threadIdx.x, share = blockIdx.y, shares = gridDim.y;
     const int Dk = a.Dk, qk = a.groups * Dk, C = 2 * qk + a.H * a.Dv, R = a.taps - 1;
     const int at = share * blockDim.x + tid, step = shares * blockDim.x;  // this thread's first channel (or four) and the stride
@@ -217,7 +217,7 @@ extern "C" int cw_delta_prepare(const float* x, int ldx, const float* weight, in
     while (shares < 32 && (long long)N * shares < 148 && shares * threads * 4 < C) shares *= 2;
     const DeltaPrepareArgs args = {x, ldx, weight, taps, state, state_stride, conv_off, slots, tok_seq, q_start, groups, Dk, H, Dv, eps,
                                    q_scale, beta, ldb, decay, lda, dt_bias, a_log, out, coef};
-    return cw_launch_ordered(vec ? delta_prepare_kernel<true> : delta_prepare_kernel<false>, dim3(N, shares), dim3(threads), 0, stream, args);
+    return cw_launch(vec ? delta_prepare_kernel<true> : delta_prepare_kernel<false>, dim3(N, shares), dim3(threads), 0, stream, 1, args);
 }
 
 // ---- the delta rule ---------------------------------------------------------------------------------------
@@ -278,7 +278,7 @@ delta_scan_kernel(const DeltaScanArgs g) {
     extern __shared__ __align__(16) float ds_smem[];
     __shared__ __align__(16) float nothing[4];  // zeros: what lanes without channels read
     if (threadIdx.x < 4) nothing[threadIdx.x] = 0.f;
-    pdl_wait();
+    pdl_enter();
     // (the request is the slowest index: the blocks of a request that brings tokens then start side by side on as many SMs,
     // however many requests of a fixed-shape step bring none)
     const int seq = blockIdx.z, h = blockIdx.y, tid = threadIdx.x;
@@ -496,7 +496,7 @@ extern "C" int cw_delta_scan(const float* q, int ldq, const float* k, int ldk, c
     }
     const DeltaScanArgs args = {q, ldq, k, ldk, v, ldv, a, lda, beta, ldb, state, state_stride, state_off, slots, tok_seq, q_start, Dk, Dv,
                                 heads_per_group, IP, wide, below, out, ldo, R > 0 ? carry : nullptr, ldc, C, R, carry_off};
-    return cw_launch_ordered(kernels[by_head][which], grid, dim3(threads), smem, stream, args);
+    return cw_launch(kernels[by_head][which], grid, dim3(threads), smem, stream, 1, args);
 }
 
 // ---- the gates of a matrix memory -----------------------------------------------------------------------

@@ -90,7 +90,7 @@ rotate_store_kernel(const float* __restrict__ src, int ld, const int* __restrict
                     int* __restrict__ status) {
     extern __shared__ float rs_table[];  // cosines, then sines, of the token's pairs
     __shared__ float scratch[33];
-    pdl_wait();
+    pdl_enter();
     const int n = blockIdx.x;
     const int at = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
     const int HQ = H * dk, row = dk + dv, half = rot.dims >> 1;
@@ -230,13 +230,13 @@ extern "C" int cw_rotate_store(const float* src, int ld, const int* positions, c
     if (dtype == 0) {
         const auto kernel = q_norm != nullptr ? (vec ? rotate_store_kernel<float, true, true> : rotate_store_kernel<float, true, false>)
                                               : (vec ? rotate_store_kernel<float, false, true> : rotate_store_kernel<float, false, false>);
-        return cw_launch_ordered(kernel, grid, block, smem, stream, src, ld, positions, tok_seq, slots, rot, q_norm, k_norm, eps, H, G, dk, dv, tied,
+        return cw_launch(kernel, grid, block, smem, stream, 1, src, ld, positions, tok_seq, slots, rot, q_norm, k_norm, eps, H, G, dk, dv, tied,
                                  (float*)q_out, (float*)cache, total_rows, status);
     }
     if (dtype == 1) {
         const auto kernel = q_norm != nullptr ? (vec ? rotate_store_kernel<bf16, true, true> : rotate_store_kernel<bf16, true, false>)
                                               : (vec ? rotate_store_kernel<bf16, false, true> : rotate_store_kernel<bf16, false, false>);
-        return cw_launch_ordered(kernel, grid, block, smem, stream, src, ld, positions, tok_seq, slots, rot, q_norm, k_norm, eps, H, G, dk, dv, tied,
+        return cw_launch(kernel, grid, block, smem, stream, 1, src, ld, positions, tok_seq, slots, rot, q_norm, k_norm, eps, H, G, dk, dv, tied,
                                  (bf16*)q_out, (bf16*)cache, total_rows, status);
     }
     return CW_ERR_BAD_DTYPE;
@@ -506,7 +506,7 @@ window_merge_kernel(const float* __restrict__ partial, const int* __restrict__ p
                     int gate_entries) {
     __shared__ float factor[64];
     __shared__ float denominator;
-    pdl_wait();
+    pdl_enter();
     const int n = blockIdx.x, h = blockIdx.y;
     if (tok_seq[n] < 0) return;  // (the attention kernel wrote the zeros)
     const int HV = H * dv, stride = HV + 2 * H;
@@ -1033,7 +1033,7 @@ extern "C" int cw_window_attention(const void* q, int ldq, const void* cache, co
         if (rc != 0) return rc;
         if (launched) {
             if (parts == 1) return CW_OK;
-            return cw_launch_ordered(window_merge_kernel<bf16>, dim3(N, H), dim3(merge_threads), 0, stream, (const float*)partial, positions, tok_seq, H,
+            return cw_launch(window_merge_kernel<bf16>, dim3(N, H), dim3(merge_threads), 0, stream, 1, (const float*)partial, positions, tok_seq, H,
                                      dv, window, parts, 0, sigmoid_weights, 1, blocked, sink, (bf16*)out, pool, keep, gate, ldg, gate_entries);
         }
         if (tc && parts <= WC_MAX_PARTS) return window_tc_run(base, q_start, S, N, stream);  // (sizes that the mma.sync form does not take)
@@ -1072,9 +1072,9 @@ extern "C" int cw_window_attention(const void* q, int ldq, const void* cache, co
                         : cw_launch_ordered(window_attention_kernel<bf16>, grid, dim3(threads), smem, stream, a);
     if (rc != 0 || parts == 1) return rc;
     if (dtype == 0)
-        return cw_launch_ordered(window_merge_kernel<float>, dim3(N, H), dim3(merge_threads), 0, stream, (const float*)partial, positions, tok_seq,
+        return cw_launch(window_merge_kernel<float>, dim3(N, H), dim3(merge_threads), 0, stream, 1, (const float*)partial, positions, tok_seq,
                                  H, dv, window, parts, part_keys, sigmoid_weights, 0, blocked, sink, (float*)out, pool, keep, gate, ldg, gate_entries);
-    return cw_launch_ordered(window_merge_kernel<bf16>, dim3(N, H), dim3(merge_threads), 0, stream, (const float*)partial, positions, tok_seq, H,
+    return cw_launch(window_merge_kernel<bf16>, dim3(N, H), dim3(merge_threads), 0, stream, 1, (const float*)partial, positions, tok_seq, H,
                              dv, window, parts, part_keys, sigmoid_weights, 0, blocked, sink, (bf16*)out, pool, keep, gate, ldg, gate_entries);
 }
 
