@@ -531,7 +531,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     const uint32_t stage_tx = C::A_BYTES * (SWIGLU ? 2 : 1) + bn * BK * 2;
     // The token tiles of a weight tile are neighbours in the walk: the CTAs at work at a time share few weight tiles, which L2
     // holds however large the matrix is.  (Weight tiles next to one another instead read weights beyond L2, as the 272 MB of gate
-    // and up at the 7B sizes, from HBM once per token tile: 640 tokens 253 us, this way 180; 2,048 tokens at the 1.5B sizes 114 and 108 us.)
+    // and up at the 7B sizes, from HBM once per token tile: 640 tokens 253 us, this way 180; 2,048 tokens at the 1.5B sizes 114 and 108 us, before the issuing threads were elected; 78 since.)
     const int tiles = m_tiles * n_tiles;
 
     if (tid == 0) {

@@ -16,8 +16,8 @@
 // tensor cores take about equally long for, and waits of one for the other (HBM at 53 % of its peak for gate and up, 60 % for down, the tensor
 // pipe at 43 and 40 %); single tokens are bound by the weights alone, and BN = 32 leaves room for more
 // weight tiles in flight.  The mma.sync kernel it replaced for these sizes stages both operands by cp.async, three steps of 32.
-// Measured (B200, 2,048 tokens, 64 experts of 1,408 of which 6, width 2,048): gate and up 672 -> 190 us, down 366 -> 102 us; 8 tokens:
-// 128 -> 70 us and 72 -> 39 us (5.6 TB/s of weights); per-head products of 2,048 tokens (16 x 128 to 512, gated 16 x 512 to 128): 36 -> 23 us and 61 -> 44 us.
+// Measured (B200, 2,048 tokens, 64 experts of 1,408 of which 6, width 2,048): gate and up 672 -> 169 us, down 366 -> 99 us; 8 tokens:
+// 128 -> 67 us and 72 -> 34 us; per-head products of 2,048 tokens (16 x 128 to 512, gated 16 x 512 to 128): 36 -> 23 us and 61 -> 44 us.
 //
 // Every wait on an mbarrier is bounded, as in gemm_tc.cu.
 #include "grouped_gemm.cuh"

@@ -12,8 +12,8 @@
 // S of the next tile is formed while the warps work on this one, before this one's sums if its keys have come, else behind.  Rows of the last tile behind the context are set to zero in
 // shared memory, whatever the cache holds there.  CTAs of a request's last rows, which see the most keys, come first.
 // What bounds it: the latency of a tile's chain of loads, scores (36 MMAs of 128 x 64 x 16 for 576 columns), weights and sums, with the two
-// stages that 147 KB hold: the tensor pipe is 28 % busy, the issue slots 15 %, L2 7 %.  With tiles of 32 keys it ran 332 us, with all of Q in shared memory as well (two stages of 32 keys) 446.
-// Measured (B200, 2,048 tokens of 16 heads over 512 + 64): the mma.sync kernel it replaced for uncut keys 494 us, this one 261 us.
+// stages that 147 KB hold: the tensor pipe was 28 % busy, the issue slots 15 %, L2 7 % at 261 us.  With tiles of 32 keys it ran 332 us, with all of Q in shared memory as well (two stages of 32 keys) 446.
+// Measured (B200, 2,048 tokens of 16 heads over 512 + 64): the mma.sync kernel it replaced for uncut keys 494 us, this one 199 us (261 before the issuing threads were elected).
 #include "latent_attention.cuh"
 #include "tc_attention.cuh"
 
