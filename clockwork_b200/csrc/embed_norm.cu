@@ -119,14 +119,21 @@ __device__ __forceinline__ float warp_square_sum(const float4 (&v)[NV], int lane
 template <typename T, int NV, bool CENTER>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_warp_kernel(float* __restrict__ resid, const T* __restrict__ delta, const float* __restrict__ weight,
-                        T* __restrict__ out, int num_rows, float eps, int H, const float* __restrict__ weight2, T* __restrict__ out2) {
+                        T* __restrict__ out, const int* __restrict__ rows, int num_rows, int num_resid_rows, float eps, int H, int* status,
+                        const float* __restrict__ weight2, T* __restrict__ out2) {
     pdl_launch_dependents();
     pdl_wait();
     const int lane = threadIdx.x & 31;
     const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (r >= num_rows) return;
-    float* x = resid + (size_t)r * H;
-    const T* d = delta ? delta + (size_t)r * H : nullptr;
+    const int src_row = rows != nullptr ? rows[r] : r;
+    if (src_row < 0 || src_row >= num_resid_rows) {
+        if (lane == 0) cw_report(status, CW_ST_ROW_RANGE, r, src_row);
+        for (int c = lane * 4; c < H; c += 128) Vec4<T>::store(out + (size_t)r * H + c, make_float4(0.f, 0.f, 0.f, 0.f));
+        return;
+    }
+    float* x = resid + (size_t)src_row * H;
+    const T* d = delta ? delta + (size_t)src_row * H : nullptr;
     float4 v[NV];
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
@@ -159,13 +166,14 @@ add_rmsnorm_warp_kernel(float* __restrict__ resid, const T* __restrict__ delta, 
 }
 
 template <typename T, bool CENTER>
-static int launch_rmsnorm_warp(float* resid, const T* delta, const float* weight, T* out, int rows, int H, float eps,
-                               const float* weight2, T* out2, cudaStream_t stream) {
-    const int warps = 8;
-    const dim3 grid((rows + warps - 1) / warps), block(warps * 32);
+static int launch_rmsnorm_warp(float* resid, const T* delta, const float* weight, T* out, const int* rows, int num_rows, int num_resid_rows,
+                               int H, float eps, int* status, const float* weight2, T* out2, cudaStream_t stream) {
+    int warps = 8;  // (smaller blocks where those of eight rows would leave SMs without one)
+    while (warps > 1 && num_rows < warps * 148) warps >>= 1;
+    const dim3 grid((num_rows + warps - 1) / warps), block(warps * 32);
     const int nv = (H + 127) / 128;
 #define CW_NV(n) \
-    if (nv <= n) return cw_launch(add_rmsnorm_warp_kernel<T, n, CENTER>, grid, block, 0, stream, 1, resid, delta, weight, out, rows, eps, H, weight2, out2);
+    if (nv <= n) return cw_launch(add_rmsnorm_warp_kernel<T, n, CENTER>, grid, block, 0, stream, 1, resid, delta, weight, out, rows, num_rows, num_resid_rows, eps, H, status, weight2, out2);
     CW_NV(4) CW_NV(8) CW_NV(12) CW_NV(16) CW_NV(24) CW_NV(32)
 #undef CW_NV
     return CW_ERR_UNSUPPORTED;
@@ -174,12 +182,15 @@ static int launch_rmsnorm_warp(float* resid, const T* delta, const float* weight
 template <typename T, bool CENTER>
 static int launch_add_rmsnorm(float* resid, const T* delta, const float* weight, T* out, const int* rows, int num_out_rows,
                               int num_resid_rows, int H, float eps, int* status, const float* weight2, T* out2, cudaStream_t stream) {
-    // many rows: a warp per row; few rows (decode): a block per row, for the latency of the one row
+    // many rows: a warp per row; few rows (decode): a block per row, for the latency of the one row.  Picked rows (those whose
+    // logits are wanted) from 768 on, but in float32, where the sums' order is not to follow from how many rows a step wants.
+    // us on B200, picked rows in a captured chain, a block per row -> a warp per row: 512 rows of 1536 4.5 -> 4.3, of 3584 6.2 ->
+    // 8.5 (a warp's 28 loads are a longer chain than a block's); 768 rows 4.9 -> 4.7, 10.8 -> 9.1; 2048 rows 10.8 -> 6.0, 23.6 -> 18.8
     const bool aligned = H % 4 == 0 && H <= 4096 && ((uintptr_t)resid & 15) == 0 && ((uintptr_t)weight & 15) == 0 &&
                          ((uintptr_t)out & 15) == 0 && ((uintptr_t)delta & 15) == 0 && ((uintptr_t)weight2 & 15) == 0 &&
                          ((uintptr_t)out2 & 15) == 0;
-    if (rows == nullptr && num_out_rows >= 256 && aligned)
-        return launch_rmsnorm_warp<T, CENTER>(resid, delta, weight, out, num_out_rows, H, eps, weight2, out2, stream);
+    if (num_out_rows >= 256 && (rows == nullptr || (sizeof(T) == 2 && num_out_rows >= 768)) && aligned)
+        return launch_rmsnorm_warp<T, CENTER>(resid, delta, weight, out, rows, num_out_rows, num_resid_rows, H, eps, status, weight2, out2, stream);
     const int threads = H >= 2048 ? 512 : (H >= 512 ? 256 : 128);
     return cw_launch(add_rmsnorm_kernel<T, CENTER>, dim3(num_out_rows), dim3(threads), 0, stream, 1, resid, delta, weight, out, rows,
                      num_resid_rows, eps, H, status, weight2, out2);

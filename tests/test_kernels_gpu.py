@@ -76,6 +76,25 @@ def test_add_rmsnorm(ops, status, dtype, n, h):
     ops.raise_on_status(status)
 
 
+@pytest.mark.parametrize("n", [767, 768, 1185])  # a block per row below 768 picked rows, a warp per row from there (blocks of 4 and 8)
+@pytest.mark.parametrize("h,center", [(200, False), (1536, True), (4096, False), (4100, False)])
+def test_rmsnorm_of_many_picked_rows(ops, status, n, h, center):
+    resid, weight = rand(300, h, scale=3.0).to(DEV), (1 + 0.1 * rand(h, seed=2)).float().to(DEV)
+    rows = ((torch.arange(n) * 7) % 300).to(torch.int32)
+    out = ops.rmsnorm_rows(resid, rows.to(DEV), weight, 1e-5, torch.bfloat16, status, center=center)
+    x = resid.cpu()[rows.long()]
+    if center:
+        x = x - x.mean(1, keepdim=True)
+    torch.testing.assert_close(out.float().cpu(), plain.rms_norm(x, weight.cpu(), 1e-5), **tol(torch.bfloat16, 3))
+    ops.raise_on_status(status)
+    rows[[0, n - 1]] = torch.tensor([300, -1], dtype=torch.int32)  # rows that are not there: zeros, and a status
+    bad = ops.new_status(DEV)
+    out = ops.rmsnorm_rows(resid, rows.to(DEV), weight, 1e-5, torch.bfloat16, bad, center=center)
+    assert not out[0].any() and not out[n - 1].any() and bool(out[1].any())
+    with pytest.raises(Exception):
+        ops.raise_on_status(bad)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_gemm_ref_shapes_epilogues_and_row_independence(ops, dtype):
     m, n, k = 37, 129, 200
