@@ -137,7 +137,6 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // before its first kernel; only q and the newest keys and values come from the preceding kernels.
     // So everything up to the first TMA load runs while the preceding kernel finishes, and only the
     // producer warp, whose loads are the kernel's only reads of that data, waits for it.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int h = blockIdx.x, item = blockIdx.y;
     const int s = p.item_seq[item], q0 = p.item_q0[item];
@@ -185,6 +184,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
     tc_fence_before();
     __syncthreads();
+    pdl_release();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 

@@ -130,7 +130,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     uint32_t* tmem_slot = (uint32_t*)(bars + 2 * C::STAGES + 2);
     volatile int* give_up = (volatile int*)(tmem_slot + 1);
 
-    pdl_launch_dependents();
+    cw_trace(0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN, split = blockIdx.z;
     const int kb0 = split * p.kb_per_split;
@@ -162,6 +162,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant_
     if (warp == 2) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
     tc_fence_before();
     __syncthreads();
+    pdl_release();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     // Every inbox barrier of the cluster is initialised before any CTA can push (long before: the
@@ -522,7 +523,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     // Only the activations come from the preceding kernel, and only the producer thread reads them
     // (everything else follows from its copies): it alone waits for that kernel, after the set-up and
     // after the weight tiles of the first stages have gone out.
-    pdl_launch_dependents();
+    cw_trace(0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + C::STAGES);
     const uint32_t accf0 = smem_u32(bars + 2 * C::STAGES), acce0 = smem_u32(bars + 2 * C::STAGES + 2);
@@ -550,6 +551,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
     tc_fence_before();
     __syncthreads();
+    pdl_release();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 

@@ -111,7 +111,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     // Only the activations come from the preceding kernel, and only the producer threads read them
     // (everything else follows from their copies): they alone wait for it, after the set-up and after
     // the weight tiles of the first stages have gone out.
-    pdl_launch_dependents();
+    cw_trace(0);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = cluster_rank();  // 0: the leader, which issues the MMAs
     const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + PAIR_MAX_STAGES);
@@ -137,6 +137,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_cons
     if (warp == 1) tmem_alloc_pair(smem_u32(tmem_slot), C::TMEM_COLS);
     tc_fence_before();
     cluster_sync();  // both CTAs' barriers are initialised before either signals the other's
+    pdl_release();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 

@@ -105,7 +105,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), C::TMEM_COLS);
-    pdl_enter();
+    pdl_wait();
     if (warp == 0) {
         int run = 0;
         for (int g0 = 0; g0 < p.G; g0 += 32) {
@@ -130,6 +130,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     }
     tc_fence_before();
     __syncthreads();
+    pdl_release();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
     const int ftiles = (p.Nout + GT_BM - 1) / GT_BM, tiles = cum[p.G] * ftiles, num_kb = (p.K + GT_BK - 1) / GT_BK;

@@ -69,7 +69,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     const int split = blockIdx.x % p.splits, block = blockIdx.x / p.splits;
     const long long total_rows = (long long)a.N * H;
 
-    pdl_enter();
+    pdl_wait();
     if (split == 0) {  // rows of no request (padding of a fixed-shape step) come out as zeros
         const long long first = (long long)block * LC_ROWS, last = min(total_rows, first + LC_ROWS);
         for (long long t = first / H; t * H < last; ++t)
@@ -105,6 +105,7 @@ latent_attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
     tc_fence_before();
     __syncthreads();
+    pdl_release();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot, s_col = tmem + LC_S_COL;
     const int tok0 = row0 / H, head0 = row0 - tok0 * H, p0 = a.positions[tok0];
