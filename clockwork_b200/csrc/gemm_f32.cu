@@ -1,14 +1,22 @@
 // Float32 products on the 5th-generation tensor cores, as exact as on the CUDA cores.
 //
-// A float32 number is the sum of three bfloat16 numbers of 8 bits each: w = w0 + w1 + w2, x = x0 + x1 + x2, the first cut off (so
-// that it does not overflow), the second rounded (so that the third has either sign and what is left out below has no
-// direction).  The tensor cores form w0 x0 and the six products w1 x0, w0 x1, w1 x1, w2 x0, w0 x2 and w2 x1 exactly and add
-// them up in float32, cutting off what falls below the last bit; w1 x2 and w2 x2, at most 2^-24 of w0 x0, are left out.  So that little falls off, w0 x0 has an
-// accumulator of its own for every 16 k, the small products two for 64 k; per 64 k the six are read out of tensor memory,
-// added, and their sum is added into a running sum that carries its rounding errors along (Kahan).  Measured against float64
-// (B200, K 1,536 and 8,960, this kernel and the chains of 16 fmaf with the same running sum that it replaced): normal operands
-// 6.8e-8 and 7.3e-8, chains 8.1e-8 and 8.6e-8; sizes spread over e^3 8.5e-8 and 8.1e-8, chains 7.8e-8; operands of one sign 3.1e-8
-// and 2.8e-8, chains 2.3e-8.  With one accumulator for all products of 64 k 8.6e-8 to 1.5e-7.
+// A float32 number is the sum of three bfloat16 numbers: w = w0 + w1 + w2, x = x0 + x1 + x2, the first of 6 bits, the second of 8,
+// both rounded, the third what is left, 8 bits at most.  The second comes times 2^8, the third times 2^16, so that none of it falls
+// below bfloat16's range: the parts of every finite number are the number.  The tensor cores form w0 x0 and the seven products
+// w1 x0, w0 x1 | w1 x1, w2 x0, w0 x2 | w1 x2, w2 x1 exactly and add them up in float32, cutting off what falls below the last bit;
+// w2 x2, at most 2^-30 of w0 x0, is left out.  So that little falls off, w0 x0 (12 bits, a sum of which mostly fits whole) has an
+// accumulator of its own for every 16 k, the small products three by their factor, 2^8, 2^16 and 2^24, for 64 k; per 64 k the four
+// are read out of tensor memory, added in pairs, and the pairs are added into a running sum that carries its rounding errors
+// along (Kahan); the small ones join what it carries.  Outputs that are not finite are formed again by fmaf (f32_plain).
+// Root mean square of the error over the sum of the products' magnitudes, in 2^-24 (B200, 200 x 4,000 outputs six times, K 64,
+// 1,536 and 8,960), this kernel and the chains of 16 fmaf with the same running sum that it replaced:
+//   normal operands          0.093 0.025 0.0104   chains 0.261 0.055 0.0238
+//   sizes spread over e      0.251 0.091 0.0404          0.475 0.139 0.0637
+//   sizes spread over e^3    0.755 0.638 0.543           0.931 0.672 0.563
+//   one sign                 0.495 0.336 0.417           0.732 0.349 0.444
+//   between 0 and 1          0.478 0.391 0.529           0.720 0.402 0.562
+// Tried: first parts of 8 bits, one sign 0.45 at K of 1,536; all four of w0 x0 and the small ones carried along one by one, 10 % less
+// of an error and 296 us instead of 242 for [gate, up] of 200 rows.
 //
 // Every output's sum has the same order whatever M, N or the tile it falls in, so a row's result does not depend on the rest of
 // the batch: 64 k at a time, a long K cut into segments of about F32_SEGMENT by K alone, each segment on a CTA of a cluster;
@@ -16,13 +24,13 @@
 //
 // A CTA: up to 128 weight rows (the MMA's M) by up to 64 tokens (its N).  Eight warps copy the operands' next 64 k into
 // shared memory, cut them in three and store them there as the MMAs read them (K-major, 128-byte swizzle), two stages;
-// a thread of another issues the MMAs.  The parts of the token rows follow one another, so that one MMA of twice the width forms
-// w1 [x0 | x1], w0 [x1 | x2] or w2 [x0 | x1]: 16 MMAs per 64 k, none of which takes less than about 64 cycles however narrow.
+// a thread of another issues the MMAs.  The parts of the token rows follow one another, so that one MMA of two or three times the width
+// forms w1 [x0 | x1 | x2], w2 [x0 | x1] or w0 [x1 | x2]: 16 MMAs per 64 k, none of which takes less than about 64 cycles however narrow.
 // Eight other warps read out and add up what has been formed.  What bounds it: few rows, the 16 MMAs in a row (about 1,600 cycles per
-// 64 k); many, the issue slots (60 % busy: the cutting in three, then the sums) beside them.  Measured (B200, us, chains of fmaf
-// -> this): 200 rows, [gate, up] 2 x 8,960 by 1,536 370 -> 200, 1,536 by 8,960 217 -> 125, 2,048 by 1,536 62 -> 38; 64 rows
-// 168 -> 56, 105 -> 44, 32 -> 29; 1 row 36 -> 35, 34 -> 39, 27 -> 25.  Tried: the same eight warps for both jobs, one after the
-// other (207 us for [gate, up] of 200 rows: every step's latency in a row), sixteen (199).
+// 64 k); many, the way through shared memory and the cutting in three, then the sums (without either of the two [gate, up] of 200
+// rows takes 214 us).  Measured (B200, us, chains of fmaf -> this): 200 rows, [gate, up] 2 x 8,960 by 1,536 373 -> 242, 1,536 by
+// 8,960 219 -> 150, 2,048 by 1,536 64 -> 40; 64 rows 170 -> 70, 108 -> 47, 33 -> 33; 1 row 37 -> 37, 36 -> 41, 27 -> 27.
+// Tried: the same eight warps for both jobs, one after the other: every step's latency in a row.
 //
 // Every wait on an mbarrier is bounded.
 #include "cluster_places.cuh"
@@ -47,13 +55,71 @@ __device__ __forceinline__ void f32_add(float& sum, float& lost, float x) {
     sum = t;
 }
 
-// The first 8 of a float's 24 bits as a float; of two such floats, the upper halves side by side.
-__device__ __forceinline__ float first8(float x) { return __uint_as_float(__float_as_uint(x) & 0xffff0000u); }
-__device__ __forceinline__ uint32_t upper2(float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); }
+// Two floats in one 64-bit register: an instruction for both (the issue slots bound this kernel).
+typedef unsigned long long float_pair;
+__device__ __forceinline__ float_pair pair_of(uint32_t x, uint32_t y) {
+    float_pair v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(x), "r"(y));
+    return v;
+}
+__device__ __forceinline__ void apart(float_pair v, uint32_t& x, uint32_t& y) { asm("mov.b64 {%0, %1}, %2;" : "=r"(x), "=r"(y) : "l"(v)); }
+__device__ __forceinline__ float_pair pair_add(float_pair a, float_pair b) {
+    float_pair v;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ float_pair pair_sub(float_pair a, float_pair b) {
+    float_pair v;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ float_pair pair_mul(float_pair a, float_pair b) {
+    float_pair v;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(v) : "l"(a), "l"(b));
+    return v;
+}
+__device__ __forceinline__ float_pair pair_fma(float_pair a, float_pair b, float_pair c) {
+    float_pair v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(v) : "l"(a), "l"(b), "l"(c));
+    return v;
+}
+__device__ __forceinline__ float_pair both(float x) { return pair_of(__float_as_uint(x), __float_as_uint(x)); }
+__device__ __forceinline__ void pair_add(float_pair& sum, float_pair& lost, float_pair x) {  // f32_add
+    const float_pair y = pair_sub(x, lost);
+    const float_pair t = pair_add(sum, y);
+    lost = pair_sub(pair_sub(t, sum), y);
+    sum = t;
+}
 
-__device__ __forceinline__ uint32_t rounded2(float x, float y) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
-    return *reinterpret_cast<const uint32_t*>(&v);
+// The first 6 of a float's 24 bits, rounded (half a step away from zero).
+__device__ __forceinline__ uint32_t first6(uint32_t x) { return (x + 0x20000u) & 0xfffc0000u; }
+// Of two floats, the upper halves side by side.
+__device__ __forceinline__ uint32_t upper2(uint32_t x, uint32_t y) { return __byte_perm(x, y, 0x7632); }
+
+// The three parts of two numbers, as bfloat16 side by side; the second comes times 2^8, the third times 2^16.  The parts of numbers
+// from 2^126 on may be infinite: see f32_plain().
+__device__ __forceinline__ void three_parts(uint32_t x, uint32_t y, uint32_t& q0, uint32_t& q1, uint32_t& q2) {
+    const uint32_t x0 = first6(x), y0 = first6(y);
+    q0 = upper2(x0, y0);
+    const float_pair rest = pair_mul(pair_sub(pair_of(x, y), pair_of(x0, y0)), both(256.f));
+    uint32_t u, v;
+    apart(rest, u, v);
+    const __nv_bfloat162 rounded = __floats2bfloat162_rn(__uint_as_float(u), __uint_as_float(v));
+    q1 = *reinterpret_cast<const uint32_t*>(&rounded);
+    apart(pair_mul(pair_sub(rest, pair_of(q1 << 16, q1 & 0xffff0000u)), both(256.f)), u, v);
+    q2 = upper2(u, v);  // (whole: 8 bits at most are left)
+}
+
+// The product of two rows by fmaf, 16 k at a time: for the outputs that are not finite.  Parts of an infinite operand are no numbers, and
+// those of the largest ones are infinite, where the product may be infinite, or finite.
+__device__ __noinline__ float f32_plain(const float* a, const float* w, int K) {
+    float sum = 0.f, lost = 0.f;
+    for (int k0 = 0; k0 < K; k0 += 16) {
+        float chain = 0.f;
+        for (int k = k0; k < min(K, k0 + 16); ++k) chain = fmaf(a[k], w[k], chain);
+        f32_add(sum, lost, chain);
+    }
+    return sum;
 }
 
 __device__ __forceinline__ void f32_cluster_barrier() {
@@ -67,6 +133,8 @@ __device__ __forceinline__ float2 load_of_rank(const void* mine, int rank) {  //
 
 template <bool SWIGLU>
 __device__ __forceinline__ void f32_store(const F32Args& p, int m, int n, float v, float up) {
+    if (!isfinite(v)) v = f32_plain(p.A + (size_t)m * p.lda, p.W + (size_t)n * p.K, p.K);
+    if (SWIGLU && !isfinite(up)) up = f32_plain(p.A + (size_t)m * p.lda, p.W2 + (size_t)n * p.K, p.K);
     if (p.bias) v += p.bias[n];
     float* to = p.C + (size_t)m * p.ldc + n;
     if (SWIGLU) {
@@ -87,8 +155,8 @@ struct F32Cfg {
     static constexpr int W_PART = F32_ROWS * F32_BK * 2, X_PART = BN * F32_BK * 2;  // one of the three parts of an operand (rows: at most)
     static constexpr int STAGE = 3 * (W_PART + X_PART);
     static constexpr int MINE = BN / 32;                          // groups of 16 tokens of an adding warp
-    // Tensor memory: four accumulators of w0 x0 (twice where there is room), two of the small products twice, so that the next
-    // 64 k's are formed while these are read out.
+    // Tensor memory: four accumulators of w0 x0 and three of the small products, twice where there is room, so that the next 64 k's
+    // are formed while these are read out.
     static constexpr int SETS = BN <= 32 ? 2 : 1, SMALL = SETS * 4 * BN, TMEM_COLS = 512;
     // Pieces of eight numbers of 64 k that a converting thread brings, and how many times 64 k it has on their way: as many as there
     // is room for (few rows per CTA are bound by the latency of these copies).
@@ -97,7 +165,7 @@ struct F32Cfg {
     static constexpr int AHEAD = ROOM < 6 ? ROOM : 6;
     static constexpr int RAW = AHEAD * PIECES * 32 * F32_CONVERTERS * 32;
     static constexpr int SMEM = 2 * STAGE + RAW + 1024 + 256;
-    static_assert(SMALL + 4 * BN <= TMEM_COLS && BN % 32 == 0, "accumulators");
+    static_assert(SETS * 7 * BN <= TMEM_COLS && BN % 32 == 0, "accumulators");
     static_assert(BN * F32_ROWS * 8 <= 2 * STAGE, "sums and what they lost fit where the operands were");
     static_assert(AHEAD >= 1 && SMEM <= 226 * 1024, "shared memory");
 };
@@ -152,7 +220,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
         if (warp == F32_ADDERS + F32_CONVERTERS && elect_one()) {
             // ---- MMA issuer ------------------------------------------------------------------------------------------
             const int x_part = groups * 16 * F32_BK * 2;
-            const uint32_t idesc = instr_desc(F32_ROWS, 16 * groups), idesc2 = instr_desc(F32_ROWS, 32 * groups);
+            const uint32_t wide = 16 * groups, idesc = instr_desc(F32_ROWS, wide), idesc2 = instr_desc(F32_ROWS, 2 * wide), idesc3 = instr_desc(F32_ROWS, 3 * wide);
             bool ok = true;
             for (int b = 0; b < blocks && ok; ++b) {
                 const int set = b % C::SETS;
@@ -163,21 +231,21 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
                 const uint32_t stage = smem_u32(smem) + (b & 1) * C::STAGE;
                 const uint64_t w0 = smem_desc_sw128(stage), w1 = w0 + C::W_PART / 16, w2 = w1 + C::W_PART / 16;
                 const uint64_t x0 = w2 + C::W_PART / 16, x1 = x0 + x_part / 16;
-                const uint32_t small = tmem + C::SMALL + (b & 1) * 2 * BN;
+                const uint32_t small = tmem + C::SMALL + set * 3 * BN;
 #pragma unroll
                 for (int k = 0; k < F32_BK / 16; ++k) umma_bf16(tmem + (set * 4 + k) * BN, w0 + 2 * k, x0 + 2 * k, idesc, 0u);
                 umma_commit(first_full + 8 * set);
-                ok = mbar_wait(small_empty + 8 * (b & 1), ((b >> 1) & 1) ^ 1, give_up);
+                ok = mbar_wait(small_empty + 8 * set, ((b / C::SETS) & 1) ^ 1, give_up);
                 if (!ok) break;
                 tc_fence_after();
 #pragma unroll
-                for (int k = 0; k < F32_BK / 16; ++k) umma_bf16(small, w2 + 2 * k, x0 + 2 * k, idesc2, k > 0 ? 1u : 0u);
+                for (int k = 0; k < F32_BK / 16; ++k) umma_bf16(small, w1 + 2 * k, x0 + 2 * k, idesc3, k > 0 ? 1u : 0u);
+#pragma unroll
+                for (int k = 0; k < F32_BK / 16; ++k) umma_bf16(small + wide, w2 + 2 * k, x0 + 2 * k, idesc2, 1u);
 #pragma unroll
                 for (int k = 0; k < F32_BK / 16; ++k) umma_bf16(small, w0 + 2 * k, x1 + 2 * k, idesc2, 1u);
-#pragma unroll
-                for (int k = 0; k < F32_BK / 16; ++k) umma_bf16(small, w1 + 2 * k, x0 + 2 * k, idesc2, 1u);
                 umma_commit(empty0 + 8 * (b & 1));  // the stage has been read
-                umma_commit(small_full + 8 * (b & 1));
+                umma_commit(small_full + 8 * set);
             }
         }
         __syncwarp();
@@ -242,28 +310,22 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
 #pragma unroll
             for (int at = 0; at < BATCHES; ++at) {
                 asm volatile("cp.async.wait_group %0;" ::"n"(C::AHEAD * BATCHES - 1) : "memory");
-                float4 x[2][2];
+                uint4 x[2][2];
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
                     if (2 * at + h < C::PIECES) {
                         const float* from = raw + (b % C::AHEAD * C::PIECES + 2 * at + h) * 8 * NT;
-                        x[h][0] = *reinterpret_cast<const float4*>(from);
-                        x[h][1] = *reinterpret_cast<const float4*>(from + 4);
+                        x[h][0] = *reinterpret_cast<const uint4*>(from);
+                        x[h][1] = *reinterpret_cast<const uint4*>(from + 4);
                     }
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int i = 2 * at + h;
                     if (i >= C::PIECES || !has(i)) continue;
-                    const float y[8] = {x[h][0].x, x[h][0].y, x[h][0].z, x[h][0].w, x[h][1].x, x[h][1].y, x[h][1].z, x[h][1].w};
+                    const uint32_t y[8] = {x[h][0].x, x[h][0].y, x[h][0].z, x[h][0].w, x[h][1].x, x[h][1].y, x[h][1].z, x[h][1].w};
                     uint32_t q[3][4];
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float u = y[2 * j], v = y[2 * j + 1], u1 = u - first8(u), v1 = v - first8(v);
-                        const uint32_t rounded = rounded2(u1, v1);
-                        q[0][j] = upper2(u, v);
-                        q[1][j] = rounded;
-                        q[2][j] = upper2(u1 - __uint_as_float(rounded << 16), v1 - first8(__uint_as_float(rounded)));
-                    }
+                    for (int j = 0; j < 4; ++j) three_parts(y[2 * j], y[2 * j + 1], q[0][j], q[1][j], q[2][j]);
                     const bool of_w = i < C::W_PIECES;
                     uint8_t* to = stage + (of_w ? i * APART * 128 : 3 * C::W_PART + (i - C::W_PIECES) * APART * 128);
                     const int part = of_w ? C::W_PART : x_part;
@@ -283,13 +345,13 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
         }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
-        float sum[C::MINE][16] = {}, lost[C::MINE][16] = {};  // [group][token]: this thread's feature, half of the groups of 16 tokens
+        float_pair sum[C::MINE][8] = {}, lost[C::MINE][8] = {};  // [group][tokens]: this thread's feature, half of the groups of 16 tokens
         const int quarter = warp & 3, half = (groups + 1) >> 1, group0 = (warp >> 2) * half, mine_groups = min(half, groups - group0);
         const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16) + 16 * group0;
         bool ok = true;
         auto add_up = [&](int b) {
-            // One accumulator's columns of all groups are loaded before the first is used: a load from tensor memory takes
-            // about 200 cycles, and a group after the other paid them each time (80 tokens: 2,400 cycles per 64 k).
+            // One accumulator's columns of all groups are loaded before the first is used, and while the last ones are added: a load
+            // from tensor memory takes about 200 cycles.
             uint32_t t[C::MINE][16], r[C::MINE][16];
             const bool reads = quarter * 32 < p.rows;
             auto load = [&](uint32_t (&to)[C::MINE][16], uint32_t column) {
@@ -301,49 +363,60 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
 #pragma unroll
                 for (int g = 0; g < C::MINE; ++g) tmem_landed(at[g]);
             };
-            auto add = [&]() {
+            auto each_pair = [&](auto f) {
 #pragma unroll
                 for (int g = 0; g < C::MINE; ++g)
                     if (g < mine_groups)
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) t[g][j] = __float_as_uint(__fadd_rn(__uint_as_float(t[g][j]), __uint_as_float(r[g][j])));
+                        for (int j = 0; j < 8; ++j) f(g, j);
+            };
+            auto add = [&](uint32_t (&x)[C::MINE][16]) {
+                each_pair([&](int g, int j) { pair_add(sum[g][j], lost[g][j], pair_of(x[g][2 * j], x[g][2 * j + 1])); });
+            };
+            auto plus = [&](uint32_t (&x)[C::MINE][16], uint32_t (&y)[C::MINE][16]) {
+                each_pair([&](int g, int j) {
+                    apart(pair_add(pair_of(x[g][2 * j], x[g][2 * j + 1]), pair_of(y[g][2 * j], y[g][2 * j + 1])), x[g][2 * j], x[g][2 * j + 1]);
+                });
+            };
+            auto later = [&](uint32_t (&x)[C::MINE][16], float less) {  // the small products join what the sum has lost
+                each_pair([&](int g, int j) { lost[g][j] = pair_fma(pair_of(x[g][2 * j], x[g][2 * j + 1]), both(less), lost[g][j]); });
+            };
+            auto read_out = [&](uint32_t barrier) {  // this warp has read the accumulators
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(barrier) : "memory");
             };
             const int set = b % C::SETS;
-            const uint32_t main0 = set * 4 * BN, small = C::SMALL + (b & 1) * 2 * BN;
-            ok = __all_sync(0xffffffffu, mbar_wait(first_full + 8 * set, (b / C::SETS) & 1, give_up));
+            const uint32_t parity = (b / C::SETS) & 1, main0 = set * 4 * BN, small = C::SMALL + set * 3 * BN, wide = 16 * groups;
+            ok = __all_sync(0xffffffffu, mbar_wait(first_full + 8 * set, parity, give_up));
             if (!ok) return;
             tc_fence_after();
             load(t, main0);
             load(r, main0 + BN);
             landed(t);
             landed(r);
-            add();
+            plus(t, r);
             load(r, main0 + 2 * BN);
+            add(t);
+            load(t, main0 + 3 * BN);
+            landed(t);
             landed(r);
-            add();
-            load(r, main0 + 3 * BN);
-            landed(r);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(first_empty + 8 * set) : "memory");
-            add();
-            ok = __all_sync(0xffffffffu, mbar_wait(small_full + 8 * (b & 1), (b >> 1) & 1, give_up));
+            read_out(first_empty + 8 * set);
+            plus(t, r);
+            add(t);
+            ok = __all_sync(0xffffffffu, mbar_wait(small_full + 8 * set, parity, give_up));
             if (!ok) return;
             tc_fence_after();
-            load(r, small);
+            load(t, small);
+            load(r, small + wide);
+            landed(t);
             landed(r);
-            add();
-            load(r, small + 16 * groups);
-            landed(r);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(small_empty + 8 * (b & 1)) : "memory");
-            add();
-#pragma unroll
-            for (int g = 0; g < C::MINE; ++g)
-                if (g < mine_groups)
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) f32_add(sum[g][j], lost[g][j], __uint_as_float(t[g][j]));
+            later(t, -0x1p-8f);
+            load(t, small + 2 * wide);
+            later(r, -0x1p-16f);
+            landed(t);
+            read_out(small_empty + 8 * set);
+            later(t, -0x1p-24f);
         };
         for (int b = 0; b < blocks && ok; ++b) add_up(b);
         // ---- results: this thread's feature (tensor-memory lane `row`), tokens 16 (group0 + g) + j ---------------------------------------
@@ -356,18 +429,21 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
                     const int t = 16 * (group0 + g) + j;
-                    if (g < half && t < tokens) f(t, sum[g][j], lost[g][j]);
+                    uint32_t s[2], l[2];
+                    apart(sum[g][j / 2], s[0], s[1]);
+                    apart(lost[g][j / 2], l[0], l[1]);
+                    if (g < half && t < tokens) f(t, __uint_as_float(s[j & 1]), __uint_as_float(l[j & 1]));
                 }
         };
         if (segments == 1) {
             float* ups = (float*)smem;  // [token][64 features]
             if (SWIGLU) {
-                if (mine && (quarter & 1)) each([&](int t, float s, float) { ups[t * 64 + (quarter >> 1) * 32 + lane] = s; });
+                if (mine && (quarter & 1)) each([&](int t, float s, float l) { ups[t * 64 + (quarter >> 1) * 32 + lane] = s - l; });
                 asm volatile("bar.sync 1, %0;" ::"n"(32 * F32_ADDERS) : "memory");
             }
             const int n = n0 + (SWIGLU ? (quarter >> 1) * 32 + lane : row);
             if (mine && !(SWIGLU && (quarter & 1)) && n < p.N)
-                each([&](int t, float s, float) { f32_store<SWIGLU>(p, m0 + t, n, s, SWIGLU ? ups[t * 64 + (quarter >> 1) * 32 + lane] : 0.f); });
+                each([&](int t, float s, float l) { f32_store<SWIGLU>(p, m0 + t, n, s - l, SWIGLU ? ups[t * 64 + (quarter >> 1) * 32 + lane] : 0.f); });
         } else {
             float2* part = (float2*)smem;  // [token][weight row]: (sum, lost)
             if (mine) each([&](int t, float s, float l) { part[t * F32_ROWS + row] = make_float2(s, l); });
@@ -387,10 +463,12 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
                     total[u] = s[0].x;
 #pragma unroll
                     for (int i = 1; i < F32_MAX_SEGMENTS; ++i)
-                        if (i < segments) {
-                            f32_add(total[u], left, s[i].x);
-                            left += s[i].y;
+                        if (i < segments) {  // (the segments are alike in size: what either addend loses goes into `left`)
+                            const float sum = __fadd_rn(total[u], s[i].x), of_total = __fsub_rn(sum, s[i].x), of_next = __fsub_rn(sum, of_total);
+                            left = __fadd_rn(left, __fsub_rn(s[i].y, __fadd_rn(__fsub_rn(total[u], of_total), __fsub_rn(s[i].x, of_next))));
+                            total[u] = sum;
                         }
+                    total[u] -= left;
                 }
                 f32_store<SWIGLU>(p, m0 + t, n, total[0], total[1]);
             }

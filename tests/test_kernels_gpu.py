@@ -123,10 +123,13 @@ def test_gemm_ref_shapes_epilogues_and_row_independence(ops, dtype):
 
 
 @pytest.mark.parametrize("m,n,k", [(1, 33, 4), (8, 64, 36), (16, 32, 16), (17, 31, 20), (33, 129, 200), (200, 2048, 1536), (257, 6000, 52)])
-def test_gemm_ref_float32_tiles_give_the_plain_kernels_bits(ops, m, n, k):
-    """The kernel for rows of whole 16-byte pieces at the edges of its tile sizes, against the one that takes any
-    row (a left operand whose rows lie an odd number of words apart): the same sums in the same order, so the same bits."""
+def test_gemm_ref_float32_rows_aligned_or_not_give_the_same_bits(ops, m, n, k):
+    """Rows of whole 16-byte pieces at the edges of the tile sizes, against rows that lie an odd number of words apart, which are
+    copied a word at a time: the same sums in the same order, so the same bits, and those within the bound of the chains (see the
+    next test)."""
     a, w, bias = rand(m, k).to(DEV), rand(n, k, scale=0.1, seed=1).to(DEV), rand(n, seed=2).to(DEV)
+    exact, sizes = a.cpu().double() @ w.cpu().double().T, a.cpu().double().abs() @ w.cpu().double().abs().T
+    assert ((ops.gemm_ref(a, w).cpu().double() - exact).abs() <= 19 * 2.0**-24 * sizes).all()
     odd = torch.zeros(m + 1, k + 1, device=DEV)[:m, :k].copy_(a)
     assert odd.stride(0) % 4
     for epilogue in (ops.EPILOGUE_STORE, ops.EPILOGUE_STORE_F32, ops.EPILOGUE_RELU2):
@@ -137,15 +140,15 @@ def test_gemm_ref_float32_tiles_give_the_plain_kernels_bits(ops, m, n, k):
     ops.gemm_ref(odd, w, bias, out=want, epilogue=ops.EPILOGUE_ADD_F32)
     assert torch.equal(got, want)
     up = rand(n, k, scale=0.1, seed=4).to(DEV)
-    shifted = torch.zeros(n * k + 1, device=DEV)[1:].view(n, k).copy_(up)  # not on a 16-byte boundary: the plain kernel
+    shifted = torch.zeros(n * k + 1, device=DEV)[1:].view(n, k).copy_(up)  # not on a 16-byte boundary
     assert torch.equal(ops.gemm_ref_swiglu(a, w, up), ops.gemm_ref_swiglu(a, w, shifted))
 
 
 @pytest.mark.parametrize("n,k", [(100, 1540), (65, 3584), (96, 8960), (33, 18948)])
 def test_gemm_ref_float32_cut_inner_dimension(ops, n, k):
-    """Inner dimensions that are cut over a cluster: the error bound of chains of 16 (16 units of 2^-24 of the sum of
-    magnitudes) and of the compensated sums behind them (2 more, and 1 for the store), and the same bits for a row
-    whatever the number of rows, which picks the tile."""
+    """Inner dimensions that are cut over a cluster: the error bound that chains of 16 fmaf have (16 units of 2^-24 of the sum of
+    magnitudes) with the compensated sums behind them (2 more, and 1 for the store), to which these products are held
+    whatever forms them, and the same bits for a row whatever the number of rows, which picks the tile."""
     rows = 150
     a, w = rand(rows, k), rand(n, k, scale=0.1, seed=1)
     ad, wd = a.to(DEV), w.to(DEV)
