@@ -29,7 +29,7 @@
 // Eight other warps read out and add up what has been formed.  What bounds it: few rows, the 16 MMAs in a row (about 1,600 cycles per
 // 64 k); many, the way through shared memory and the cutting in three, then the sums (without either of the two [gate, up] of 200
 // rows takes 214 us).  Measured (B200, us, chains of fmaf -> this): 200 rows, [gate, up] 2 x 8,960 by 1,536 373 -> 242, 1,536 by
-// 8,960 219 -> 150, 2,048 by 1,536 64 -> 40; 64 rows 170 -> 70, 108 -> 47, 33 -> 33; 1 row 37 -> 37, 36 -> 41, 27 -> 27.
+// 8,960 219 -> 150, 2,048 by 1,536 64 -> 40; 64 rows 170 -> 70, 108 -> 47, 33 -> 33; 1 row 37 -> 37, 36 -> 34, 27 -> 27.
 // Tried: the same eight warps for both jobs, one after the other: every step's latency in a row.
 //
 // Every wait on an mbarrier is bounded.
@@ -508,8 +508,9 @@ static int launch_f32_any(const F32Args& p, int segments, cudaStream_t stream) {
 }
 
 // The tile with the least time by cycles per 64 k that fit what was measured: 11 for a row of either operand, 15 for a token, 600
-// besides; a round of CTAs costs 5,000 more.  32 weight rows per CTA (64 with SwiGLU) pay where there are few tiles: 1 row by
-// 2,048 x 1,536 takes 25 us so and 33 with 128.  The sums do not depend on the choice.
+// besides; a round of CTAs costs 5,000 more (six products at 1 to 600 rows: within 5 % of the best tile, once 10 %).  32 or 64 weight
+// rows per CTA pay where there are few tiles: 1 row by 2,048 x 1,536 takes 27 us with 32 and 35 with 128, 1 row by 1,536 x 8,960, five
+// segments, 34 us with 64, whose 24 clusters all find a place at once, 41 with 128.  The sums do not depend on the choice.
 int gemm_f32_run(F32Args p, cudaStream_t stream) {
     int device = 0, sms = 0;
     cudaError_t e = cudaGetDevice(&device);
@@ -520,8 +521,7 @@ int gemm_f32_run(F32Args p, cudaStream_t stream) {
     if (segments > F32_MAX_SEGMENTS) segments = F32_MAX_SEGMENTS;
     const long long places = clusters_at_once(segments, 1, sms), blocks = ((p.K + F32_BK - 1) / F32_BK + segments - 1) / segments;
     double least = -1;
-    const int few = swiglu ? 64 : 32;
-    for (int rows = F32_ROWS; rows >= few; rows = rows > few ? few : 0)
+    for (int rows = F32_ROWS; rows >= (swiglu ? 64 : 32); rows /= 2)
         for (int width = rows == F32_ROWS ? F32_MAX_TOKENS : 32; width >= 16; width -= 16) {
             if (width > 16 && width - 16 >= p.M) continue;
             const int features = swiglu ? rows / 2 : rows;
@@ -530,8 +530,8 @@ int gemm_f32_run(F32Args p, cudaStream_t stream) {
             const double cost = (double)((tiles + places - 1) / places) * ((double)blocks * block + 5000);
             if (least < 0 || cost < least) least = cost, p.width = width, p.rows = rows;
         }
-    if (p.rows < F32_ROWS)  // (with tiles of up to 32 tokens)
-        return swiglu ? launch_f32_any<32, 64, true>(p, segments, stream) : launch_f32_any<32, 32, false>(p, segments, stream);
+    if (p.rows == 32) return launch_f32_any<32, 32, false>(p, segments, stream);  // (with tiles of up to 32 tokens, like the next two)
+    if (p.rows == 64) return swiglu ? launch_f32_any<32, 64, true>(p, segments, stream) : launch_f32_any<32, 64, false>(p, segments, stream);
     if (p.width <= 32) return swiglu ? launch_f32_any<32, 128, true>(p, segments, stream) : launch_f32_any<32, 128, false>(p, segments, stream);
     return swiglu ? launch_f32_any<F32_MAX_TOKENS, 128, true>(p, segments, stream) : launch_f32_any<F32_MAX_TOKENS, 128, false>(p, segments, stream);
 }

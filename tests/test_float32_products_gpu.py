@@ -101,3 +101,12 @@ def test_numbers_that_are_not_finite(k, gated):
     exact, size = a[9].double() @ w.double().T, a[9].double().abs() @ w.double().abs().T
     assert ((got[9].double() - exact).abs() <= 19 * 2.0**-24 * size)[finite].all()
     torch.testing.assert_close(got[9][~finite], want[9][~finite], rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 32])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_few_rows_over_a_long_inner_dimension(rows, offset):
+    """1,536 features over an inner dimension of five segments: tiles of 64 weight rows, whose sums are those of tiles of 128."""
+    g = torch.Generator().manual_seed(rows)
+    a, w = torch.randn(200, 8960 + offset, generator=g).to(DEV)[:, offset:], torch.randn(1500, 8960, generator=g).to(DEV)
+    assert torch.equal(ops.gemm_ref(a[:rows], w), ops.gemm_ref(a, w)[:rows])
