@@ -1036,6 +1036,8 @@ extern "C" int cw_gemm_tc_plan(int T, int N, int K, int swiglu, int sm_count, in
     *ctas = pl.pair ? 2 * pl.tiles * pl.splits : pl.tiles * pl.splits;
     return CW_OK;
 }
+// ... and how many of its CTAs are meant to share an SM.
+extern "C" int cw_gemm_tc_plan_per_sm(int T, int N, int K, int swiglu, int sm_count) { return make_plan(T, N, K, swiglu != 0, sm_count).per_sm; }
 
 // X [T, K] (row stride ldx), W [N, K] (and W2 for SwiGLU), C [T, ldc].  Epilogues: 0 bfloat16 store, 1 add into float32, 2
 // float32 store, 4 bfloat16 store of max(v, 0)^2 (v: the product plus the bias).  K must be a multiple of 8

@@ -740,6 +740,10 @@ def test_gemm_tc_few_tokens_over_many_weight_tiles(ops, gemm_tc, t, n, k):
 def test_gemm_tc_splits_beyond_one_cta_per_sm(ops, gemm_tc, t, n, k):
     """Weight tiles times splits that no single wave of clusters holds with a CTA to an SM: two share one up to 64 tokens,
     more tokens are cut in fewer parts."""
+    from tests.test_product_plans import few_token_plan
+
+    splits, per_sm = few_token_plan(t, n, k)
+    assert splits > 1 and per_sm == (2 if t <= 64 else 1)
     test_gemm_tc_against_float64(ops, gemm_tc, t, n, k)
 
 
