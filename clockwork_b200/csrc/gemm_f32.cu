@@ -214,7 +214,11 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
 
-    // Registers: 640 threads of 96 at launch, 61,440 in all; 256 x 152 + 256 x 72 + 128 x 32 of them after the split.
+    // Registers: 640 threads of 96 at launch, 61,440 in all; 256 x 152 + 256 x 72 + 128 x 32 of them after the split (tiles of up to 32
+    // tokens 144 and 80, with which their loops keep everything in registers).
+    constexpr int ADDER_REGS = BN <= 32 ? 144 : 152, CONVERTER_REGS = BN <= 32 ? 80 : 72;
+    static_assert(32 * (F32_ADDERS * ADDER_REGS + F32_CONVERTERS * CONVERTER_REGS) + (F32_THREADS - 32 * (F32_ADDERS + F32_CONVERTERS)) * 32 <= F32_THREADS * 96,
+                  "the split draws on the registers of the launch");
     if (warp >= F32_ADDERS + F32_CONVERTERS) {
         asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
         if (warp == F32_ADDERS + F32_CONVERTERS && elect_one()) {
@@ -254,7 +258,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
             f32_cluster_barrier();
         }
     } else if (warp >= F32_ADDERS) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(CONVERTER_REGS));
         // ---- operands: eight numbers of a row a piece, eight pieces a row; a thread converts what it has copied itself.  Its
         // pieces lie 32 rows apart; two of them (a batch) are copied, awaited and converted together, so that their latencies
         // overlap (with one piece after the other a piece took a warp 400 cycles). ------------------------------------------------
@@ -344,7 +348,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
             f32_cluster_barrier();
         }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 152;");
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(ADDER_REGS));
         float_pair sum[C::MINE][8] = {}, lost[C::MINE][8] = {};  // [group][tokens]: this thread's feature, half of the groups of 16 tokens
         const int quarter = warp & 3, half = (groups + 1) >> 1, group0 = (warp >> 2) * half, mine_groups = min(half, groups - group0);
         const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16) + 16 * group0;
