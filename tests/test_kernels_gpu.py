@@ -87,6 +87,11 @@ def test_rmsnorm_of_many_picked_rows(ops, status, n, h, center):
         x = x - x.mean(1, keepdim=True)
     torch.testing.assert_close(out.float().cpu(), plain.rms_norm(x, weight.cpu(), 1e-5), **tol(torch.bfloat16, 3))
     ops.raise_on_status(status)
+    # the exact row rounded to bfloat16 (2^-8) with float32 sums behind it, and beside the other kernel's rows a neighbour here and there
+    exact = x.double() / ((x.double() ** 2).mean(1, keepdim=True) + 1e-5).sqrt() * weight.cpu().double()
+    assert ((out.double().cpu() - exact).abs() <= (2.0**-8 + 2.0**-20) * exact.abs() + 1e-30 + 2.0**-20 * center).all()
+    few = torch.cat([ops.rmsnorm_rows(resid, part.to(DEV), weight, 1e-5, torch.bfloat16, status, center=center) for part in rows.split(500)])
+    assert (few != out).float().mean().item() < 1e-3
     rows[[0, n - 1]] = torch.tensor([300, -1], dtype=torch.int32)  # rows that are not there: zeros, and a status
     bad = ops.new_status(DEV)
     out = ops.rmsnorm_rows(resid, rows.to(DEV), weight, 1e-5, torch.bfloat16, bad, center=center)
