@@ -5,8 +5,8 @@
 // tile it falls in, so a row's result does not depend on the rest of the batch: fmaf chains over 16 consecutive k, in ascending
 // order, whose results are added up with a compensated (Kahan) running sum.
 //
-// Epilogues: 0 store as T; 1 add into a float32 matrix (the residual stream); 2 store float32
-// (logits); 4 store max(v, 0)^2 as T.  The SwiGLU variant computes silu(A Wg^T) * (A Wu^T) (clockwork/engine/model.py:62-63).
+// Epilogues: 0 store as bfloat16; 1 add into a float32 matrix (the residual stream); 2 store float32
+// (logits); 4 store max(v, 0)^2 as bfloat16.  The SwiGLU variant computes silu(A Wg^T) * (A Wu^T) (clockwork/engine/model.py:62-63).
 #include "attention_mma.cuh"
 #include "gemm_f32.cuh"
 
@@ -23,9 +23,9 @@ __device__ __forceinline__ void kahan_add(float& sum, float& lost, float x) {
     sum = t;
 }
 
-template <typename T, bool SWIGLU>
+template <bool SWIGLU>
 __global__ void __launch_bounds__(256)
-gemm_ref_kernel(const T* __restrict__ A, const T* __restrict__ W, const T* __restrict__ W2,
+gemm_ref_kernel(const bf16* __restrict__ A, const bf16* __restrict__ W, const bf16* __restrict__ W2,
                 const float* __restrict__ bias, void* __restrict__ Cout, int M, int N, int K,
                 int lda, int ldc, int epilogue) {
     __shared__ float As[BK][BM + 4];
@@ -98,12 +98,12 @@ gemm_ref_kernel(const T* __restrict__ A, const T* __restrict__ W, const T* __res
             const size_t idx = (size_t)m * ldc + n;
             if (SWIGLU) {
                 const float g = v, u = sum2[i][j];
-                ((T*)Cout)[idx] = from_f<T>(g / (1.0f + expf(-g)) * u);
+                ((bf16*)Cout)[idx] = from_f<bf16>(g / (1.0f + expf(-g)) * u);
             } else if (epilogue == 0) {
-                ((T*)Cout)[idx] = from_f<T>(v);
+                ((bf16*)Cout)[idx] = from_f<bf16>(v);
             } else if (epilogue == 4) {  // the square of what is positive
                 v = fmaxf(v, 0.f);
-                ((T*)Cout)[idx] = from_f<T>(v * v);
+                ((bf16*)Cout)[idx] = from_f<bf16>(v * v);
             } else if (epilogue == 1) {
                 ((float*)Cout)[idx] += v;
             } else {
@@ -127,7 +127,7 @@ extern "C" int cw_gemm_ref(const void* A, const void* W, const float* bias, void
         return gemm_f32_run({(const float*)A, (const float*)W, nullptr, bias, (float*)C, M, N, K, lda, ldc, epilogue, status, 0, 0,
                              whole_pieces(A, lda) && whole_pieces(W, K)}, stream);
     if (dtype == 1)
-        gemm_ref_kernel<bf16, false><<<grid, 256, 0, stream>>>(
+        gemm_ref_kernel<false><<<grid, 256, 0, stream>>>(
             (const bf16*)A, (const bf16*)W, nullptr, bias, C, M, N, K, lda, ldc, epilogue);
     else
         return CW_ERR_BAD_DTYPE;
@@ -144,7 +144,7 @@ extern "C" int cw_gemm_ref_swiglu(const void* A, const void* Wgate, const void* 
         return gemm_f32_run({(const float*)A, (const float*)Wgate, (const float*)Wup, nullptr, (float*)C, M, N, K, K, N, 0, status, 0, 0,
                              whole_pieces(A, K) && whole_pieces(Wgate, K) && whole_pieces(Wup, K)}, stream);
     if (dtype == 1)
-        gemm_ref_kernel<bf16, true><<<grid, 256, 0, stream>>>(
+        gemm_ref_kernel<true><<<grid, 256, 0, stream>>>(
             (const bf16*)A, (const bf16*)Wgate, (const bf16*)Wup, nullptr, C, M, N, K, K, N, 0);
     else
         return CW_ERR_BAD_DTYPE;

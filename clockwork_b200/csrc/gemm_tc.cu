@@ -52,7 +52,7 @@ struct GemmParams {
     int kb_per_split;     // k-blocks per blockIdx.z
     int splits;
     int bn;               // persistent kernel: token-tile width chosen at run time (multiple of 16)
-    int tma_store;        // 1: unsplit tiles leave through shared memory and one TMA store / reduce-add
+    int tma_store;        // gemm_tc_kernel.  1: unsplit tiles leave through shared memory and one TMA store / reduce-add
     const float* bias;    // [N] or null
     void* C;
     int* status;
@@ -924,7 +924,7 @@ extern "C" int cw_gemm_tc_set_persistent_from(int tokens) {
 
 static Plan make_plan(int T, int N, int K, bool swiglu, int sm_count, bool c_by_tma = true, bool adds = false) {
     Plan pl;
-    pl.persistent = T >= g_persistent_from && sm_count > 0 && c_by_tma;  // its epilogue has no other way out than TMA
+    pl.persistent = T >= g_persistent_from && sm_count > 0 && c_by_tma;  // (the single-CTA kernel's epilogue has no other way out than TMA; the CTA-pair kernel's would)
     // (token tiles of the one-tile-per-CTA kernel are at most 128 wide: wider ones cannot be split over K,
     // and a product of a few hundred tokens has too few tiles to do without)
     pl.bn = T <= 16 ? 16 : (T <= 32 ? 32 : (T <= 64 ? 64 : 128));
@@ -1106,11 +1106,11 @@ static int gemm_tc_run(const void* X, const void* W, const void* W2, const float
     if (make_map(&mw, W, N, K, K, BM) != 0) return CW_ERR_UNSUPPORTED;
     if (make_map(&mw2, swiglu ? W2 : W, N, K, K, BM) != 0) return CW_ERR_UNSUPPORTED;
     if (make_map(&mx, X, T, K, ldx, pl.pair ? pl.bn / 2 : pl.bn) != 0) return CW_ERR_UNSUPPORTED;
-    const bool tma_store = (pl.splits == 1 || pl.pair) && c_by_tma && !emits;  // beginning a norm needs the new values in hand
+    const bool tma_store = !pl.pair && pl.splits == 1 && c_by_tma && !emits;  // beginning a norm needs the new values in hand
     // prompt portions: the persistent kernel, whose epilogue overlaps the next tile's MMAs
     const bool persistent = pl.persistent;
     CUtensorMap mc = mx;
-    if (tma_store && !pl.pair && make_map_c(&mc, C, T, N, ldc, persistent ? P_CHUNK : pl.bn, c_f32) != 0) return CW_ERR_UNSUPPORTED;
+    if (tma_store && make_map_c(&mc, C, T, N, ldc, persistent ? P_CHUNK : pl.bn, c_f32) != 0) return CW_ERR_UNSUPPORTED;
     GemmParams p;
     p.tma_store = tma_store ? 1 : 0;
     p.T = T; p.N = N; p.K = K; p.ldc = ldc; p.epilogue = epilogue;
@@ -1182,7 +1182,6 @@ extern "C" int cw_gemm_tc_parts(const void* X, const void* W, float* parts, int 
     if (make_map(&mw, W, N, K, K, BM) != 0) return CW_ERR_UNSUPPORTED;
     if (make_map(&mx, X, T, K, ldx, bn / 2) != 0) return CW_ERR_UNSUPPORTED;
     GemmParams p = {};
-    p.tma_store = 1;
     p.T = T; p.N = N; p.K = K; p.ldc = N; p.epilogue = 3; p.part_rows = part_rows;
     p.num_kb = num_kb; p.kb_per_split = num_kb / splits; p.splits = splits;
     p.bias = nullptr; p.C = parts; p.status = status; p.bn = bn;
