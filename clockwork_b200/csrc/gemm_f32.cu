@@ -395,12 +395,13 @@ __global__ void __launch_bounds__(F32_THREADS, 1) gemm_f32_kernel(const F32Args 
             ok = __all_sync(0xffffffffu, mbar_wait(first_full + 8 * set, parity, give_up));
             if (!ok) return;
             tc_fence_after();
+            // (which two are added first says nothing about the error, but every bit of a step follows from it)
             load(t, main0);
-            load(r, main0 + BN);
+            load(r, main0 + 2 * BN);
             landed(t);
             landed(r);
             plus(t, r);
-            load(r, main0 + 2 * BN);
+            load(r, main0 + BN);
             add(t);
             load(t, main0 + 3 * BN);
             landed(t);
