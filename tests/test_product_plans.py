@@ -45,6 +45,13 @@ def test_splits_are_equal_runs_of_whole_blocks():
     assert plan(256, 1536, 8960) > 1  # the down projection of the 1.5B layer at a few hundred tokens
 
 
+@pytest.mark.parametrize("t", [545, 600, 640, 700, 768])
+def test_slabs_do_not_run_in_rounds_that_cost_more_than_they_save(t):
+    """The down product of the 7B layer: its tiles fill most pairs once, and four splits of each would run in two rounds and more."""
+    assert plan(t, 3584, 18944) == 1 and plan(t, 4096, 14336) == 1
+    assert plan(t, 1536, 8960) > 1  # (few tiles, a long inner dimension)
+
+
 def test_other_token_counts_are_not_cut():
     for t in (1, 8, 64, 128, 1025, 2048, 4096):
         assert plan(t, 1536, 8960) == 1
