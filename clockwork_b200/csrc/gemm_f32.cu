@@ -10,11 +10,11 @@
 // along (Kahan); the small ones join what it carries.  Outputs that are not finite are formed again by fmaf (f32_plain).
 // Root mean square of the error over the sum of the products' magnitudes, in 2^-24 (B200, 200 x 4,000 outputs six times, K 64,
 // 1,536 and 8,960), this kernel and the chains of 16 fmaf with the same running sum that it replaced:
-//   normal operands          0.093 0.025 0.0104   chains 0.261 0.055 0.0238
-//   sizes spread over e      0.251 0.091 0.0404          0.475 0.139 0.0637
-//   sizes spread over e^3    0.755 0.638 0.543           0.931 0.672 0.563
-//   one sign                 0.495 0.336 0.417           0.732 0.349 0.444
-//   between 0 and 1          0.478 0.391 0.529           0.720 0.402 0.562
+//   normal operands          0.093 0.025 0.010   chains 0.261 0.055 0.024
+//   sizes spread over e      0.250 0.091 0.041          0.475 0.139 0.064
+//   sizes spread over e^3    0.754 0.638 0.543          0.931 0.672 0.563
+//   one sign                 0.494 0.336 0.417          0.732 0.349 0.444
+//   between 0 and 1          0.478 0.391 0.529          0.720 0.402 0.562
 // Tried: first parts of 8 bits, one sign 0.45 at K of 1,536; all four of w0 x0 and the small ones carried along one by one, 10 % less
 // of an error and 296 us instead of 242 for [gate, up] of 200 rows.
 //
@@ -27,9 +27,10 @@
 // a thread of another issues the MMAs.  The parts of the token rows follow one another, so that one MMA of two or three times the width
 // forms w1 [x0 | x1 | x2], w2 [x0 | x1] or w0 [x1 | x2]: 16 MMAs per 64 k, none of which takes less than about 64 cycles however narrow.
 // Eight other warps read out and add up what has been formed.  What bounds it: few rows, the 16 MMAs in a row (about 1,600 cycles per
-// 64 k); many, the way through shared memory and the cutting in three, then the sums (without either of the two [gate, up] of 200
-// rows takes 214 us).  Measured (B200, us, chains of fmaf -> this): 200 rows, [gate, up] 2 x 8,960 by 1,536 373 -> 242, 1,536 by
-// 8,960 219 -> 150, 2,048 by 1,536 64 -> 40; 64 rows 170 -> 70, 108 -> 47, 33 -> 33; 1 row 37 -> 37, 36 -> 34, 27 -> 27.
+// 64 k); many, the latencies of copying, cutting and adding with two warps of each a scheduler (issue slots 53 % busy, shared-memory
+// pipe 36 %, tensor pipe 18 %; [gate, up] of 200 rows takes 214 us without the cutting and the carried errors).
+// Measured (B200, us, chains of fmaf -> this): 200 rows, [gate, up] 2 x 8,960 by 1,536 373 -> 242, 1,536 by 8,960 219 -> 150, 2,048 by
+// 1,536 64 -> 39; 64 rows 170 -> 70, 108 -> 47, 33 -> 29; 8 rows 39 -> 37, 37 -> 33, 27 -> 27; 1 row 37 -> 37, 36 -> 33, 27 -> 25.
 // Tried: the same eight warps for both jobs, one after the other: every step's latency in a row.
 //
 // Every wait on an mbarrier is bounded.

@@ -17,7 +17,7 @@
 //                              received, in rank order, and finishes its slice of columns.  No global
 //                              scratch, no atomics, no cluster-wide barrier after the main loop, and
 //                              the result does not depend on which CTA finished first.
-//   gemm_tc_persistent_kernel  prompt portions (more than 256 tokens): one CTA per SM walks tiles with
+//   gemm_tc_persistent_kernel  prompt portions (more than 128 tokens): one CTA per SM walks tiles with
 //                              two TMEM accumulators (the epilogue of a tile overlaps the next one's MMAs);
 //                              also few tokens against three rounds of weight tiles or more (the logits)
 //   gemm_tc_pair_kernel        the same on CTA pairs (cta_group::2), in gemm_tc_pair.cuh
@@ -827,9 +827,9 @@ static int balanced_bn(int T, int N, bool swiglu, int sm_count) {
 
 static int g_pair_enabled = 1;
 static int g_pair_swiglu = 0;
-// Whether the SwiGLU product of prompt portions runs on CTA pairs too.  Off: measured equal to the
-// single-CTA persistent kernel within 2 % from 256 to 4,096 tokens (under the power cap the product's
-// rate is a matter of energy per FLOP, not of shared-memory traffic per tile).
+// Whether the SwiGLU product of prompt portions runs on CTA pairs too.  Off: within 5 % of the single-CTA persistent kernel at the
+// 1.5B sizes (8,960 by 1,536, 150 to 2,048 tokens; 3,000: 8 % slower, 4,096: 4 % faster), but 1.3 to 1.5 times as long at the 7B sizes
+// (18,944 by 3,584: 545 tokens 208 us against 135, 2,048 tokens 678 against 473).
 extern "C" int cw_gemm_tc_set_pair_swiglu(int on) { g_pair_swiglu = on ? 1 : 0; return CW_OK; }
 static int g_forced_bn = 0;
 static int* g_split_flags = nullptr;  // device words for the CTA-pair kernel's split products (zero between launches)
@@ -855,7 +855,9 @@ static int pair_splits(int tiles, int num_kb, int sm_count) {
 
 // How many ways a CTA-pair product that adds into its output is cut over K.  The number decides the order of an output's sum, so
 // it follows from a rule of its own, in which a k-block of any width counts 330 + 0.2 bn ns and a split's turn to add 1000 + 25
-// bn, and does not move with the widths that the tiles then get (balanced_bn_pair).
+// bn, and does not move with the widths that the tiles then get (balanced_bn_pair).  That is what they took before the issuing
+// threads were elected and the epilogue went straight to global memory.  Against the best of all splits of the kernel as it is (B200, 8
+// products above 1,024 tokens): within 1 % but for 1536 x 8960 at 1,298 and 1,500 tokens, 6 and 11 %, and 1024 x 4096 to 2,048, 3 to 27 %.
 static int add_splits(int T, int N, int num_kb, int sm_count) {
     const int m_tiles = (N + 2 * BM - 1) / (2 * BM), pairs = sm_count / 2;
     long long best_cost = -1;

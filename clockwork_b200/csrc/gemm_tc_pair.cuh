@@ -15,15 +15,15 @@
 // bounded; a CTA that gives up records CW_ST_WAIT_TIMEOUT, and both CTAs meet at the cluster
 // barrier before tensor memory is freed.
 //
-// Few tiles and a long inner dimension (a few hundred tokens against K = 8960): a pair streams its
-// weight rows at the rate its six stages in flight allow (about 3 k-blocks per microsecond), so
-// with fewer tiles than pairs the product's time is K's, whatever the tile's width.  The products
-// that add into the residual are then split over K (p.splits > 1): a unit of work is (tile, split),
-// every split adds its partial tile into the residual with the same reductions, and the splits
-// of a tile add in split order: split k waits, before its first store, until split k - 1 has
-// published (its word of p.split_flags == k) that its adds are complete.  Units are handed out in the
-// order (tile, split) to pairs that all run at once and take their units in ascending order, so the
-// unit waited for is always running or done.
+// Few tiles and a long inner dimension (a few hundred tokens against K = 8960): a k-block takes a pair
+// at least 180 ns, a stage's round trip over the stages in flight (wide tiles 1.3 ns a token), so with
+// fewer tiles than pairs the product's time is K's, whatever the tile's width.  The products that add
+// into the residual are then split over K (p.splits > 1): a unit of work is (tile, split), every split
+// adds its partial tile into the residual with the same reductions, and the splits of a tile add in
+// split order: split k waits, before its first store, until split k - 1 has published (its word of
+// p.split_flags == k) that its adds are complete.  Units are handed out in the order (tile, split) to
+// pairs that all run at once and take their units in ascending order, so the unit waited for is always
+// running or done.
 #pragma once
 #include "tc_common.cuh"
 
@@ -43,8 +43,9 @@ struct PairCfgT {
     static constexpr int A_BYTES = BM * BK * 2;                  // this CTA's 128 rows of W (of each W)
     static constexpr int SMEM_BYTES = PAIR_MAX_SMEM;
     static constexpr int TMEM_COLS = 512;                        // two buffers of up to 256 columns
-    // A stage holds the weight rows and half of a token tile of bn, so that narrow tiles have more stages (10 at 64 tokens, 6 at
-    // 256): what bounds the products of few tiles and a long K is the latency of a stage's round trip over the stages in flight.
+    // A stage holds the weight rows and half of a token tile of bn, so that narrow tiles have more stages (11 at 64 tokens, 7 at
+    // 256; SwiGLU 6 and, at 128, 5): what bounds the products of few tiles and a long K is the latency of a stage's round trip over
+    // the stages in flight.
     __host__ __device__ static constexpr int stage_bytes(int bn) { return (SWIGLU ? 2 : 1) * A_BYTES + bn / 2 * BK * 2; }
     __host__ __device__ static constexpr int stages(int bn) {
         const int n = (SMEM_BYTES - 2048) / stage_bytes(bn);
