@@ -876,26 +876,30 @@ static int add_splits(int T, int N, int num_kb, int sm_count) {
 }
 // A product whose splits over K are kept apart (epilogue 3): every split stores its partial tile in a
 // slab of its own and whoever reads the result next adds the slabs, in split order (the RMSNorm that
-// follows a product into the residual reads the residual anyway).  Nothing takes turns, so splits may
-// outnumber the pairs and run in rounds.  The number of splits is that of the least time as pair_cost has it, with about
-// d T N / 500 ns for d slabs (their bytes, written and read again).  Measured with the norm behind it (B200, 8 products at 130 to
-// 1,024 tokens, us by a rule that counted 330 + 0.2 bn ns a k-block, which the kernel no longer takes -> this): 3584 x 18944, 545
-// tokens 129 -> 76, 768 tokens 141 -> 90 (four slabs in two rounds; now added straight), 512 tokens 74 -> 72; 2.5 % behind the best
-// of all splits on average, before 5.
+// follows a product into the residual reads the residual anyway).  Nothing takes turns.  The number of splits (which
+// decides the order of the sums) follows from a rule of its own as in add_splits: a k-block 330 + 0.2 bn ns, a tile's store
+// 1000 + 25 bn ns once, and each further slab costs its reader about T N / 500 ns (its bytes, written and read again); and only splits
+// that all run at once.  With splits in rounds as well, products whose tiles fill most pairs once were cut in four that ran in two
+// (B200, with the norm behind it, us, four slabs -> added straight): 3584 x 18944, 545 tokens 129 -> 76, 768 tokens 141 -> 90; 4096 x
+// 14336, 640 tokens 114 -> 71.
 // Measured in the step (Qwen2.5-1.5B sizes, K = 8,960): 15 % of a 256-token prompt's time, 10 % at 512, 4 % at
 // 1,024; from 1,056 tokens on the slabs cost what the splits save (a mixed step of 1,056 tokens 5 % slower),
 // so longer products add into their output with splits that take turns, as before.
 #define PARTS_MAX_TOKENS 1024
 static void parts_plan(int T, int N, int K, int sm_count, int* splits_out, int* bn_out) {
-    const int num_kb = (K + BK - 1) / BK;
+    const int m_tiles = (N + 2 * BM - 1) / (2 * BM), pairs = sm_count / 2, num_kb = (K + BK - 1) / BK;
     long long best_cost = -1;
     int best_d = 1;
-    for (int d = 1; d <= 8; ++d) {
-        if (num_kb % d != 0 || (d > 1 && num_kb / d < 8)) continue;
-        const long long cost = pair_cost(balanced_bn_pair(T, N, num_kb, d, sm_count), T, N, num_kb, d, sm_count) + (d > 1 ? (long long)d * T * N / 500 : 0);
-        if (best_cost < 0 || cost < best_cost) {
-            best_cost = cost;
-            best_d = d;
+    for (int bn = 256; bn >= 64; bn -= 16) {
+        const int tiles = m_tiles * ((T + bn - 1) / bn);
+        for (int d = 1; d <= 8; ++d) {
+            if (num_kb % d != 0 || (d > 1 && (num_kb / d < 8 || tiles * d > pairs))) continue;
+            const long long rounds = ((long long)tiles * d + pairs - 1) / pairs;
+            const long long cost = rounds * (num_kb / d) * (330 + bn / 5) + 1000 + 25 * bn + (long long)(d - 1) * T * N / 500;
+            if (best_cost < 0 || cost < best_cost) {
+                best_cost = cost;
+                best_d = d;
+            }
         }
     }
     *splits_out = best_d;
